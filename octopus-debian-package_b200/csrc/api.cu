@@ -1945,7 +1945,7 @@ hpsi_status hpsi_dotp_matrix(hpsi_mesh *m, const hpsi_batch *a, const hpsi_batch
     return HPSI_ERR_ARG;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int nst = a->nst, splits = gram_splits(m->np);
+  const int nst = a->nst, splits = gram_splits(m->np, nst, a->ptr == b->ptr && a->ld == b->ld);
   const size_t pbytes = size_t(splits) * 4 * nst * nst * sizeof(double);
   s = m->scratch.ensure(pbytes + 2 * size_t(nst) * nst * sizeof(double));
   if (s) return s;
@@ -1973,7 +1973,7 @@ hpsi_status hpsi_orthonormalize_cholesky(hpsi_mesh *m, hpsi_batch *psi, void *st
     return HPSI_ERR_ARG;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int nst = psi->nst, splits = gram_splits(m->np);
+  const int nst = psi->nst, splits = gram_splits(m->np, nst, true);
   const size_t pbytes = size_t(splits) * 4 * nst * nst * sizeof(double);
   const size_t mbytes = 2 * size_t(nst) * nst * sizeof(double);
   s = m->scratch.ensure(pbytes + 3 * mbytes + 16);

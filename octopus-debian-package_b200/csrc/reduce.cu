@@ -9,6 +9,7 @@
 // 970-1167) and the cholesky_serial branch of
 // X(states_elec_orthogonalization_full) (src/states/states_elec_calc_inc.F90:66-98).
 #include <algorithm>
+#include <mutex>
 
 #include "reduce.cuh"
 
@@ -98,69 +99,154 @@ __global__ void state_sum_finalize(const double *partial, int nblk, int nst, dou
 }
 
 // ---------------------------------------------------------------------------
-// Gram matrix of the real views: G[u][v] = sum_p Ar[p][u] Br[p][v],
-// u, v over 2*nst real lanes.  grid (ceil(n/32), ceil(n/32), splits),
-// block (16,16); each thread a 2x2 block.  Partials [splits][n][n].
+// Matrix products of a batch on the FP64 tensor cores (mma.sync.m8n8k4.f64)
+// over the batch's real view (lane 2 s = re, 2 s + 1 = im of state s).  They
+// run at the FP64 pipe's rate, like plain multiply-adds, but a fragment feeds
+// 8 products per value read from shared memory: with 64 x 64 tiles (8 warps of
+// 16 x 32) the FP64 pipe is the bound.  Sums stay FP64 for both storage types.
+constexpr int GT = 64;   // tile edge (real lanes, rows)
+constexpr int GK = 16;   // K step staged at once
+constexpr int GST = 4;   // staged steps
+
+__device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d0), "+d"(d1)
+               : "d"(a), "d"(b));
+}
+
+// One complex state (16 bytes FP64, 8 FP32) to shared memory, zero where !ok.
+__device__ __forceinline__ void copy_state(double *d, const double *g, bool ok) {
+  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(d));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(g), "r"(ok ? 16 : 0));
+}
+__device__ __forceinline__ void copy_state(float *d, const float *g, bool ok) {
+  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(d));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(g), "r"(ok ? 8 : 0));
+}
+// Row pitch of a staged K x 64 block: the four K rows of a fragment read fall
+// into different bank groups (FP64 pitch = 4 mod 16, FP32 = 8 mod 32).
+template <typename T>
+constexpr int gram_pitch() {
+  return sizeof(T) == 8 ? GT + 4 : GT + 8;
+}
+
+// Gram matrix of the real views: G[u][v] = sum_p Ar[p][u] Br[p][v], u, v over
+// n = 2 nst lanes.  grid (tile pairs, splits over the points); block 256.
+// sym: a is b, only the tiles on and above the diagonal are listed (the matrix
+// is Hermitian).  Partials [splits][n][n].
+// 96 states, 267,761 points, FP64 (gram alone, one side): 3.97 ms with 2 x 2
+// register blocks per thread over 32 x 32 tiles.
 template <typename T>
 __global__ void __launch_bounds__(256) gram_kernel(const T *a, long long lda, const T *b, long long ldb, int np,
-                                                  int n, double *partial) {
-  __shared__ double sa[32][33];
-  __shared__ double sb[32][33];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int t = ty * 16 + tx;
-  const int u0 = blockIdx.y * 32, v0 = blockIdx.x * 32;
-  const long long per = (np + gridDim.z - 1) / gridDim.z;
-  const long long p0 = blockIdx.z * per, p1 = min((long long)np, p0 + per);
-  double c[2][2] = {{0, 0}, {0, 0}};
-  for (long long pb = p0; pb < p1; pb += 32) {
-    for (int i = t; i < 32 * 32; i += 256) {
-      const int pp = i / 32, l = i % 32;
-      const long long row = pb + pp;
-      sa[pp][l] = (row < p1 && u0 + l < n) ? double(a[row * 2 * lda + u0 + l]) : 0.0;
-      sb[pp][l] = (row < p1 && v0 + l < n) ? double(b[row * 2 * ldb + v0 + l]) : 0.0;
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int pp = 0; pp < 32; ++pp) {
-      const double a0 = sa[pp][ty * 2], a1 = sa[pp][ty * 2 + 1];
-      const double b0 = sb[pp][tx * 2], b1 = sb[pp][tx * 2 + 1];
-      c[0][0] = fma(a0, b0, c[0][0]);
-      c[0][1] = fma(a0, b1, c[0][1]);
-      c[1][0] = fma(a1, b0, c[1][0]);
-      c[1][1] = fma(a1, b1, c[1][1]);
-    }
-    __syncthreads();
+                                                  int n, int tiles, int sym, double *partial) {
+  constexpr int PITCH = gram_pitch<T>();
+  extern __shared__ __align__(16) unsigned char gsm[];
+  T *sa = reinterpret_cast<T *>(gsm);           // [GST][GK][PITCH]
+  T *sb = sa + GST * GK * PITCH;
+  int tu, tv;
+  if (sym) {
+    // pair index -> (row, column) of the upper triangle
+    int r = 0, i = blockIdx.x;
+    while (i >= tiles - r) i -= tiles - r++;
+    tu = r;
+    tv = r + i;
+  } else {
+    tu = blockIdx.x / tiles;
+    tv = blockIdx.x % tiles;
   }
-  double *o = partial + (long long)blockIdx.z * n * n;
+  const int u0 = tu * GT, v0 = tv * GT;
+  const bool same = sym && tu == tv;  // one staged block serves both sides
+  const long long per = (np + gridDim.y - 1) / gridDim.y;
+  const long long p0 = blockIdx.y * per, p1 = min((long long)np, p0 + per);
+  const int nk = p1 > p0 ? int((p1 - p0 + GK - 1) / GK) : 0;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int wu = (warp & 3) * 16, wv = (warp >> 2) * 32;
+  auto stage = [&](int k) {
+    if (k < nk) {
+      const int s = k % GST;
+      for (int i = t; i < GK * (GT / 2); i += 256) {
+        const int pp = i / (GT / 2), l = 2 * (i % (GT / 2));
+        const long long row = p0 + (long long)k * GK + pp;
+        const bool in = row < p1;
+        const bool ua = in && u0 + l < n, vb = in && v0 + l < n;
+        copy_state(sa + (s * GK + pp) * PITCH + l, ua ? a + row * 2 * lda + u0 + l : a, ua);
+        if (!same) copy_state(sb + (s * GK + pp) * PITCH + l, vb ? b + row * 2 * ldb + v0 + l : b, vb);
+      }
+    }
+    cp_async_commit();
+  };
+  double c[2][4][2] = {};
+  for (int k = 0; k < GST - 1; ++k) stage(k);
+  for (int k = 0; k < nk; ++k) {
+    cp_async_wait<GST - 2>();
+    __syncthreads();
+    stage(k + GST - 1);
+    const T *xa = sa + (k % GST) * GK * PITCH, *xb = (same ? sa : sb) + (k % GST) * GK * PITCH;
+#pragma unroll
+    for (int kk = 0; kk < GK; kk += 4) {
+      double fa[2], fb[4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) fa[i] = double(xa[(kk + (lane & 3)) * PITCH + wu + 8 * i + (lane >> 2)]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) fb[j] = double(xb[(kk + (lane & 3)) * PITCH + wv + 8 * j + (lane >> 2)]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dmma(c[i][j][0], c[i][j][1], fa[i], fb[j]);
+    }
+  }
+  cp_async_wait<0>();
+  double *o = partial + (long long)blockIdx.y * n * n;
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int u = u0 + ty * 2 + i, v = v0 + tx * 2 + j;
-      if (u < n && v < n) o[(long long)u * n + v] = c[i][j];
+    for (int j = 0; j < 4; ++j) {
+      const int u = u0 + wu + 8 * i + (lane >> 2), v = v0 + wv + 8 * j + 2 * (lane & 3);
+      if (u < n && v < n) *reinterpret_cast<double2 *>(o + (long long)u * n + v) = make_double2(c[i][j][0], c[i][j][1]);
     }
 }
 
-// S[i][j] = dV * (conj(a_i) . b_j) from the real Gram G (n = 2*nst)
-__global__ void gram_finalize(const double *partial, int splits, int nst, double dv, double *S) {
-  const int i = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nst) return;
+// S[i][j] = dV * (conj(a_i) . b_j) from the real Gram G (n = 2 * nst); sym:
+// G holds the tiles on and above the diagonal, entries below it are conjugates.
+// block (32, 8): 8 slices of the splits per entry, folded in a fixed order.
+__global__ void __launch_bounds__(256) gram_finalize(const double *partial, int splits, int nst, double dv, int sym,
+                                                     double *S) {
+  __shared__ double red[8][32][4];
+  const int i = blockIdx.y, j = blockIdx.x * 32 + threadIdx.x;
   const int n = 2 * nst;
+  const bool flip = sym && 2 * i / GT > 2 * j / GT;
+  const int r = flip ? j : i, q = flip ? i : j;
   Kahan re = {0, 0}, im = {0, 0};
-  for (int z = 0; z < splits; ++z) {
-    const double *G = partial + (long long)z * n * n;
-    const double rr = G[(2 * i) * n + 2 * j], ii = G[(2 * i + 1) * n + 2 * j + 1];
-    const double ri = G[(2 * i) * n + 2 * j + 1], ir = G[(2 * i + 1) * n + 2 * j];
-    kadd(re, rr);
-    kadd(re, ii);
-    kadd(im, ri);
-    kadd(im, -ir);
+  if (j < nst) {
+#pragma unroll 4
+    for (int z = threadIdx.y; z < splits; z += 8) {
+      const double2 *G0 = reinterpret_cast<const double2 *>(partial + ((long long)z * n + 2 * r) * n) + q;
+      const double2 g0 = G0[0], g1 = G0[nst];  // {rr, ri}, {ir, ii}
+      kadd(re, g0.x);
+      kadd(re, g1.y);
+      kadd(im, g0.y);
+      kadd(im, -g1.x);
+    }
   }
+  red[threadIdx.y][threadIdx.x][0] = re.s;
+  red[threadIdx.y][threadIdx.x][1] = re.c;
+  red[threadIdx.y][threadIdx.x][2] = im.s;
+  red[threadIdx.y][threadIdx.x][3] = im.c;
+  __syncthreads();
+  if (threadIdx.y != 0 || j >= nst) return;
+  for (int z = 1; z < 8; ++z) {
+    kadd(re, red[z][threadIdx.x][0]);
+    re.c += red[z][threadIdx.x][1];
+    kadd(im, red[z][threadIdx.x][2]);
+    im.c += red[z][threadIdx.x][3];
+  }
+  const double y = (im.s + im.c) * dv;
   S[2 * ((long long)i * nst + j)] = (re.s + re.c) * dv;
-  S[2 * ((long long)i * nst + j) + 1] = (im.s + im.c) * dv;
+  S[2 * ((long long)i * nst + j) + 1] = flip ? -y : y;
 }
 
-// Cholesky S = U^H U (upper) and the inverse of U, one CTA.  S, U, Uinv are
+// Cholesky S = U^H U (upper) and the inverse of U, one CTA, in global memory:
+// for batches whose triangle does not fit shared memory.  S, U, Uinv are
 // complex nst x nst row-major (interleaved).  err[0] = 1 if S is not
 // positive definite.
 __global__ void cholesky_inverse_kernel(const double *S, int nst, double *U, double *Uinv, int *err) {
@@ -216,44 +302,166 @@ __global__ void cholesky_inverse_kernel(const double *S, int nst, double *U, dou
   }
 }
 
-// psi[p][j] <- sum_{i<=j} psi[p][i] Uinv[i][j]; one CTA per row block.
+// The same in shared memory, the upper triangle packed by columns (entry
+// (i, j), i <= j, at j (j + 1) / 2 + i): right-looking Cholesky, then the
+// triangle inverted in place column by column.  A step's updates are spread
+// over the CTA instead of one thread's chain of dependent global loads.
+__global__ void __launch_bounds__(512) cholesky_inverse_smem_kernel(const double *S, int nst, double *U, double *Uinv,
+                                                                   int *err) {
+  extern __shared__ __align__(16) double2 M[];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, nw = blockDim.x >> 5;
+  auto at = [](int i, int j) { return j * (j + 1) / 2 + i; };
+  for (int j = warp; j < nst; j += nw)
+    for (int i = lane; i <= j; i += 32)
+      M[at(i, j)] = make_double2(S[2 * ((long long)i * nst + j)], S[2 * ((long long)i * nst + j) + 1]);
+  __syncthreads();
+  for (int j = 0; j < nst; ++j) {
+    double d = M[at(j, j)].x;
+    __syncthreads();
+    if (!(d > 0.0)) {
+      if (t == 0) err[0] = 1;
+      d = 1.0;
+    }
+    const double r = sqrt(d);
+    if (t == 0) M[at(j, j)] = make_double2(r, 0.0);
+    for (int c = j + 1 + t; c < nst; c += blockDim.x) {
+      double2 &x = M[at(j, c)];
+      x.x /= r;
+      x.y /= r;
+    }
+    __syncthreads();
+    // trailing update: M(i, c) -= conj(U(j, i)) U(j, c)
+    for (int c = j + 1 + warp; c < nst; c += nw) {
+      const double2 b = M[at(j, c)];
+      for (int i = j + 1 + lane; i <= c; i += 32) {
+        const double2 a = M[at(j, i)];
+        double2 &x = M[at(i, c)];
+        x.x -= a.x * b.x + a.y * b.y;
+        x.y -= a.x * b.y - a.y * b.x;
+      }
+    }
+    __syncthreads();
+  }
+  for (int j = warp; j < nst; j += nw)
+    for (int i = lane; i < nst; i += 32) {
+      const double2 x = i <= j ? M[at(i, j)] : make_double2(0.0, 0.0);
+      U[2 * ((long long)i * nst + j)] = x.x;
+      U[2 * ((long long)i * nst + j) + 1] = x.y;
+    }
+  __syncthreads();
+  // column j of the inverse: -X(0..j-1, 0..j-1) U(0..j-1, j) / U(j, j), X the
+  // inverse of the leading block (four lanes per row: all rows at once)
+  double2 *v = M + nst * (nst + 1) / 2;  // the new column
+  for (int j = 0; j < nst; ++j) {
+    const double d = M[at(j, j)].x;
+    for (int i0 = 0; i0 < j; i0 += blockDim.x / 4) {
+      const int i = i0 + t / 4;
+      double sr = 0.0, si = 0.0;
+      if (i < j) {
+#pragma unroll 4
+        for (int k = i + (t & 3); k < j; k += 4) {
+          const double2 x = M[at(i, k)], u = M[at(k, j)];
+          sr += x.x * u.x - x.y * u.y;
+          si += x.x * u.y + x.y * u.x;
+        }
+      }
+#pragma unroll
+      for (int o = 2; o > 0; o >>= 1) {
+        sr += __shfl_xor_sync(0xffffffffu, sr, o);
+        si += __shfl_xor_sync(0xffffffffu, si, o);
+      }
+      if (i < j && (t & 3) == 0) v[i] = make_double2(-sr / d, -si / d);
+    }
+    __syncthreads();
+    for (int i = t; i < j; i += blockDim.x) M[at(i, j)] = v[i];
+    if (t == 0) M[at(j, j)] = make_double2(1.0 / d, 0.0);
+    __syncthreads();
+  }
+  for (int j = warp; j < nst; j += nw)
+    for (int i = lane; i < nst; i += 32) {
+      const double2 x = i <= j ? M[at(i, j)] : make_double2(0.0, 0.0);
+      Uinv[2 * ((long long)i * nst + j)] = x.x;
+      Uinv[2 * ((long long)i * nst + j) + 1] = x.y;
+    }
+}
+
+// psi[p][j] <- sum_{i<=j} psi[p][i] Uinv[i][j], in place: a CTA owns 64 rows
+// and takes the 64-lane column tiles from the last to the first, so that a
+// tile is written only after every tile that reads it; per tile the rows times
+// the real form of Uinv's columns (K up to the tile's end: the matrix is
+// triangular) on the FP64 tensor cores.
 template <typename T>
 __global__ void __launch_bounds__(256) trsm_apply_kernel(T *psi, long long ld, int np, int nst,
                                                         const double *Uinv) {
-  using V = typename C2<T>::type;
-  extern __shared__ double rowbuf[];  // rows_per_iter x nst complex
-  const int t = threadIdx.x;
-  const int R = max(1, 256 / nst);  // rows per iteration
-  const long long per = (np + gridDim.x - 1) / gridDim.x;
-  const long long p0 = blockIdx.x * per, p1 = min((long long)np, p0 + per);
-  for (long long pb = p0; pb < p1; pb += R) {
-    __syncthreads();
-    for (int i = t; i < R * nst; i += blockDim.x) {
-      const long long row = pb + i / nst;
-      const int s = i % nst;
-      if (row < p1) {
-        const V x = reinterpret_cast<const V *>(psi + row * 2 * ld)[s];
-        rowbuf[2 * i] = double(x.x);
-        rowbuf[2 * i + 1] = double(x.y);
+  constexpr int APITCH = sizeof(T) == 8 ? GK + 4 : GK + 4;  // row pitch of the staged rows
+  constexpr int WPITCH = GT + 4;
+  extern __shared__ __align__(16) unsigned char gsm[];
+  double *sw = reinterpret_cast<double *>(gsm);          // [2][GK][WPITCH]
+  T *sx = reinterpret_cast<T *>(sw + 2 * GK * WPITCH);   // [GST][GT][APITCH]
+  const int n = 2 * nst;
+  const long long r0 = (long long)blockIdx.x * GT;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int wr = (warp & 3) * 16, wv = (warp >> 2) * 32;
+  for (int v0 = (n - 1) / GT * GT; v0 >= 0; v0 -= GT) {
+    const int kend = min(n, v0 + GT), nk = (kend + GK - 1) / GK;
+    auto stage = [&](int k) {
+      if (k < nk) {
+        for (int i = t; i < GT * (GK / 2); i += 256) {
+          const int rr = i / (GK / 2), l = 2 * (i % (GK / 2));
+          const bool ok = r0 + rr < np && k * GK + l < kend;
+          copy_state(sx + ((k % GST) * GT + rr) * APITCH + l, ok ? psi + (r0 + rr) * 2 * ld + k * GK + l : psi, ok);
+        }
+      }
+      cp_async_commit();
+    };
+    // one complex entry of Uinv per thread and step: rows 2 i, 2 i + 1 of the
+    // real form are {ur, ui}, {-ui, ur}
+    const int wi = t / (GT / 2), wj = t % (GT / 2);
+    auto entry = [&](int k) {
+      const int i = k * (GK / 2) + wi, j = v0 / 2 + wj;
+      return k < nk && i < nst && j < nst ? __ldg(reinterpret_cast<const double2 *>(Uinv) + (long long)i * nst + j)
+                                          : make_double2(0.0, 0.0);
+    };
+    double c[2][4][2] = {};
+    for (int k = 0; k < GST - 1; ++k) stage(k);
+    double2 w = entry(0);
+    for (int k = 0; k < nk; ++k) {
+      double *swk = sw + (k & 1) * GK * WPITCH;
+      *reinterpret_cast<double2 *>(swk + (2 * wi) * WPITCH + 2 * wj) = w;
+      *reinterpret_cast<double2 *>(swk + (2 * wi + 1) * WPITCH + 2 * wj) = make_double2(-w.y, w.x);
+      w = entry(k + 1);
+      cp_async_wait<GST - 2>();
+      __syncthreads();
+      stage(k + GST - 1);
+      const T *xk = sx + (k % GST) * GT * APITCH;
+#pragma unroll
+      for (int kk = 0; kk < GK; kk += 4) {
+        double fa[2], fb[4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) fa[i] = double(xk[(wr + 8 * i + (lane >> 2)) * APITCH + kk + (lane & 3)]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) fb[j] = swk[(kk + (lane & 3)) * WPITCH + wv + 8 * j + (lane >> 2)];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) dmma(c[i][j][0], c[i][j][1], fa[i], fb[j]);
       }
     }
-    __syncthreads();
-    for (int i = t; i < R * nst; i += blockDim.x) {
-      const int rr = i / nst, j = i % nst;
-      const long long row = pb + rr;
-      if (row >= p1) continue;
-      double yr = 0.0, yi = 0.0;
-      const double *x = rowbuf + 2 * rr * nst;
-      for (int k = 0; k <= j; ++k) {
-        const double ur = __ldg(Uinv + 2 * (k * nst + j)), ui = __ldg(Uinv + 2 * (k * nst + j) + 1);
-        yr = fma(x[2 * k], ur, fma(-x[2 * k + 1], ui, yr));
-        yi = fma(x[2 * k], ui, fma(x[2 * k + 1], ur, yi));
+    cp_async_wait<0>();
+    __syncthreads();  // every read of this tile's columns is done
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const long long row = r0 + wr + 8 * i + (lane >> 2);
+        const int v = v0 + wv + 8 * j + 2 * (lane & 3);
+        if (row < np && v < n) {
+          typename C2<T>::type y;
+          y.x = T(c[i][j][0]);
+          y.y = T(c[i][j][1]);
+          *reinterpret_cast<typename C2<T>::type *>(psi + row * 2 * ld + v) = y;
+        }
       }
-      V y;
-      y.x = static_cast<decltype(y.x)>(yr);
-      y.y = static_cast<decltype(y.y)>(yi);
-      reinterpret_cast<V *>(psi + row * 2 * ld)[j] = y;
-    }
   }
 }
 
@@ -352,40 +560,68 @@ hpsi_status launch_state_sum(int mode, const T *a, long long lda, const T *b, lo
   return HPSI_OK;
 }
 
-int gram_splits(int np) {
-  int s = (np + 8191) / 8192;
-  return s < 1 ? 1 : (s > 256 ? 256 : s);
+// Splits of the points: as many CTAs as the SMs hold at once (three each), at
+// least 64 points each, and partial matrices of at most 64 MB.
+int gram_splits(int np, int nst, bool sym) {
+  const long long tiles = (2LL * nst + GT - 1) / GT, pairs = sym ? tiles * (tiles + 1) / 2 : tiles * tiles;
+  long long s = std::max<long long>(1, 3LL * 148 / pairs);
+  s = std::min<long long>(s, (np + 63) / 64);
+  s = std::min<long long>(s, std::max<long long>(1, (64LL << 20) / (4LL * nst * nst * 8)));
+  return int(std::max<long long>(1, std::min<long long>(s, 65535)));
 }
 
 template <typename T>
 hpsi_status launch_gram(const T *a, long long lda, const T *b, long long ldb, int np, int nst, double *partial,
                         int splits, double dv, double *S, cudaStream_t st) {
-  const int n = 2 * nst;
-  dim3 grid((n + 31) / 32, (n + 31) / 32, splits);
-  gram_kernel<T><<<grid, dim3(16, 16), 0, st>>>(a, lda, b, ldb, np, n, partial);
+  const int n = 2 * nst, tiles = (n + GT - 1) / GT;
+  const bool sym = a == b && lda == ldb;
+  constexpr size_t smem = size_t(2) * GST * GK * gram_pitch<T>() * sizeof(T);
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  std::call_once(once, [&] {
+    attr = cudaFuncSetAttribute(gram_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  });
+  HPSI_TRY_CUDA(attr);
+  const long long pairs = sym ? (long long)tiles * (tiles + 1) / 2 : (long long)tiles * tiles;
+  gram_kernel<T><<<dim3(unsigned(pairs), unsigned(splits)), 256, smem, st>>>(a, lda, b, ldb, np, n, tiles, sym,
+                                                                             partial);
   HPSI_CHECK_LAUNCH();
-  gram_finalize<<<dim3((nst + 127) / 128, nst), 128, 0, st>>>(partial, splits, nst, dv, S);
+  gram_finalize<<<dim3((nst + 31) / 32, nst), dim3(32, 8), 0, st>>>(partial, splits, nst, dv, sym, S);
   HPSI_CHECK_LAUNCH();
   return HPSI_OK;
 }
 
 hpsi_status launch_cholesky_inverse(const double *S, int nst, double *U, double *Uinv, int *err, cudaStream_t st) {
-  cholesky_inverse_kernel<<<1, 256, 0, st>>>(S, nst, U, Uinv, err);
+  const size_t smem = (size_t(nst) * (nst + 1) / 2 + nst) * sizeof(double2);
+  if (smem <= 226 * 1024) {
+    static std::once_flag once;
+    static cudaError_t attr = cudaSuccess;
+    std::call_once(once, [&] {
+      attr = cudaFuncSetAttribute(cholesky_inverse_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+    });
+    HPSI_TRY_CUDA(attr);
+    cholesky_inverse_smem_kernel<<<1, 512, smem, st>>>(S, nst, U, Uinv, err);
+  } else {
+    cholesky_inverse_kernel<<<1, 256, 0, st>>>(S, nst, U, Uinv, err);
+  }
   HPSI_CHECK_LAUNCH();
   return HPSI_OK;
 }
 
 template <typename T>
 hpsi_status launch_trsm_apply(T *psi, long long ld, int np, int nst, const double *Uinv, cudaStream_t st) {
-  const int R = nst >= 256 ? 1 : 256 / nst;
-  const size_t smem = size_t(R) * nst * 2 * sizeof(double);
-  if (smem > 48 * 1024) {
+  constexpr size_t smem = size_t(2) * GK * (GT + 4) * sizeof(double) + size_t(GST) * GT * (GK + 4) * sizeof(T);
+  if (nst > 1536) {
     set_error("orthonormalisation supports at most 1536 states");
     return HPSI_ERR_UNSUPPORTED;
   }
-  int nb = (np + 1023) / 1024;
-  nb = nb < 1 ? 1 : (nb > 2368 ? 2368 : nb);
-  trsm_apply_kernel<T><<<nb, 256, smem, st>>>(psi, ld, np, nst, Uinv);
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  std::call_once(once, [&] {
+    attr = cudaFuncSetAttribute(trsm_apply_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  });
+  HPSI_TRY_CUDA(attr);
+  trsm_apply_kernel<T><<<unsigned((np + GT - 1) / GT), 256, smem, st>>>(psi, ld, np, nst, Uinv);
   HPSI_CHECK_LAUNCH();
   return HPSI_OK;
 }

@@ -1,0 +1,58 @@
+"""Overlap matrix and Cholesky orthonormalisation at the edges of their tiles:
+64 real lanes (32 states), 16 points or lanes per step, and the largest triangle
+the shared-memory Cholesky holds (168 states)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _mesh():
+    from hpsi.mesh import index_box_mesh
+    return index_box_mesh((13, 11, 9), 0.4)  # 1287 points: not a multiple of 16 or 64
+
+
+@pytest.mark.parametrize("dtype", ["c128", "c64"])
+@pytest.mark.parametrize("nst,ld", [(1, 2), (5, 6), (31, 32), (32, 32), (33, 36), (64, 72), (97, 98), (168, 168), (169, 170)])
+def test_overlap_and_orthonormalisation(cuda, dtype, nst, ld):
+    import torch
+    from hpsi import lib
+    m = _mesh()
+    rng = np.random.default_rng(nst)
+    cdt = np.complex128 if dtype == "c128" else np.complex64
+    a, b = (np.full((m.np_part, ld), np.nan, dtype=cdt) for _ in range(2))
+    for x in (a, b):
+        x[: m.np, :nst] = rng.standard_normal((m.np, nst)) + 1j * rng.standard_normal((m.np, nst))
+    dm = lib.DeviceMesh(m)
+    xa, xb = torch.from_numpy(a).to(cuda), torch.from_numpy(b).to(cuda)
+    A, B = (x[: m.np, :nst].astype(np.complex128) for x in (a, b))
+    # sums of np products of order 1 in FP64: rounding error below np * eps of
+    # the sum of magnitudes (np)
+    tol = 4 * m.np * np.finfo(float).eps * m.np * m.vol_pp
+    S = dm.dotp_matrix(xa, xb, nst=nst)
+    assert np.max(np.abs(S - m.vol_pp * (A.conj().T @ B))) <= tol
+    Sa = dm.dotp_matrix(xa, xa, nst=nst)
+    assert np.max(np.abs(Sa - m.vol_pp * (A.conj().T @ A))) <= tol
+    assert np.array_equal(Sa, Sa.conj().T)
+    dm.orthonormalize_cholesky(xa, nst=nst)
+    U = np.linalg.cholesky(m.vol_pp * (A.conj().T @ A)).conj().T
+    ref = np.linalg.solve(U.T, A.T).T
+    got = xa.cpu().numpy()
+    # the Gram matrix is well conditioned (np >> nst): a few hundred roundings
+    eps = 1e-13 if dtype == "c128" else 1e-6
+    assert np.max(np.abs(got[: m.np, :nst] - ref)) <= eps * np.max(np.abs(ref))
+    # nothing beyond the batch is touched
+    assert np.isnan(got[m.np:]).all() and np.isnan(got[:, nst:]).all()
+
+
+def test_indefinite_overlap_is_refused(cuda):
+    import torch
+    from hpsi import lib
+    m = _mesh()
+    dm = lib.DeviceMesh(m)
+    x = torch.zeros((m.np_part, 4), dtype=torch.complex128, device=cuda)
+    x[: m.np, 0] = 1.0
+    keep = x.clone()
+    with pytest.raises(lib.HpsiError):
+        dm.orthonormalize_cholesky(x, nst=2)  # a zero state
+    assert torch.equal(x, keep)
