@@ -1327,6 +1327,7 @@ hpsi_status run_pass(hpsi_hamiltonian *h, int terms, const int *src_map, const T
       shape = legacy_shape(dtype, ld);
       si = build_pass_args<T>(h, terms, src_map, in, in_ld, out, out_ld, ld, mode, psi0, psi0_ld, a_re, a_im, shape,
                               a);
+  p.phase64 = h->d_kb_phase;
       if (si) return si;
     }
   }

@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(128) bra_dmma_kernel(const ProjArgs p) {
   const int4 md = p.mat[m];  // npoints, nproj, map_off, pt_off
   const int kbeg = int((long long)md.x * blockIdx.z / gridDim.z);
   const int kend = int((long long)md.x * (blockIdx.z + 1) / gridDim.z);
+  __shared__ __align__(16) double2 sP[PHASE ? NS : 1][PHASE ? KB : 1];
   const int npts = kend - kbeg, npr = md.y;
   const int *map = p.map + md.z + kbeg;
   const double *pt = p.pt64 + md.w + (long long)kbeg * npr;
@@ -100,6 +101,15 @@ __global__ void __launch_bounds__(128) bra_dmma_kernel(const ProjArgs p) {
   double c0[2] = {0.0, 0.0}, c1[2] = {0.0, 0.0};
   const int nblk = (npts + KB - 1) / KB;
   load_map(0);
+    if constexpr (PHASE) {
+      const double2 *ph = static_cast<const double2 *>(p.phase64) + md.z + kbeg;
+      if (tid < KB) {
+        if (k0 + tid < npts)
+          cp_async16(&sP[b][tid], ph + k0 + tid);
+        else
+          sP[b][tid] = make_double2(0.0, 0.0);
+      }
+    }
   if (nblk > 0) stage(0, 0);
   cp_async_commit();
   load_map(KB);
@@ -115,7 +125,12 @@ __global__ void __launch_bounds__(128) bra_dmma_kernel(const ProjArgs p) {
     __syncthreads();
 #pragma unroll
     for (int kk = 0; kk < KB; kk += 4) {
-      const double a = double(sA[b][kk + (ln & 3)][warp * 8 + (ln >> 2)]);
+      double a = double(sA[b][kk + (ln & 3)][warp * 8 + (ln >> 2)]);
+      if constexpr (PHASE) {
+        const double other = double(sA[b][kk + (ln & 3)][(warp * 8 + (ln >> 2)) ^ 1]);
+        const double2 ph = sP[b][kk + (ln & 3)];
+        a = ((ln >> 2) & 1) ? other * ph.y + a * ph.x : a * ph.x - other * ph.y;
+      }
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
         const double bb = sB[b][kk + (ln & 3)][nt * 8 + (ln >> 2)];
@@ -151,6 +166,7 @@ __global__ void bra_reduce_kernel(const ProjArgs p, int ksplit) {
 }
 
 // SIMT bra: grid (nmat, ceil(ld2/32)); block 128 = 32 lanes x 4 point groups.
+#pragma unroll 8
 // PHASE: each gathered point is first multiplied by its projector phase
 // (lpsi = psi(map) * projector_phases, hamiltonian_elec_base_inc.F90:680-701);
 // lane pairs (2s, 2s + 1) hold one complex number, exchanged by a shuffle.
@@ -226,19 +242,12 @@ hpsi_status launch_bra(const ProjArgs &p, bool use_tensor, int ksplit, cudaStrea
   if (p.nmat == 0) return HPSI_OK;
   const long long ld2 = 2 * p.psi_ld;
   // the staged rows are copied in 16-byte pieces: FP32 needs an even width
-  if (p.phase) {  // projector phases: the SIMT kernel rotates each gathered point
-    if (p.max_nproj > 32) {
-      set_error("projector matrices with more than 32 projectors are not supported");
-      return HPSI_ERR_UNSUPPORTED;
-    }
-    dim3 grid(p.nmat, unsigned((ld2 + 31) / 32));
-    bra_simt_kernel<T, true><<<grid, 128, 0, st>>>(p);
-    HPSI_CHECK_LAUNCH();
-    return HPSI_OK;
-  }
   if (use_tensor && p.max_nproj <= NMAX && ld2 % (16 / sizeof(T)) == 0) {
     dim3 grid(p.nmat, unsigned((ld2 + LANES - 1) / LANES), ksplit);
-    bra_dmma_kernel<T><<<grid, 128, 0, st>>>(p);
+    if (p.phase)
+      bra_dmma_kernel<T, true><<<grid, 128, 0, st>>>(p);
+    else
+      bra_dmma_kernel<T, false><<<grid, 128, 0, st>>>(p);
     HPSI_CHECK_LAUNCH();
     const long long n = (long long)p.nprojections * ld2;
     bra_reduce_kernel<T><<<unsigned((n + 255) / 256), 256, 0, st>>>(p, ksplit);
@@ -250,7 +259,10 @@ hpsi_status launch_bra(const ProjArgs &p, bool use_tensor, int ksplit, cudaStrea
     return HPSI_ERR_UNSUPPORTED;
   }
   dim3 grid(p.nmat, unsigned((ld2 + 31) / 32));
-  bra_simt_kernel<T, false><<<grid, 128, 0, st>>>(p);
+  if (p.phase)
+    bra_simt_kernel<T, true><<<grid, 128, 0, st>>>(p);
+  else
+    bra_simt_kernel<T, false><<<grid, 128, 0, st>>>(p);
   HPSI_CHECK_LAUNCH();
   return HPSI_OK;
 }

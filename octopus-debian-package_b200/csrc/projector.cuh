@@ -23,6 +23,7 @@ struct ProjArgs {
   int min_npoints;       // smallest sphere (bounds the K split)
   double *partial;       // split-K partials [ksplit][nprojections][proj_ld] complex, FP64
   const void *phase = nullptr;  // per sphere point complex phase (storage type), or null
+  const void *phase64 = nullptr;  // the same phases in FP64 (tensor-core path)
 };
 
 struct KetArgs {
