@@ -46,7 +46,11 @@ __device__ __forceinline__ void dmma_m8n8k4(double &d0, double &d1, double a, do
 // scal.  T is the storage type of psi: FP32 rows are staged as stored and
 // widened to FP64 when the A fragment is read, so both precisions contract
 // in FP64 against the FP64 projector values.
-template <typename T>
+// PHASE: each gathered point is first multiplied by its projector phase
+// (lpsi = psi(map) * projector_phases, hamiltonian_elec_base_inc.F90:680-701):
+// the phases of a block are staged with it, and a fragment value is rotated
+// with its partner lane (2s, 2s + 1: one complex number) when it is read.
+template <typename T, bool PHASE>
 __global__ void __launch_bounds__(128) bra_dmma_kernel(const ProjArgs p) {
   constexpr int AP = sizeof(T) == 8 ? APAD : 40;  // 40 floats: conflict-free fragment reads
   constexpr int CPR = LANES * int(sizeof(T)) / 16;  // 16-byte copies per staged row
@@ -54,11 +58,11 @@ __global__ void __launch_bounds__(128) bra_dmma_kernel(const ProjArgs p) {
   __shared__ __align__(16) T sA[NS][KB][AP];
   __shared__ __align__(16) double sB[NS][KB][NMAX];
   const int m = blockIdx.x;
+  __shared__ __align__(16) double2 sP[PHASE ? NS : 1][PHASE ? KB : 1];
   const int l0 = blockIdx.y * LANES;
   const int4 md = p.mat[m];  // npoints, nproj, map_off, pt_off
   const int kbeg = int((long long)md.x * blockIdx.z / gridDim.z);
   const int kend = int((long long)md.x * (blockIdx.z + 1) / gridDim.z);
-  __shared__ __align__(16) double2 sP[PHASE ? NS : 1][PHASE ? KB : 1];
   const int npts = kend - kbeg, npr = md.y;
   const int *map = p.map + md.z + kbeg;
   const double *pt = p.pt64 + md.w + (long long)kbeg * npr;
@@ -96,11 +100,6 @@ __global__ void __launch_bounds__(128) bra_dmma_kernel(const ProjArgs p) {
       const bool ok = k0 + k < npts && j < npr;
       cp_async8_zfill(&sB[b][k][j], ok ? pt + (long long)(k0 + k) * npr + j : p.pt64, ok ? 8 : 0);
     }
-  };
-
-  double c0[2] = {0.0, 0.0}, c1[2] = {0.0, 0.0};
-  const int nblk = (npts + KB - 1) / KB;
-  load_map(0);
     if constexpr (PHASE) {
       const double2 *ph = static_cast<const double2 *>(p.phase64) + md.z + kbeg;
       if (tid < KB) {
@@ -111,6 +110,11 @@ __global__ void __launch_bounds__(128) bra_dmma_kernel(const ProjArgs p) {
       }
     }
   if (nblk > 0) stage(0, 0);
+  };
+
+  double c0[2] = {0.0, 0.0}, c1[2] = {0.0, 0.0};
+  const int nblk = (npts + KB - 1) / KB;
+  load_map(0);
   cp_async_commit();
   load_map(KB);
   if (nblk > 1) stage(KB, 1);
@@ -162,11 +166,11 @@ __global__ void bra_reduce_kernel(const ProjArgs p, int ksplit) {
   const int j = int(i / (2 * p.proj_ld));
   double acc = 0.0;
   for (int z = 0; z < ksplit; ++z) acc += p.partial[(long long)z * n + i];
+#pragma unroll 8
   static_cast<T *>(p.proj)[i] = T(acc * p.scal64[j]);
 }
 
 // SIMT bra: grid (nmat, ceil(ld2/32)); block 128 = 32 lanes x 4 point groups.
-#pragma unroll 8
 // PHASE: each gathered point is first multiplied by its projector phase
 // (lpsi = psi(map) * projector_phases, hamiltonian_elec_base_inc.F90:680-701);
 // lane pairs (2s, 2s + 1) hold one complex number, exchanged by a shuffle.
