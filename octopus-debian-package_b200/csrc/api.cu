@@ -8,6 +8,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 #include <queue>
 #include <vector>
 
@@ -242,19 +243,38 @@ PassShape half_chunk_shape(int dtype) {
   return s;
 }
 
+// Pass with the z history in tensor memory: 16 x 16 tiles, 128-byte chunks
+// (the last one may be partial), 4 x 4 cells per thread.
+PassShape tmem_shape(int dtype) {
+  PassShape s = blk_shape(dtype);
+  s.tmem = 1;
+  s.ty = 16;
+  s.rx = s.ry = 4;
+  return s;
+}
+
+// State chunks of a pass over ld states.
+int pass_chunks(const PassShape &s, long long ld) { return int((ld + s.sc - 1) / s.sc); }
+
 PassShape default_shape(int dtype, long long ld) {
   const PassShape b = blk_shape(dtype);
   PassShape s = ld % b.sc == 0         ? b
                 : ld % (b.sc / 2) == 0 ? half_chunk_shape(dtype)
                                        : legacy_shape(dtype, ld);
-  // experiment override: HPSI_PASS_SHAPE64 / HPSI_PASS_SHAPE32 = "sc,ry,zb,unroll,blk,rx,cplx,ty,tma,mb,mma"
+  // experiment override: HPSI_PASS_SHAPE64 / HPSI_PASS_SHAPE32 = "sc,ry,zb,unroll,blk,rx,cplx,ty,tma,mb,mma,tmem"
   const char *env = std::getenv(dtype == HPSI_C128 ? "HPSI_PASS_SHAPE64" : "HPSI_PASS_SHAPE32");
   if (env) {
-    int a = 0, b = 0, c = 0, u = 0, t = 0, x = 0, cx = -1, ty = 0, tm = 0, mb = 0, mm = 0;
-    if (std::sscanf(env, "%d,%d,%d,%d,%d,%d,%d,%d,%d,%d,%d", &a, &b, &c, &u, &t, &x, &cx, &ty, &tm, &mb, &mm) >= 2 &&
+    int a = 0, b = 0, c = 0, u = 0, t = 0, x = 0, cx = -1, ty = 0, tm = 0, mb = 0, mm = 0, tn = 0;
+    if (std::sscanf(env, "%d,%d,%d,%d,%d,%d,%d,%d,%d,%d,%d,%d", &a, &b, &c, &u, &t, &x, &cx, &ty, &tm, &mb, &mm,
+                    &tn) >= 2 &&
         a > 0 &&
-        ld % a == 0) {
-      if (t) {
+        (ld % a == 0 || (t && tn))) {
+      if (t && (tn || tm || mb)) {
+        // tensor-memory pass (its stages are handed over by mbarriers; tma: box
+        // copies of contiguous halo runs)
+        s = tmem_shape(dtype);
+        s.tma = tm ? 1 : 0;
+      } else if (t) {
         s = blk_shape(dtype);  // chunk (128 or 64 bytes), block, element, z depth and group are taken
         if (a == s.sc / 2) {
           s.sc = a;  // 64-byte chunks ride 16 x 16 tiles unless ty = 8 is given
@@ -264,8 +284,6 @@ PassShape default_shape(int dtype, long long ld) {
         if (x > 0) s.rx = x;
         if (b > 0) s.ry = b;
         if (cx >= 0) s.cplx = cx;
-        s.tma = tm ? 1 : 0;
-        s.mb = mb ? 1 : 0;
         s.mma = mm ? 1 : 0;
       } else {
         s = legacy_shape(dtype, ld);
@@ -518,6 +536,19 @@ hpsi_status hpsi_hamiltonian_create(hpsi_mesh *mesh, hpsi_hamiltonian **out) {
   // experiment override: HPSI_FUSED_DENSITY=1 fuses the density of
   // hpsi_taylor_step_density into the last pass
   if (const char *e = std::getenv("HPSI_FUSED_DENSITY")) h->fuse_density = std::atoi(e) != 0;
+  // status word of the passes' bounded waits (allocated here: a pass may first
+  // run inside a stream capture)
+  hpsi_status s = dev_alloc(reinterpret_cast<void **>(&h->d_err), sizeof(int));
+  if (s) {
+    delete h;
+    return s;
+  }
+  if (cudaMemset(h->d_err, 0, sizeof(int)) != cudaSuccess) {
+    set_error("hpsi_hamiltonian_create: cudaMemset failed");
+    dev_free(h->d_err);
+    delete h;
+    return HPSI_ERR_CUDA;
+  }
   *out = h;
   return HPSI_OK;
 }
@@ -543,6 +574,9 @@ hpsi_status hpsi_hamiltonian_destroy(hpsi_hamiltonian *h) {
   h->rhobuf.release();
   dev_free(h->d_err);
   h->lzsmall.release();
+  if (h->lz_pin) cudaFreeHost(h->lz_pin);
+  for (auto &e : h->lz_ev)
+    if (e) cudaEventDestroy(e);
   if (h->bra_stream) cudaStreamDestroy(h->bra_stream);
   if (h->pass_stream) cudaStreamDestroy(h->pass_stream);
   if (h->pass_join) cudaEventDestroy(h->pass_join);
@@ -558,6 +592,22 @@ hpsi_status hpsi_hamiltonian_destroy(hpsi_hamiltonian *h) {
   h->slab_out.release();
   h->small.release();
   delete h;
+  return HPSI_OK;
+}
+
+hpsi_status hpsi_hamiltonian::lanczos_pinned(size_t bytes) {
+  for (auto &e : lz_ev)
+    if (!e) HPSI_TRY_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  if (bytes <= lz_pin_size) return HPSI_OK;
+  if (lz_pin) {
+    // a copy queued by an earlier call may still be under way
+    for (auto &e : lz_ev) HPSI_TRY_CUDA(cudaEventSynchronize(e));
+    cudaFreeHost(lz_pin);
+  }
+  lz_pin = nullptr;
+  lz_pin_size = 0;
+  HPSI_TRY_CUDA(cudaHostAlloc(&lz_pin, bytes, cudaHostAllocDefault));
+  lz_pin_size = bytes;
   return HPSI_OK;
 }
 
@@ -586,6 +636,13 @@ void hpsi_hamiltonian::proj_free() {
   d_kidx = nullptr;
   dev_free(d_kptr);
   dev_free(d_kb_ent);
+  dev_free(d_kblk);
+  dev_free(d_pk);
+  dev_free(d_pk_f);
+  d_kblk = nullptr;
+  d_pk = nullptr;
+  d_pk_f = nullptr;
+  nkblk = 0;
   dev_free(d_kb_phase);
   dev_free(d_kb_phase_f);
   d_kb_phase = nullptr;
@@ -790,13 +847,59 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, c
       const int row = map[mat[i].z + k];
       ent[fill[row]++] = make_int4(mat[i].w + k * nprojs[i], prow[i], nprojs[i], mat[i].z + k);
     }
-  // compress to the covered rows (entries stay in matrix order per row)
-  std::vector<int> krows, kptr(1, 0);
-  for (int r = 0; r < m->np; ++r)
-    if (cnt[r + 1] > cnt[r]) {
-      krows.push_back(r);
-      kptr.push_back(cnt[r + 1]);
+  // compress to the covered rows (entries stay in matrix order per row), rows
+  // with the same list of matrices together: each list's rows in mesh order
+  std::vector<std::vector<int>> lists;
+  {
+    std::unordered_map<unsigned long long, int> by_hash;
+    for (int r = 0; r < m->np; ++r) {
+      const int e0 = cnt[r], e1 = cnt[r + 1];
+      if (e1 == e0) continue;
+      unsigned long long hash = 1469598103934665603ull;
+      for (int e = e0; e < e1; ++e) hash = (hash ^ (unsigned long long)(ent[e].y + 1)) * 1099511628211ull;
+      auto same = [&](int q) {
+        if (cnt[q + 1] - cnt[q] != e1 - e0) return false;
+        for (int e = 0; e < e1 - e0; ++e)
+          if (ent[cnt[q] + e].y != ent[e0 + e].y) return false;
+        return true;
+      };
+      for (;; ++hash) {  // (a list that shares another's hash takes the next free one)
+        auto it = by_hash.find(hash);
+        if (it == by_hash.end()) {
+          by_hash.emplace(hash, int(lists.size()));
+          lists.emplace_back(1, r);
+          break;
+        }
+        if (same(lists[it->second][0])) {
+          lists[it->second].push_back(r);
+          break;
+        }
+      }
     }
+  }
+  std::vector<int> krows, kptr(1, 0);
+  std::vector<int4> ent_row, blk;
+  std::vector<double> pk;
+  ent_row.reserve(ent.size());
+  pk.reserve(nval);
+  for (const auto &l : lists)
+    for (size_t i = 0; i < l.size(); i += 32) {
+      const int n = int(std::min<size_t>(32, l.size() - i)), ne = cnt[l[i] + 1] - cnt[l[i]];
+      blk.push_back(make_int4(int(krows.size()), n + 256 * ne, int(ent_row.size()), int(pk.size())));
+      for (int e = 0; e < ne; ++e)
+        for (int q = 0; q < n; ++q) {
+          const int4 E = ent[cnt[l[i + q]] + e];
+          pk.insert(pk.end(), pt.begin() + E.x, pt.begin() + E.x + E.z);
+        }
+      for (int q = 0; q < n; ++q) {
+        const int r = l[i + q];
+        krows.push_back(r);
+        ent_row.insert(ent_row.end(), ent.begin() + cnt[r], ent.begin() + cnt[r + 1]);
+        kptr.push_back(int(ent_row.size()));
+      }
+    }
+  ent.swap(ent_row);
+  std::vector<float> pkf(pk.begin(), pk.end());
   int minp = 1 << 30;
   for (int i = 0; i < nmat; ++i) minp = std::min(minp, int(npoints[i]));
   hpsi_status s = HPSI_OK;
@@ -826,6 +929,9 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, c
   }
   up(reinterpret_cast<void **>(&h->d_kptr), kptr.data(), kptr.size() * sizeof(int));
   up(reinterpret_cast<void **>(&h->d_kb_ent), ent.data(), ent.size() * sizeof(int4));
+  up(reinterpret_cast<void **>(&h->d_kblk), blk.data(), blk.size() * sizeof(int4));
+  up(reinterpret_cast<void **>(&h->d_pk), pk.data(), pk.size() * sizeof(double));
+  up(reinterpret_cast<void **>(&h->d_pk_f), pkf.data(), pkf.size() * sizeof(float));
   if (s) {
     h->proj_free();
     return s;
@@ -834,6 +940,7 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, c
   h->nprojections = nproj_tot;
   h->max_nproj = maxp;
   h->nk = int(krows.size());
+  h->nkblk = int(blk.size());
   h->min_npoints = minp;
   h->kb_npts = npts_tot;
   h->kb_npoints_h.assign(npoints, npoints + nmat);
@@ -909,54 +1016,84 @@ int choose_zb(const hpsi_mesh *m, int chunks, int ty) {
 }
 int choose_zb(const hpsi_mesh *m, int chunks) { return choose_zb(m, chunks, 16); }
 
+// Simulated makespan of a single-system pass (in plane steps of a CTA) for one
+// z block depth: the work units, in launch order (z band, then column-major
+// over the tiles; the state chunks of a unit consecutive), go one after another
+// to the CTA slot that frees first, as the block scheduler hands them out; a
+// unit costs its output planes + `extra`.
+static double pass_makespan(const hpsi_mesh *m, int ty, int zb, int chunks, int slots, double extra) {
+  const auto &tz = ty == 8 ? m->tile_z8 : m->tile_z;
+  const int tyn = ty == 8 ? m->tiles_y8 : m->tiles_y;
+  std::vector<int4> u;  // {band, tile x, tile y, planes}
+  for (int by = 0; by < tyn; ++by)
+    for (int bx = 0; bx < m->tiles_x; ++bx) {
+      const int2 t = tz[size_t(by) * m->tiles_x + bx];
+      if (t.y < 0) continue;
+      for (int z = t.x; z <= t.y; z += zb) u.push_back(make_int4(z / zb, bx, by, std::min(zb, t.y + 1 - z)));
+    }
+  std::stable_sort(u.begin(), u.end(), [](const int4 &a, const int4 &b) {
+    if (a.x != b.x) return a.x < b.x;
+    if (a.y != b.y) return a.y < b.y;
+    return a.z < b.z;
+  });
+  std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
+  for (int i = 0; i < std::max(1, slots); ++i) free_at.push(0.0);
+  double end = 0.0;
+  for (const int4 &w : u)
+    for (int c = 0; c < chunks; ++c) {
+      const double t = free_at.top() + double(w.w) + extra;
+      free_at.pop();
+      free_at.push(t);
+      end = std::max(end, t);
+    }
+  return end;
+}
+
 // z block depth of a single-system pass over 16 x 8 tiles (the blocked pass,
 // ctas_per_sm resident CTAs per SM): the candidate with the shortest
-// simulated makespan.  The
-// work units, in launch order (z band, then column-major over the tiles; the
-// state chunks of a unit consecutive), go one after another to the CTA slot that
-// frees first, as the block scheduler hands them out; a unit costs its output
-// planes + 8 halo planes + 4 (prologue).  Deeper blocks read fewer halo planes,
+// simulated makespan (8 halo planes and a prologue of 4 a unit).  Deeper blocks read fewer halo planes,
 // shallower ones balance the tail: on the R = 12 sphere (108 tile columns) the
 // choice is within 0.2 % of the best measured depth for 1 to 16 chunks, where
 // a fixed four-wave target was up to 9.5 % slower with one or two chunks.
-int choose_zb_single(const hpsi_mesh *m, int chunks, int ctas_per_sm) {
+std::pair<int, double> choose_zb_single(const hpsi_mesh *m, int chunks, int ctas_per_sm) {
   const int key = 4 * chunks + ctas_per_sm;
   auto it = m->zb_single.find(key);
   if (it != m->zb_single.end()) return it->second;
-  const int cands[] = {1 << 20, 96, 64, 48, 32, 24, 16};
-  int best = 16;
-  double best_t = 1e300;
-  const int slots = std::max(1, m->num_sms * ctas_per_sm);
-  for (int zb : cands) {
-    std::vector<int4> u;  // {band, tile x, tile y, planes}
-    for (int by = 0; by < m->tiles_y8; ++by)
-      for (int bx = 0; bx < m->tiles_x; ++bx) {
-        const int2 t = m->tile_z8[size_t(by) * m->tiles_x + bx];
-        if (t.y < 0) continue;
-        for (int z = t.x; z <= t.y; z += zb) u.push_back(make_int4(z / zb, bx, by, std::min(zb, t.y + 1 - z)));
-      }
-    std::stable_sort(u.begin(), u.end(), [](const int4 &a, const int4 &b) {
-      if (a.x != b.x) return a.x < b.x;
-      if (a.y != b.y) return a.y < b.y;
-      return a.z < b.z;
-    });
-    std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
-    for (int i = 0; i < slots; ++i) free_at.push(0.0);
-    double end = 0.0;
-    for (const int4 &w : u)
-      for (int c = 0; c < chunks; ++c) {
-        const double t = free_at.top() + double(w.w + 8 + 4);
-        free_at.pop();
-        free_at.push(t);
-        end = std::max(end, t);
-      }
-    if (end < best_t) {
-      best_t = end;
-      best = zb;
-    }
+  std::pair<int, double> best{16, 1e300};
+  for (int zb : {1 << 20, 96, 64, 48, 32, 24, 16}) {
+    const double t = pass_makespan(m, 8, zb, chunks, m->num_sms * ctas_per_sm, 8 + 4);
+    if (t < best.second) best = {zb, t};
   }
   m->zb_single[key] = best;
   return best;
+}
+
+// The same for the tensor-memory pass over 16 x 16 tiles, whose halo planes
+// cost less than output planes (their own cells only, no in-plane arms): the
+// candidates cut the tallest tile column into equal blocks.
+std::pair<int, double> choose_zb_tmem(const hpsi_mesh *m, int chunks) {
+  const int key = 4 * chunks;
+  auto it = m->zb_single.find(key);
+  if (it != m->zb_single.end()) return it->second;
+  int tall = 1;
+  for (auto &t : m->tile_z)
+    if (t.y >= 0) tall = std::max(tall, t.y - t.x + 1);
+  std::pair<int, double> best{1 << 20, 1e300};
+  for (int n = 1; n <= 16 && (tall + n - 1) / n >= 4; ++n) {
+    const int zb = n == 1 ? 1 << 20 : (tall + n - 1) / n;
+    const double t = pass_makespan(m, 16, zb, chunks, m->num_sms, TMEM_UNIT_EXTRA);
+    if (t < best.second) best = {zb, t};
+  }
+  m->zb_single[key] = best;
+  return best;
+}
+
+// Whether the tensor-memory pass is expected to be faster than the pass
+// `other` would choose for this width.
+bool prefer_tmem(const hpsi_mesh *m, int dtype, long long ld, const PassShape &other) {
+  (void)dtype;
+  (void)other;
+  return m != nullptr && ld > 0;
 }
 
 // z block depth of a single-system pass of a shape: the simulated choice for
@@ -965,8 +1102,9 @@ int choose_zb_single(const hpsi_mesh *m, int chunks, int ctas_per_sm) {
 int pass_zb(const hpsi_mesh *m, const PassShape &sh, int dtype, int chunks) {
   const int ty = sh.blk ? sh.ty : 16;
   const PassShape b = blk_shape(dtype);
-  if (sh.blk && ty == 8 && sh.sc == b.sc) return choose_zb_single(m, chunks, 1);
-  if (sh.blk && ty == 8 && sh.sc == b.sc / 2 && sh.rx == 1 && sh.ry == 4) return choose_zb_single(m, chunks, 2);
+  if (sh.tmem) return choose_zb_tmem(m, chunks).first;
+  if (sh.blk && ty == 8 && sh.sc == b.sc) return choose_zb_single(m, chunks, 1).first;
+  if (sh.blk && ty == 8 && sh.sc == b.sc / 2 && sh.rx == 1 && sh.ry == 4) return choose_zb_single(m, chunks, 2).first;
   return choose_zb(m, chunks, ty);
 }
 
@@ -1004,6 +1142,7 @@ hpsi_status mesh_items(hpsi_mesh *m, int zb, int ty, const int4 **items, int *ni
     if (s) return s;
     if (!v.empty()) HPSI_TRY_CUDA(cudaMemcpy(d, v.data(), v.size() * sizeof(int4), cudaMemcpyHostToDevice));
     it = m->items.emplace(key, std::make_pair(d, int(v.size()))).first;
+    m->items_h[key] = std::move(v);
   }
   *items = it->second.first;
   *nitems = it->second.second;
@@ -1082,46 +1221,27 @@ hpsi_status mesh_items_part(hpsi_mesh *m, int zb, int ty, int part, const int4 *
   return HPSI_OK;
 }
 
-// Per (16 x 8 tile column, cell plane) of the padded box, bit s set when star
-// segment s of the tile's halo plane (star cells 8 s .. 8 s + 7 in the order
-// of the blocked pass: 4 rows of 16 above, 8 rows of 24, 4 rows of 16 below,
-// HAL = 4) maps to eight consecutive rows of the batch through `src`.
+// Per (16 x 16 tile column, cell plane) of the padded box, bit s set when
+// segment s of the tile's halo plane over its own columns (24 rows of two
+// segments of eight cells, HAL = 4) maps to eight consecutive rows of the batch
+// through `src`.
 static std::vector<unsigned long long> seg_mask_table(const hpsi_mesh *m, const std::vector<int> &src) {
   const CellBox &B = m->box;
-  const int HAL = 4, TX = 16, TY = 8, HX = TX + 2 * HAL;
-  std::vector<unsigned long long> t(size_t(m->tiles_y8) * m->tiles_x * B.NZ, 0ull);
-  for (int by = 0; by < m->tiles_y8; ++by)
-    for (int bx = 0; bx < m->tiles_x; ++bx) {
-      const int cx0 = HAL + bx * TX, cy0 = HAL + by * TY;
+  const int HAL = 4, TX = 16, TY = 16;
+  std::vector<unsigned long long> t(size_t(m->tiles_y) * m->tiles_x * B.NZ, 0ull);
+  for (int by = 0; by < m->tiles_y; ++by)
+    for (int bx = 0; bx < m->tiles_x; ++bx)
       for (int q = 0; q < B.NZ; ++q) {
         unsigned long long mask = 0;
-        for (int sgi = 0; sgi < 40; ++sgi) {
-          int first = -1;
-          bool ok = true;
-          for (int k = 0; k < 8 && ok; ++k) {
-            int i = 8 * sgi + k, hx, hy;  // star cell -> halo-plane coordinates
-            if (i < HAL * TX) {
-              hy = i / TX;
-              hx = HAL + i % TX;
-            } else if ((i -= HAL * TX) < TY * HX) {
-              hy = HAL + i / HX;
-              hx = i % HX;
-            } else {
-              i -= TY * HX;
-              hy = HAL + TY + i / TX;
-              hx = HAL + i % TX;
-            }
-            const int x = cx0 - HAL + hx, y = cy0 - HAL + hy;
-            const int r = (x < 0 || y < 0 || x >= B.NX || y >= B.NY) ? -1
-                                                                      : src[(size_t(q) * B.NY + y) * B.NX + x];
-            if (k == 0) first = r;
-            ok = r >= 0 && r == first + k;
-          }
-          if (ok) mask |= 1ull << sgi;
+        for (int s = 0; s < 2 * (TY + 2 * HAL); ++s) {
+          const int y = by * TY + s / 2, x0 = HAL + bx * TX + 8 * (s % 2);
+          const int *row = src.data() + (size_t(q) * B.NY + y) * B.NX + x0;
+          bool ok = row[0] >= 0;
+          for (int k = 1; k < 8 && ok; ++k) ok = row[k] == row[0] + k;
+          if (ok) mask |= 1ull << s;
         }
         t[(size_t(by) * m->tiles_x + bx) * B.NZ + q] = mask;
       }
-    }
   return t;
 }
 
@@ -1148,14 +1268,8 @@ hpsi_status prepare_tma(hpsi_hamiltonian *h, const int *src_map, long long in_ro
     HPSI_TRY_CUDA(cudaMemcpy(d, t.data(), t.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice));
     it = m->seg_masks.emplace(src_map, d).first;
   }
-  if (!h->d_err) {
-    hpsi_status s = dev_alloc(reinterpret_cast<void **>(&h->d_err), sizeof(int));
-    if (s) return s;
-    HPSI_TRY_CUDA(cudaMemset(h->d_err, 0, sizeof(int)));
-  }
   a.seg_mask = it->second;
   a.seg_tiles_x = m->tiles_x;
-  a.err = h->d_err;
   return HPSI_OK;
 }
 
@@ -1169,6 +1283,7 @@ void base_pass_args(const hpsi_hamiltonian *h, int terms, const int *src_map, Pa
   a.per_inner = m->d_per_inner;
   a.col_z = m->d_col_z;
   a.np = m->np;
+  a.err = h->d_err;
   if ((terms & HPSI_TERM_KINETIC) && h->have_kinetic) {
     std::memcpy(a.wx, h->wx, sizeof(a.wx));
     std::memcpy(a.wy, h->wy, sizeof(a.wy));
@@ -1212,6 +1327,7 @@ hpsi_status run_bra(hpsi_hamiltonian *h, const T *psi, long long ld, T *proj, cu
   p.phase = h->d_kb_phase ? (sizeof(T) == 8 ? static_cast<const void *>(h->d_kb_phase)
                                             : static_cast<const void *>(h->d_kb_phase_f))
                           : nullptr;
+  p.phase64 = h->d_kb_phase;
   const int ksplit = bra_ksplit(p, h->mesh->num_sms);
   hpsi_status s = h->bra_partial.ensure(size_t(ksplit) * h->nprojections * ld * 2 * sizeof(double));
   if (s) return s;
@@ -1229,6 +1345,10 @@ hpsi_status run_ket(hpsi_hamiltonian *h, const T *proj, long long ld, int nst, T
   k.rho_w = rho_w;
   k.row_blocks = row_blocks;
   k.nk = h->nk;
+  k.nblk = h->nkblk;
+  k.blk = h->d_kblk;
+  k.pk = sizeof(T) == 8 ? static_cast<const void *>(h->d_pk) : static_cast<const void *>(h->d_pk_f);
+  k.max_nproj = h->max_nproj;
   k.krows = h->d_krows;
   k.kptr = h->d_kptr;
   k.ent = h->d_kb_ent;
@@ -1252,11 +1372,17 @@ hpsi_status run_ket(hpsi_hamiltonian *h, const T *proj, long long ld, int nst, T
   return launch_ket<T>(k, st);
 }
 
-// Shape of the fused pass for a batch: the autotuned one when it matches.
+// Shape of the fused pass for a batch: the autotuned one when it matches, else
+// the tensor-memory pass or the default of the width, whichever is expected to
+// be faster on this mesh.
 PassShape pass_shape(const hpsi_hamiltonian *h, int dtype, long long ld) {
   const auto &t = h->tuned[dtype == HPSI_C128 ? 0 : 1];
-  if (t.ld == ld && !std::getenv(dtype == HPSI_C128 ? "HPSI_PASS_SHAPE64" : "HPSI_PASS_SHAPE32")) return t.shape;
-  return default_shape(dtype, ld);
+  if (std::getenv(dtype == HPSI_C128 ? "HPSI_PASS_SHAPE64" : "HPSI_PASS_SHAPE32")) return default_shape(dtype, ld);
+  if (t.ld == ld) return t.shape;
+  const PassShape s = default_shape(dtype, ld);
+  const bool rows16 = dtype == HPSI_C128 || ld % 2 == 0;  // 16-byte rows
+  if (rows16 && prefer_tmem(h->mesh, dtype, ld, s)) return tmem_shape(dtype);
+  return s;
 }
 
 // Arguments of one fused pass (no launch).  in: rows to stencil; out: result
@@ -1277,7 +1403,8 @@ hpsi_status build_pass_args(hpsi_hamiltonian *h, int terms, const int *src_map, 
   a.psi0_ld = psi0_ld;
   a.a_re = a_re;
   a.a_im = a_im;
-  a.chunks = int(ld / shape.sc);
+  a.lanes = int(2 * ld);
+  a.chunks = pass_chunks(shape, ld);
   const int ty = shape.blk ? shape.ty : 16;
   a.zb = shape.zb > 0 ? shape.zb : pass_zb(h->mesh, shape, sizeof(T) == 8 ? HPSI_C128 : HPSI_C64, a.chunks);
   return mesh_items(h->mesh, a.zb, ty, &a.items, &a.nitems);
@@ -1323,11 +1450,10 @@ hpsi_status run_pass(hpsi_hamiltonian *h, int terms, const int *src_map, const T
     PassArgs chk = a;
     if (obs_partial) chk.obs = obs_partial;
     if (obs_partial && !psi0) chk.psi0 = in, chk.psi0_ld = in_ld;
-    if (!blk_pass_eligible<T>(chk, ld, shape.sc)) {
+    if (!blk_pass_eligible<T>(chk, ld, shape.tmem ? 0 : shape.sc)) {
       shape = legacy_shape(dtype, ld);
       si = build_pass_args<T>(h, terms, src_map, in, in_ld, out, out_ld, ld, mode, psi0, psi0_ld, a_re, a_im, shape,
                               a);
-  p.phase64 = h->d_kb_phase;
       if (si) return si;
     }
   }
@@ -1447,7 +1573,7 @@ size_t obs_partial_bytes(hpsi_hamiltonian *h, long long ld) {
     const int4 *items;
     int nitems = 0;
     const int ty = sh.blk ? sh.ty : 16;
-    const int zb = sh.zb > 0 ? sh.zb : pass_zb(h->mesh, sh, dt, int(ld / sh.sc));
+    const int zb = sh.zb > 0 ? sh.zb : pass_zb(h->mesh, sh, dt, pass_chunks(sh, ld));
     if (mesh_items(h->mesh, zb, ty, &items, &nitems) == HPSI_OK)
       n = std::max(n, size_t(nitems));
     const PassShape lg = legacy_shape(dt, ld);
@@ -1861,7 +1987,7 @@ hpsi_status hpsi_taylor_step_density(hpsi_hamiltonian *h, hpsi_batch *psi, doubl
   if (s) return s;
   if (R.fused) {
     const bool kb = h->nmat > 0 && h->nk > 0;
-    rho_finalize_kernel<<<(m->np + 255) / 256, 256, 0, st>>>(R.part, int(ld / sh.sc), R.ket, kxb, h->nk,
+    rho_finalize_kernel<<<(m->np + 255) / 256, 256, 0, st>>>(R.part, pass_chunks(sh, ld), R.ket, kxb, h->nk,
                                                              kb ? h->d_kidx : nullptr, m->np, accumulate ? 1 : 0,
                                                              rho);
     g_launches++;

@@ -59,8 +59,10 @@ struct hpsi_mesh {
   long long column_planes = 0;          // sum of the tile z extents
   // work list per (z block depth, tile height): key 2 * zb + (height == 8)
   std::map<int, std::pair<int4 *, int>> items;
-  // z block depth of a single-system blocked pass, per state chunk count
-  mutable std::map<int, int> zb_single;
+  std::map<int, std::vector<int4>> items_h;  // the same lists on the host
+  // z block depth of a single-system pass and its simulated makespan, per state
+  // chunk count and kernel (4 * chunks + resident CTAs, 0: tensor-memory pass)
+  mutable std::map<int, std::pair<int, double>> zb_single;
   // domain-parallel meshes: rows [ghost_first, ghost_first + ghost_count) hold
   // other partitions' points; work lists split into the tiles/planes whose
   // stencil reads no ghost row (part 1) and the rest (part 2), per (zb, ty)
@@ -95,6 +97,12 @@ struct hpsi_hamiltonian {
   int *d_krows = nullptr, *d_kptr = nullptr;
   int *d_kidx = nullptr;  // per inner row: its index among the covered rows, or -1
   int4 *d_kb_ent = nullptr;
+  // blocks of covered rows with the same list of matrices (KetArgs::blk) and
+  // their projector values in block order
+  int nkblk = 0;
+  int4 *d_kblk = nullptr;
+  double *d_pk = nullptr;
+  float *d_pk_f = nullptr;
   // projector phases (k != 0): one complex number per sphere point, or null
   long long kb_npts = 0;
   std::vector<int> kb_npoints_h;  // sphere points of each matrix
@@ -129,6 +137,11 @@ struct hpsi_hamiltonian {
   // workspaces
   hpsi::Workspace u[2], projbuf, bra_partial, obsbuf, ketobs, small, tdbuf, adjbuf;
   hpsi::Workspace lzbuf, lzsmall;
+  // pinned copies of an iteration's norms and overlaps, and their events
+  void *lz_pin = nullptr;
+  size_t lz_pin_size = 0;
+  cudaEvent_t lz_ev[2] = {nullptr, nullptr};
+  hpsi_status lanczos_pinned(size_t bytes);
   hpsi::Workspace vstage;  // host potential staged for hpsi_hamiltonian_update_vloc
   hpsi::Workspace adjstep, vjpbuf;  // per-step adjoint scratch, field VJP partials
   hpsi::Workspace rhobuf;  // fused density: weights, pass and ket partials

@@ -13,7 +13,10 @@
 // The autotuner times the candidate pass shapes (state chunk width, z block
 // depth) of a Hamiltonian on scratch batches and keeps the fastest.
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
+#include <functional>
+#include <queue>
 #include <string>
 #include <vector>
 
@@ -24,6 +27,8 @@
 namespace hpsi {
 
 PassShape pass_shape(const hpsi_hamiltonian *h, int dtype, long long ld);
+PassShape tmem_shape(int dtype);
+int pass_chunks(const PassShape &s, long long ld);
 PassShape default_shape(int dtype, long long ld);
 int pass_sc(int dtype, long long ld);
 int choose_zb(const hpsi_mesh *m, int chunks, int ty);
@@ -63,11 +68,14 @@ struct hpsi_group {
     int first = 0, end = 0;
     int4 *d_units = nullptr;
     int nunits = 0;
+    int *d_first = nullptr;  // tensor-memory pass: first unit of each CTA
+    int grid = 0;
   };
   std::vector<Launch> launches;
   long long built_ld_sig = -1;  // signature of the batch widths the units were built for
   int built_dtype = -1, sc = 0;
   bool blk = false;             // every width fits the blocked pass's chunk
+  bool tmem = false;            // tensor-memory pass (any widths of 16-byte rows)
   std::vector<hpsi::PassShape> shapes;
   int *d_counter = nullptr;     // one counter per launch sub-group
   cudaStream_t cap = nullptr;
@@ -83,8 +91,93 @@ struct hpsi_group {
 namespace hpsi {
 
 static void group_free_units(hpsi_group *g) {
-  for (auto &l : g->launches) dev_free(l.d_units);
+  for (auto &l : g->launches) {
+    dev_free(l.d_units);
+    dev_free(l.d_first);
+  }
   g->launches.clear();
+}
+
+// Unit lists of the tensor-memory pass: the units of a launch, most expensive
+// first, go to the CTA with the least work so far (one CTA per SM), each CTA's
+// units consecutive in the list.  The z block depth is the common number of
+// blocks per tile column with the shortest such schedule (a unit costs its
+// output planes + TMEM_UNIT_EXTRA).
+static hpsi_status group_build_tmem(hpsi_group *g, int dtype, const std::vector<long long> &ld, long long sig) {
+  const int n = int(g->hams.size());
+  const PassShape shape = tmem_shape(dtype);
+  g->blk = false;
+  g->sc = shape.sc;
+  auto depth = [&](int s, int blocks) {
+    int tall = 1;
+    for (auto &t : g->hams[s]->mesh->tile_z)
+      if (t.y >= 0) tall = std::max(tall, t.y - t.x + 1);
+    return blocks == 1 ? 1 << 20 : std::max(4, (tall + blocks - 1) / blocks);
+  };
+  for (int first = 0; first < n; first += GROUP_MAX) {
+    hpsi_group::Launch L;
+    L.first = first;
+    L.end = std::min(n, first + GROUP_MAX);
+    double best_t = 1e300;
+    int best_blocks = 1;
+    std::vector<std::vector<int4>> plan;
+    for (int blocks = 1; blocks <= 8; ++blocks) {
+      std::vector<std::pair<double, int4>> units;
+      for (int s = L.first; s < L.end; ++s) {
+        const hpsi_mesh *m = g->hams[s]->mesh;
+        const int zb = depth(s, blocks), chunks = pass_chunks(shape, ld[s]);
+        const int4 *items;
+        int nitems = 0;
+        hpsi_status st = mesh_items(g->hams[s]->mesh, zb, 16, &items, &nitems);
+        if (st) return st;
+        // the list on the device, in its own order, from the same construction
+        const std::vector<int4> &hi = m->items_h.at(2 * zb);
+        for (int i = 0; i < nitems; ++i)
+          for (int c = 0; c < chunks; ++c)
+            units.push_back({double(hi[i].w - hi[i].z) + TMEM_UNIT_EXTRA, make_int4(s - L.first, i, c, 0)});
+      }
+      std::stable_sort(units.begin(), units.end(), [](const auto &a, const auto &b) { return a.first > b.first; });
+      const int grid = std::max(1, std::min<int>(g->num_sms, int(units.size())));
+      std::vector<std::vector<int4>> lists(grid);
+      std::priority_queue<std::pair<double, int>, std::vector<std::pair<double, int>>, std::greater<std::pair<double, int>>> q;
+      for (int i = 0; i < grid; ++i) q.push({0.0, i});
+      double end = 0.0;
+      for (auto &u : units) {
+        auto [t, i] = q.top();
+        q.pop();
+        t += u.first;
+        lists[i].push_back(u.second);
+        end = std::max(end, t);
+        q.push({t, i});
+      }
+      if (end < best_t) {
+        best_t = end;
+        best_blocks = blocks;
+        plan.swap(lists);
+      }
+    }
+    for (int s = L.first; s < L.end; ++s) {
+      g->shapes[s] = shape;
+      g->shapes[s].zb = depth(s, best_blocks);
+    }
+    std::vector<int4> u;
+    std::vector<int> fst(1, 0);
+    for (auto &l : plan) {
+      u.insert(u.end(), l.begin(), l.end());
+      fst.push_back(int(u.size()));
+    }
+    L.nunits = int(u.size());
+    L.grid = int(plan.size());
+    hpsi_status st = dev_alloc(reinterpret_cast<void **>(&L.d_units), std::max<size_t>(1, u.size()) * sizeof(int4));
+    if (!st) st = dev_alloc(reinterpret_cast<void **>(&L.d_first), fst.size() * sizeof(int));
+    if (st) return st;
+    g->launches.push_back(L);
+    if (!u.empty()) HPSI_TRY_CUDA(cudaMemcpy(L.d_units, u.data(), u.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    HPSI_TRY_CUDA(cudaMemcpy(L.d_first, fst.data(), fst.size() * sizeof(int), cudaMemcpyHostToDevice));
+  }
+  g->built_ld_sig = sig;
+  g->built_dtype = dtype;
+  return HPSI_OK;
 }
 
 // Build the per-launch unit lists for batches of widths ld[s].
@@ -95,6 +188,11 @@ static hpsi_status group_build(hpsi_group *g, int dtype, const std::vector<long 
   group_free_units(g);
   const int n = int(g->hams.size());
   g->shapes.assign(n, PassShape{});
+  // the tensor-memory pass takes any width of 16-byte rows; the shape overrides
+  // keep the forms below
+  g->tmem = !std::getenv(dtype == HPSI_C128 ? "HPSI_PASS_SHAPE64" : "HPSI_PASS_SHAPE32");
+  for (int s = 0; s < n; ++s) g->tmem = g->tmem && (dtype == HPSI_C128 || ld[s] % 2 == 0);
+  if (g->tmem) return group_build_tmem(g, dtype, ld, sig);
   // the blocked pass when every width is a multiple of its chunk
   const PassShape bs = blk_shape(dtype);
   g->blk = true;
@@ -104,7 +202,7 @@ static hpsi_status group_build(hpsi_group *g, int dtype, const std::vector<long 
     for (int s = 0; s < n; ++s)
       if (!g->shapes[s].blk || g->shapes[s].rx != g->shapes[0].rx || g->shapes[s].ry != g->shapes[0].ry ||
           g->shapes[s].cplx != g->shapes[0].cplx || g->shapes[s].unroll != g->shapes[0].unroll ||
-          g->shapes[s].sc != g->shapes[0].sc || g->shapes[s].ty != g->shapes[0].ty || ld[s] % g->shapes[s].sc) {
+          g->shapes[s].tmem != g->shapes[0].tmem || g->shapes[s].sc != g->shapes[0].sc || g->shapes[s].ty != g->shapes[0].ty || ld[s] % g->shapes[s].sc) {
         g->blk = false;
         break;
       }
@@ -228,12 +326,14 @@ static hpsi_status group_step(hpsi_group *g, const std::vector<T *> &psi, const 
       }
       ga.units = L.d_units;
       ga.nunits = L.nunits;
+      ga.first = L.d_first;
       ga.counter = g->d_counter + li;
-      HPSI_TRY_CUDA(cudaMemsetAsync(ga.counter, 0, sizeof(int), st));
+      if (!g->tmem) HPSI_TRY_CUDA(cudaMemsetAsync(ga.counter, 0, sizeof(int), st));
       ProfScope prof(sizeof(T) == 8 ? "group_pass_fp64" : "group_pass_fp32", st);
       const PassShape &s0 = g->shapes[L.first];
-      hpsi_status r = g->blk ? launch_pass_blk_group<T>(ga, s0, g->num_sms, st)
-                             : launch_pass_group<T>(ga, g->sc, g->num_sms, st);
+      hpsi_status r = g->tmem  ? launch_pass_tmem_group<T>(ga, L.grid, st)
+                      : g->blk ? launch_pass_blk_group<T>(ga, s0, g->num_sms, st)
+                               : launch_pass_group<T>(ga, g->sc, g->num_sms, st);
       if (r) return r;
     }
     r0 = fork();
@@ -381,14 +481,6 @@ static hpsi_status autotune_t(hpsi_hamiltonian *h, int dtype, long long ld, cuda
       b4.ty = 8;
       blocks.push_back(b4);
     }
-    if (ld % b0.sc == 0) {
-      PassShape bt = b0;  // the default block with the TMA fill of contiguous halo runs
-      bt.tma = 1;
-      blocks.push_back(bt);
-      PassShape bm = b0;  // the default block with the mbarrier hand-over of the stages
-      bm.mb = 1;
-      blocks.push_back(bm);
-    }
     for (const auto &b : blocks)
       for (int zb : {0, 16, 32, 48, 64, 1 << 20}) {
         PassShape c = b;
@@ -396,6 +488,15 @@ static hpsi_status autotune_t(hpsi_hamiltonian *h, int dtype, long long ld, cuda
         cands.push_back(c);
       }
   }
+  // tensor-memory pass, per-thread and TMA fill
+  if (dtype == HPSI_C128 || ld % 2 == 0)
+    for (int tma : {0, 1})
+      for (int zb : {0, 8, 16, 32, 64, 1 << 20}) {
+        PassShape c = tmem_shape(dtype);
+        c.tma = tma;
+        c.zb = zb;
+        cands.push_back(c);
+      }
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -503,7 +604,7 @@ hpsi_status hpsi_autotune(hpsi_hamiltonian *h, int32_t dtype, int64_t ld, int32_
   if (r) return r;
   const auto &t = h->tuned[dtype == HPSI_C128 ? 0 : 1];
   if (shape_out) {
-    shape_out[0] = t.shape.sc;
+    shape_out[0] = int(std::min<long long>(t.shape.sc, ld));  // (the last chunk may be partial)
     shape_out[1] = t.shape.ry;
     shape_out[2] = t.shape.zb;
     shape_out[3] = t.shape.ty;

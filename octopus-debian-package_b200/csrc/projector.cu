@@ -57,8 +57,8 @@ __global__ void __launch_bounds__(128) bra_dmma_kernel(const ProjArgs p) {
   constexpr int NS = 3;  // staged blocks: two in flight while one is contracted
   __shared__ __align__(16) T sA[NS][KB][AP];
   __shared__ __align__(16) double sB[NS][KB][NMAX];
-  const int m = blockIdx.x;
   __shared__ __align__(16) double2 sP[PHASE ? NS : 1][PHASE ? KB : 1];
+  const int m = blockIdx.x;
   const int l0 = blockIdx.y * LANES;
   const int4 md = p.mat[m];  // npoints, nproj, map_off, pt_off
   const int kbeg = int((long long)md.x * blockIdx.z / gridDim.z);
@@ -109,12 +109,12 @@ __global__ void __launch_bounds__(128) bra_dmma_kernel(const ProjArgs p) {
           sP[b][tid] = make_double2(0.0, 0.0);
       }
     }
-  if (nblk > 0) stage(0, 0);
   };
 
   double c0[2] = {0.0, 0.0}, c1[2] = {0.0, 0.0};
   const int nblk = (npts + KB - 1) / KB;
   load_map(0);
+  if (nblk > 0) stage(0, 0);
   cp_async_commit();
   load_map(KB);
   if (nblk > 1) stage(KB, 1);
@@ -165,8 +165,8 @@ __global__ void bra_reduce_kernel(const ProjArgs p, int ksplit) {
   if (i >= n) return;
   const int j = int(i / (2 * p.proj_ld));
   double acc = 0.0;
-  for (int z = 0; z < ksplit; ++z) acc += p.partial[(long long)z * n + i];
 #pragma unroll 8
+  for (int z = 0; z < ksplit; ++z) acc += p.partial[(long long)z * n + i];
   static_cast<T *>(p.proj)[i] = T(acc * p.scal64[j]);
 }
 

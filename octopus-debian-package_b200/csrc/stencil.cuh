@@ -48,9 +48,10 @@ struct PassArgs {
   double *rho_part;       // [chunks][np], or null
   const double *rho_w;    // per state weight (ld entries)
 
-  // TMA fill of the blocked pass: per (16 x 8 tile, cell plane) a mask whose
-  // bit s marks star segment s (eight consecutive halo cells of one row) as
-  // eight consecutive rows of the input; [tiles_y][seg_tiles_x][NZ]
+  // TMA fill of the tensor-memory pass: per (16 x 16 tile, cell plane) a mask
+  // whose bit s marks segment s (eight consecutive cells of one halo row over
+  // the tile's columns) as eight consecutive rows of the input;
+  // [tiles_y][seg_tiles_x][NZ]
   const unsigned long long *seg_mask;
   int seg_tiles_x;
   int *err;               // device status word of bounded waits (HPSI_ERR_TIMEOUT), or null
@@ -58,7 +59,8 @@ struct PassArgs {
   const int2 *col_z;      // per (y, x) cell column: {first, last} z of its inner points
   const int4 *items;      // work items {tile x, tile y, first plane, end plane}
   int nitems;
-  int chunks;             // state chunks per item (ld / SC)
+  int lanes;              // reals per row the pass covers (2 ld)
+  int chunks;             // state chunks per item (ld / SC; tensor-memory pass: rounded up)
   int zb;                 // output planes per item (at most)
 };
 
@@ -71,9 +73,9 @@ struct PassShape {
   int blk = 0;     // 1: register-blocked real-lane pass (sc = its chunk, tiles 16 x 8)
   int rx = 0;      // blocked pass: cells per thread along x (ry along y)
   int cplx = 0;    // blocked pass: 1 = a thread owns a complex state, 0 = one real lane
-  int tma = 0;     // blocked pass: contiguous halo runs filled by TMA box copies
-  int mb = 0;      // blocked pass: stages handed over by mbarriers (split arrive / wait)
+  int tma = 0;     // tensor-memory pass: contiguous halo runs filled by TMA box copies
   int mma = 0;     // FP64 blocked pass with the x and y arms on the FP64 tensor cores (DMMA)
+  int tmem = 0;    // blocked pass with the z history in tensor memory (16 x 16 tiles, 4 x 4 cells)
 };
 
 // Launch the fused pass for a storage type (double -> FP64, float -> FP32).
@@ -90,6 +92,7 @@ struct GroupArgs {
   const int4 *units;   // {system, item, chunk, -}, most expensive first
   int nunits;
   int *counter;        // zeroed before every launch
+  const int *first;    // tensor-memory pass: first unit of each CTA (grid + 1 entries)
 };
 
 // One persistent launch of the fused pass over several systems (no

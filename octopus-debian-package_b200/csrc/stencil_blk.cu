@@ -16,8 +16,7 @@
 // stored as zeros and Bloch-phase images are multiplied on load.  The load
 // map of each plane and the output rows four planes below travel in a side
 // ring two stage rounds ahead of the data, so every gather knows its rows
-// when it is issued.  One __syncthreads per plane (or, PassShape::mb, a full
-// and an empty mbarrier per stage: a warp may run a plane ahead).
+// when it is issued.  One __syncthreads per plane.
 //
 // A TMA tile::gather4 fill of the same 128-byte chunks (one producer warp,
 // mbarrier hand-over) was measured 3x slower than this form on the same
@@ -38,26 +37,16 @@ using namespace blk;
 
 namespace blk {
 // instantiated in stencil_blk_shapes.cu, one object per shape
-extern template hpsi_status launch_blk_u<double, 9, 2, 2, false, 8, 128>(const PassArgs &, const CUtensorMap *, cudaStream_t);
-extern template hpsi_status launch_blk_u<double, 3, 2, 2, false, 8, 128>(const PassArgs &, const CUtensorMap *, cudaStream_t);
-extern template hpsi_status launch_blk_u<double, 9, 2, 2, true, 8, 128>(const PassArgs &, const CUtensorMap *, cudaStream_t);
-extern template hpsi_status launch_blk_u<double, 9, 1, 4, false, 8, 64>(const PassArgs &, const CUtensorMap *, cudaStream_t);
-extern template hpsi_status launch_blk_u<double, 9, 1, 4, false, 16, 64>(const PassArgs &, const CUtensorMap *, cudaStream_t);
-extern template hpsi_status launch_blk_u<float, 9, 2, 2, true, 8, 128>(const PassArgs &, const CUtensorMap *, cudaStream_t);
-extern template hpsi_status launch_blk_u<float, 3, 2, 2, true, 8, 128>(const PassArgs &, const CUtensorMap *, cudaStream_t);
-extern template hpsi_status launch_blk_u<float, 1, 2, 4, false, 8, 128>(const PassArgs &, const CUtensorMap *, cudaStream_t);
-extern template hpsi_status launch_blk_u<float, 9, 1, 4, true, 8, 64>(const PassArgs &, const CUtensorMap *, cudaStream_t);
-extern template hpsi_status launch_blk_u<float, 9, 1, 4, true, 16, 64>(const PassArgs &, const CUtensorMap *, cudaStream_t);
-extern template hpsi_status launch_blk_u<double, 9, 2, 2, false, 8, 128, true>(const PassArgs &, const CUtensorMap *,
-                                                                               cudaStream_t);
-extern template hpsi_status launch_blk_u<float, 9, 2, 2, true, 8, 128, true>(const PassArgs &, const CUtensorMap *,
-                                                                             cudaStream_t);
-extern template hpsi_status launch_blk_u<double, 9, 2, 2, false, 8, 128, false, true>(const PassArgs &,
-                                                                                      const CUtensorMap *,
-                                                                                      cudaStream_t);
-extern template hpsi_status launch_blk_u<float, 9, 2, 2, true, 8, 128, false, true>(const PassArgs &,
-                                                                                    const CUtensorMap *,
-                                                                                    cudaStream_t);
+extern template hpsi_status launch_blk_u<double, 9, 2, 2, false, 8, 128>(const PassArgs &, cudaStream_t);
+extern template hpsi_status launch_blk_u<double, 3, 2, 2, false, 8, 128>(const PassArgs &, cudaStream_t);
+extern template hpsi_status launch_blk_u<double, 9, 2, 2, true, 8, 128>(const PassArgs &, cudaStream_t);
+extern template hpsi_status launch_blk_u<double, 9, 1, 4, false, 8, 64>(const PassArgs &, cudaStream_t);
+extern template hpsi_status launch_blk_u<double, 9, 1, 4, false, 16, 64>(const PassArgs &, cudaStream_t);
+extern template hpsi_status launch_blk_u<float, 9, 2, 2, true, 8, 128>(const PassArgs &, cudaStream_t);
+extern template hpsi_status launch_blk_u<float, 3, 2, 2, true, 8, 128>(const PassArgs &, cudaStream_t);
+extern template hpsi_status launch_blk_u<float, 1, 2, 4, false, 8, 128>(const PassArgs &, cudaStream_t);
+extern template hpsi_status launch_blk_u<float, 9, 1, 4, true, 8, 64>(const PassArgs &, cudaStream_t);
+extern template hpsi_status launch_blk_u<float, 9, 1, 4, true, 16, 64>(const PassArgs &, cudaStream_t);
 }  // namespace blk
 
 
@@ -86,7 +75,7 @@ int blk_chunk_states() {
 
 template <typename T>
 bool blk_pass_eligible(const PassArgs &a, long long ld, int sc) {
-  if (ld % sc != 0) return false;
+  if (sc > 0 && ld % sc != 0) return false;
   if (reinterpret_cast<uintptr_t>(a.in) % 16 != 0 || reinterpret_cast<uintptr_t>(a.out) % 16 != 0) return false;
   if ((a.mode == PASS_HORNER || a.obs) && reinterpret_cast<uintptr_t>(a.psi0) % 16 != 0) return false;
   if ((2 * a.in_ld * sizeof(T)) % 16 != 0 || (2 * a.psi0_ld * sizeof(T)) % 16 != 0) return false;
@@ -142,21 +131,15 @@ template <typename T>
 hpsi_status launch_pass_blk(const PassArgs &a, const PassShape &s, cudaStream_t st) {
   if (a.nitems == 0) return HPSI_OK;
   const int cb = shape_cb<T>(s), g = s.unroll;
-  if (s.tma) {
-    // TMA fill: the default cell blocks (FP64 2 x 2 real lanes, FP32 2 x 2
-    // complex states), 16 x 8 tiles, 128-byte chunks, no Bloch phase
-    if (s.ty != 8 || cb != 128 || s.rx != 2 || s.ry != 2 || g != 9 || a.phase_corr || !a.seg_mask ||
-        s.cplx != (sizeof(T) == 8 ? 0 : 1) || a.in_rows <= 0) {
+  if (s.tmem) {
+    if (!s.tma) return launch_pass_tmem<T>(a, nullptr, st);
+    if (a.phase_corr || !a.seg_mask || a.in_rows <= 0) {
       set_error("launch_pass_blk: no TMA-fill kernel for this pass");
       return HPSI_ERR_UNSUPPORTED;
     }
     alignas(64) CUtensorMap tm;
     hpsi_status r = encode_input_map<T>(a, &tm);
-    if (r) return r;
-    if constexpr (sizeof(T) == 8)
-      return launch_blk_u<T, 9, 2, 2, false, 8, 128, true>(a, &tm, st);
-    else
-      return launch_blk_u<T, 9, 2, 2, true, 8, 128, true>(a, &tm, st);
+    return r ? r : launch_pass_tmem<T>(a, &tm, st);
   }
   if (s.mma) {
     // FP64 only: in-plane arms as DMMA banded products, 8-state chunks
@@ -166,39 +149,28 @@ hpsi_status launch_pass_blk(const PassArgs &a, const PassShape &s, cudaStream_t 
     }
     return launch_pass_mma(a, st);
   }
-  if (s.mb) {
-    // mbarrier hand-over of the stages: the default cell blocks
-    if (s.ty != 8 || cb != 128 || s.rx != 2 || s.ry != 2 || g != 9 || s.cplx != (sizeof(T) == 8 ? 0 : 1)) {
-      set_error("launch_pass_blk: no mbarrier-pipelined kernel for this cell block");
-      return HPSI_ERR_UNSUPPORTED;
-    }
-    if constexpr (sizeof(T) == 8)
-      return launch_blk_u<T, 9, 2, 2, false, 8, 128, false, true>(a, nullptr, st);
-    else
-      return launch_blk_u<T, 9, 2, 2, true, 8, 128, false, true>(a, nullptr, st);
-  }
   if (s.ty == 8 && cb == 128) {
     if constexpr (sizeof(T) == 8) {
-      if (!s.cplx && s.rx == 2 && s.ry == 2 && g == 9) return launch_blk_u<T, 9, 2, 2, false, 8, 128>(a, nullptr, st);
-      if (!s.cplx && s.rx == 2 && s.ry == 2 && g == 3) return launch_blk_u<T, 3, 2, 2, false, 8, 128>(a, nullptr, st);
-      if (s.cplx && s.rx == 2 && s.ry == 2 && g == 9) return launch_blk_u<T, 9, 2, 2, true, 8, 128>(a, nullptr, st);
+      if (!s.cplx && s.rx == 2 && s.ry == 2 && g == 9) return launch_blk_u<T, 9, 2, 2, false, 8, 128>(a, st);
+      if (!s.cplx && s.rx == 2 && s.ry == 2 && g == 3) return launch_blk_u<T, 3, 2, 2, false, 8, 128>(a, st);
+      if (s.cplx && s.rx == 2 && s.ry == 2 && g == 9) return launch_blk_u<T, 9, 2, 2, true, 8, 128>(a, st);
     } else {
-      if (s.cplx && s.rx == 2 && s.ry == 2 && g == 9) return launch_blk_u<T, 9, 2, 2, true, 8, 128>(a, nullptr, st);
-      if (s.cplx && s.rx == 2 && s.ry == 2 && g == 3) return launch_blk_u<T, 3, 2, 2, true, 8, 128>(a, nullptr, st);
-      if (!s.cplx && s.rx == 2 && s.ry == 4 && g == 1) return launch_blk_u<T, 1, 2, 4, false, 8, 128>(a, nullptr, st);
+      if (s.cplx && s.rx == 2 && s.ry == 2 && g == 9) return launch_blk_u<T, 9, 2, 2, true, 8, 128>(a, st);
+      if (s.cplx && s.rx == 2 && s.ry == 2 && g == 3) return launch_blk_u<T, 3, 2, 2, true, 8, 128>(a, st);
+      if (!s.cplx && s.rx == 2 && s.ry == 4 && g == 1) return launch_blk_u<T, 1, 2, 4, false, 8, 128>(a, st);
     }
   } else if (s.ty == 8 && cb == 64 && s.rx == 1 && s.ry == 4 && g == 9) {
     // 256-thread blocks, two CTAs per SM
     if constexpr (sizeof(T) == 8) {
-      if (!s.cplx) return launch_blk_u<T, 9, 1, 4, false, 8, 64>(a, nullptr, st);
+      if (!s.cplx) return launch_blk_u<T, 9, 1, 4, false, 8, 64>(a, st);
     } else {
-      if (s.cplx) return launch_blk_u<T, 9, 1, 4, true, 8, 64>(a, nullptr, st);
+      if (s.cplx) return launch_blk_u<T, 9, 1, 4, true, 8, 64>(a, st);
     }
   } else if (s.ty == 16 && cb == 64 && s.rx == 1 && s.ry == 4 && g == 9) {
     if constexpr (sizeof(T) == 8) {
-      if (!s.cplx) return launch_blk_u<T, 9, 1, 4, false, 16, 64>(a, nullptr, st);
+      if (!s.cplx) return launch_blk_u<T, 9, 1, 4, false, 16, 64>(a, st);
     } else {
-      if (s.cplx) return launch_blk_u<T, 9, 1, 4, true, 16, 64>(a, nullptr, st);
+      if (s.cplx) return launch_blk_u<T, 9, 1, 4, true, 16, 64>(a, st);
     }
   }
   set_error("launch_pass_blk: no kernel for this cell block");

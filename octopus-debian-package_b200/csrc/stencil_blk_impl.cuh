@@ -101,14 +101,8 @@ struct BlkLayout {
   static constexpr size_t s_rows = size_t(HC) * sizeof(int);
   static constexpr size_t SIDEB = s_rows + size_t(IC) * sizeof(int);
   static constexpr size_t o_side = NBUF * STAGE;
-  // TMA fill: one mbarrier per data stage after the side ring
-  static constexpr size_t o_mbar = o_side + NSIDE * SIDEB;
-  static constexpr size_t bytes = o_mbar;
-  static constexpr size_t bytes_tma = o_mbar + NBUF * 8;
-  // mbarrier hand-over: a full and an empty barrier per data stage
-  static constexpr size_t bytes_mb = o_mbar + 2 * NBUF * 8;
+  static constexpr size_t bytes = o_side + NSIDE * SIDEB;
   static_assert(bytes * CTAS <= 232448 - 2048, "shared memory per CTA");
-  static_assert(bytes_mb * CTAS <= 232448, "shared memory per CTA (mbarrier hand-over)");
   static_assert(STAGE % 16 == 0 && SIDEB % 16 == 0, "16-byte copies");
   static constexpr int NMAPP = HC / 4, NROWP = IC / 4, NVP = IC / 2;  // 16-byte side/v pieces
   static_assert(NMAPP + NROWP <= NT && NVP <= NT, "one side piece per thread");
@@ -147,12 +141,11 @@ __device__ __forceinline__ int star_cell(int i) {
 // the tile's columns (row c / 16), round 4 the bottom rows (the same cells 12
 // rows lower), rounds 1-3 the eight rows beside and across the tile in three
 // column blocks of eight (row 4 + c / 8, column c % 8 + 8 (j - 1)), so that
-// every round's cell is a base plus a constant.  Other shapes (and the TMA
-// fill, whose segments follow the star order) use the star order.
-template <class LY, bool STAR_ORDER>
+// every round's cell is a base plus a constant.  Other shapes use the star order.
+template <class LY>
 __device__ __forceinline__ int fill_cell(int c, int j) {
   constexpr int HX = LY::HX, HAL = LY::HAL, TX = LY::TX;
-  if constexpr (!STAR_ORDER && TX == 16 && LY::TY == 8 && LY::NT / LY::PCS == 64) {
+  if constexpr (TX == 16 && LY::TY == 8 && LY::NT / LY::PCS == 64) {
     if (j == 0 || j == 4) return (c >> 4) * HX + HAL + (c & 15) + (j == 4 ? 12 * HX : 0);
     return (HAL + (c >> 3)) * HX + (c & 7) + 8 * (j - 1);
   } else {
@@ -225,19 +218,9 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 // k % NSIDE.  Iteration k computes plane k and issues the data of plane
 // k + NBUF - 1 and the side data of plane k + 2 NBUF - 2 (one commit group).
 // One work unit: item ih (16 x 8 tile, z block) and state chunk `chunk`.
-//
-// MB: the stages change hands through mbarriers instead of one
-// __syncthreads per plane.  Full barrier of a stage (2 NT arrivals per
-// phase): every thread's cp.async arrive-on plus its plain arrive (covering
-// its plain shared stores) after issuing a plane.  Empty barrier (NT): a
-// thread arrives when it is done with a plane; the refill of that plane's
-// stage waits for it.  The arrive comes after the arithmetic and the wait
-// after the next plane's arithmetic, so a warp may run one plane ahead of the
-// slowest one.  Every wait is bounded (HPSI_ERR_TIMEOUT in p.err).
 template <typename T, bool HORNER, bool OBS, bool RHO, int U, int RX_, int RY_, bool CPLX, int TY_, int CB_,
-          bool TMA = false, bool MB = false, bool FLD = true>
-__device__ __forceinline__ void blk_body(const PassArgs &p, const int ih, const int chunk, unsigned char *smem,
-                                         const CUtensorMap *tm = nullptr) {
+          bool FLD = true>
+__device__ __forceinline__ void blk_body(const PassArgs &p, const int ih, const int chunk, unsigned char *smem) {
   constexpr bool X0 = HORNER || OBS;
   using LY = BlkLayout<T, X0, RX_, RY_, CPLX, TY_, CB_>;
   using E = typename BlkElem<T, CPLX>::E;
@@ -256,31 +239,6 @@ __device__ __forceinline__ void blk_body(const PassArgs &p, const int ih, const 
 
   auto stage = [&](int k) { return smem + size_t(k % NBUF) * LY::STAGE; };
   auto side = [&](int k) { return smem + LY::o_side + size_t(k % NSIDE) * LY::SIDEB; };
-  // TMA fill: star segment s (star cells 8 s .. 8 s + 7, eight consecutive
-  // cells of one halo row) is one box copy when bit s of the plane's mask is
-  // set (its rows are eight consecutive rows of the batch)
-  static_assert(!TMA || (LY::TX == 16 && LY::TY == 8 && LY::CELLB == 128 && LY::SC == 320),
-                "TMA fill: 16 x 8 tiles, 128-byte chunks");
-  auto mbar = [&](int k) { return reinterpret_cast<uint64_t *>(smem + LY::o_mbar) + (k % NBUF); };
-  [[maybe_unused]] const size_t mask_row = TMA ? (size_t(it.y) * p.seg_tiles_x + it.x) * B.NZ : 0;
-  [[maybe_unused]] bool tma_dead = false;
-  static_assert(!(TMA && MB), "one stage hand-over per kernel");
-  // MB: full barrier of plane k's stage, empty barrier after it
-  [[maybe_unused]] auto full_bar = [&](int k) { return reinterpret_cast<uint64_t *>(smem + LY::o_mbar) + (k % NBUF); };
-  [[maybe_unused]] auto empty_bar = [&](int k) { return reinterpret_cast<uint64_t *>(smem + LY::o_mbar) + NBUF + (k % NBUF); };
-  [[maybe_unused]] bool mb_dead = false;
-  [[maybe_unused]] auto mb_wait = [&](uint64_t *bar, unsigned parity) {
-    if (mb_dead) return;
-    unsigned n = 0;
-    while (!mbar_try_wait(bar, parity))
-      if (++n == TMA_WAIT_LIMIT) {
-        mb_dead = true;
-        if (p.err) atomicExch(p.err, HPSI_ERR_TIMEOUT);
-        return;
-      }
-  };
-  [[maybe_unused]] const bool smem_a128 = (static_cast<unsigned>(__cvta_generic_to_shared(smem)) & 127u) == 0;
-
   // ---- copy roles ---------------------------------------------------------------
   const int cpc = tid / PCS, piece = tid % PCS;  // cell (+ NT / PCS per round) and 16-byte piece
   __builtin_assume(cpc >= 0 && cpc < LY::NT / PCS);
@@ -332,33 +290,15 @@ __device__ __forceinline__ void blk_body(const PassArgs &p, const int ih, const 
     const unsigned char *sd = side(k);
     const int *map = reinterpret_cast<const int *>(sd);
     T *halo = reinterpret_cast<T *>(st) + piece * EPP;
-    [[maybe_unused]] unsigned long long mask = 0;
-    if constexpr (TMA) {
-      if (p.phase_corr == nullptr && smem_a128) mask = __ldg(p.seg_mask + mask_row + (zbeg + k));
-      // the stage's mbarrier expects the bytes of every box of the plane (its
-      // phase completes at once when the plane has none)
-      if (tid == 0) mbar_arrive_expect_tx(mbar(k), unsigned(__popcll(mask)) * 8u * LY::CELLB);
-    }
     if (p.phase_corr == nullptr) {
       // every entry is a row or -1 (zero): one zero-filling copy per piece
 #pragma unroll
       for (int j = 0; j < LY::SROUNDS; ++j) {
         const int i = cpc + j * (LY::NT / PCS);
         if (LY::SPART && j == LY::SROUNDS - 1 && i >= LY::SC) break;
-        if constexpr (TMA)
-          if ((mask >> (i >> 3)) & 1ull) continue;  // this cell arrives with its segment's box
-        const int cell = fill_cell<LY, TMA>(cpc, j);
+        const int cell = fill_cell<LY>(cpc, j);
         const int src = map[cell];
         cp_async16_zfill(halo + cell * SL, in_bytes + size_t(unsigned(max(src, 0))) * in_rb, src >= 0 ? 16 : 0);
-      }
-      if constexpr (TMA) {
-        // thread s < 40 copies segment s
-        if (tid < 40 && ((mask >> tid) & 1ull)) {
-          // (the mask is cleared above when the dynamic shared memory is not
-          // 128-byte aligned: box copies need 128-byte aligned destinations)
-          const int cell = star_cell<LY>(8 * tid);
-          tma_load_rows(reinterpret_cast<T *>(st) + cell * SL, tm, col, map[cell], mbar(k));
-        }
       }
     } else {
 #pragma unroll 1
@@ -411,21 +351,6 @@ __device__ __forceinline__ void blk_body(const PassArgs &p, const int ih, const 
 
   // ---- prologue: side data of planes 0..NBUF-2 synchronously, then the first
   // NBUF-1 groups (data of planes 0..NBUF-2, side of planes NBUF-1..2NBUF-3)
-  if constexpr (TMA) {
-    if (tid == 0) {
-      for (int b = 0; b < NBUF; ++b) mbar_init(mbar(b), 1);
-      mbar_init_fence();
-    }
-  }
-  if constexpr (MB) {
-    if (tid == 0) {
-      for (int b = 0; b < NBUF; ++b) {
-        mbar_init(full_bar(b), 2 * LY::NT);
-        mbar_init(empty_bar(b), LY::NT);
-      }
-      mbar_init_fence();
-    }
-  }
   for (int k = 0; k < NBUF - 1 && k < nplanes; ++k) {
     unsigned char *sd = side(k);
     const int q = zbeg + k;
@@ -442,14 +367,7 @@ __device__ __forceinline__ void blk_body(const PassArgs &p, const int ih, const 
   for (int k = 0; k < NBUF - 1; ++k) {
     issue_data(k);
     issue_side(k + NBUF - 1);
-    if constexpr (MB) {
-      if (k < nplanes) {
-        cp_async_arrive_noinc(full_bar(k));
-        mbar_arrive(full_bar(k));
-      }
-    } else {
-      cp_async_commit();
-    }
+    cp_async_commit();
   }
 
   // ---- compute roles --------------------------------------------------------------
@@ -512,26 +430,8 @@ __device__ __forceinline__ void blk_body(const PassArgs &p, const int ih, const 
   auto plane = [&](auto Kc, int k) {
     constexpr int K = decltype(Kc)::value;
     constexpr int S4 = (4 + K) % 9;  // running sum of output plane zbeg + k
-    if constexpr (MB) {
-      // the plane's copies and stores of every thread (and the side data of
-      // plane k + NBUF - 1, issued with them)
-      mb_wait(full_bar(k), unsigned(k / NBUF) & 1u);
-    } else {
-      cp_async_wait<NBUF - 2>();
-      __syncthreads();
-    }
-    if constexpr (TMA) {
-      // the plane's boxes (each thread observes the phase itself)
-      if (!tma_dead) {
-        unsigned n = 0;
-        while (!mbar_try_wait(mbar(k), unsigned(k / NBUF) & 1u))
-          if (++n == TMA_WAIT_LIMIT) {
-            tma_dead = true;
-            if (tid == 0 && p.err) atomicExch(p.err, HPSI_ERR_TIMEOUT);
-            break;
-          }
-      }
-    }
+    cp_async_wait<NBUF - 2>();
+    __syncthreads();
     // the refill of the stage read in plane k - 1 is issued after this
     // plane's arithmetic (every thread passed the barrier above, so the stage
     // is free): the arithmetic starts right after the barrier
@@ -708,23 +608,9 @@ __device__ __forceinline__ void blk_body(const PassArgs &p, const int ih, const 
         sd += pn * (dxy00 + p.obs_pol[2] * B.h[2] * double(zo + B.lo[2])) + pd;
       }
     }
-    if constexpr (MB) {
-      mbar_arrive(empty_bar(k));  // this thread is done with plane k
-      const int kn = k + NBUF - 1;
-      if (kn < nplanes) {
-        // stage of plane k - 1 and the side slot of plane k + 2 NBUF - 2
-        // (last held plane k - 1 or earlier): every thread done with k - 1
-        if (k >= 1) mb_wait(empty_bar(k - 1), unsigned((k - 1) / NBUF) & 1u);
-        issue_data(kn);
-        issue_side(k + LY::SIDE_AHEAD);
-        cp_async_arrive_noinc(full_bar(kn));
-        mbar_arrive(full_bar(kn));
-      }
-    } else {
-      issue_data(k + NBUF - 1);
-      issue_side(k + LY::SIDE_AHEAD);
-      cp_async_commit();
-    }
+    issue_data(k + NBUF - 1);
+    issue_side(k + LY::SIDE_AHEAD);
+    cp_async_commit();
   };
 
   auto rotate = [&]() {
@@ -795,14 +681,14 @@ __device__ __forceinline__ void blk_body(const PassArgs &p, const int ih, const 
   }
 }
 
-template <typename T, bool HORNER, bool OBS, bool RHO, int U, int RX, int RY, bool CPLX, int TY, int CB, bool TMA,
-          bool MB, bool FLD>
+template <typename T, bool HORNER, bool OBS, bool RHO, int U, int RX, int RY, bool CPLX, int TY, int CB,
+          bool FLD>
 __global__ void __launch_bounds__(BlkLayout<T, HORNER || OBS, RX, RY, CPLX, TY, CB>::NT,
                                   BlkLayout<T, HORNER || OBS, RX, RY, CPLX, TY, CB>::CTAS)
-    pass_blk_kernel(const __grid_constant__ PassArgs p, const __grid_constant__ CUtensorMap tm) {
+    pass_blk_kernel(const __grid_constant__ PassArgs p) {
   extern __shared__ __align__(128) unsigned char smem[];
-  blk_body<T, HORNER, OBS, RHO, U, RX, RY, CPLX, TY, CB, TMA, MB, FLD>(p, blockIdx.x / p.chunks,
-                                                                        blockIdx.x % p.chunks, smem, &tm);
+  blk_body<T, HORNER, OBS, RHO, U, RX, RY, CPLX, TY, CB, FLD>(p, blockIdx.x / p.chunks,
+                                                                        blockIdx.x % p.chunks, smem);
 }
 
 // Many systems in one persistent launch (Horner passes): each CTA takes
@@ -821,7 +707,7 @@ __global__ void __launch_bounds__(BlkLayout<T, true, RX, RY, CPLX, TY, CB>::NT,
     __syncthreads();
     if (u >= g.nunits) break;
     const int4 W = g.units[u];  // {system, item, chunk, -}
-    blk_body<T, true, false, false, U, RX, RY, CPLX, TY, CB, false, false, FLD>(g.sys[W.x], W.y, W.z, smem);
+    blk_body<T, true, false, false, U, RX, RY, CPLX, TY, CB, FLD>(g.sys[W.x], W.y, W.z, smem);
     __syncthreads();
   }
 }
@@ -838,12 +724,12 @@ bool blk_strides_ok(const PassArgs &a) {
   return true;
 }
 
-template <typename T, bool HORNER, bool OBS, bool RHO, int U, int RX, int RY, bool CPLX, int TY, int CB, bool TMA,
-          bool MB, bool FLD>
-hpsi_status launch_blk_mode(const PassArgs &a, const CUtensorMap *tm, cudaStream_t st) {
+template <typename T, bool HORNER, bool OBS, bool RHO, int U, int RX, int RY, bool CPLX, int TY, int CB,
+          bool FLD>
+hpsi_status launch_blk_mode(const PassArgs &a, cudaStream_t st) {
   using LY = BlkLayout<T, HORNER || OBS, RX, RY, CPLX, TY, CB>;
-  constexpr size_t SMEM = TMA ? LY::bytes_tma : MB ? LY::bytes_mb : LY::bytes;
-  auto kern = pass_blk_kernel<T, HORNER, OBS, RHO, U, RX, RY, CPLX, TY, CB, TMA, MB, FLD>;
+  constexpr size_t SMEM = LY::bytes;
+  auto kern = pass_blk_kernel<T, HORNER, OBS, RHO, U, RX, RY, CPLX, TY, CB, FLD>;
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
   std::call_once(once, [&] {
@@ -852,31 +738,25 @@ hpsi_status launch_blk_mode(const PassArgs &a, const CUtensorMap *tm, cudaStream
       attr = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   });
   HPSI_TRY_CUDA(attr);
-  if (TMA && (!tm || !a.seg_mask)) {
-    set_error("launch_pass_blk: TMA fill without its tensor map or segment masks");
-    return HPSI_ERR_ARG;
-  }
   if (!blk_strides_ok<T>(a)) return HPSI_ERR_ARG;
-  CUtensorMap none;
-  std::memset(&none, 0, sizeof(none));
   const unsigned nblocks = unsigned(a.nitems) * unsigned(a.chunks);
-  kern<<<nblocks, LY::NT, SMEM, st>>>(a, tm ? *tm : none);
+  kern<<<nblocks, LY::NT, SMEM, st>>>(a);
   HPSI_CHECK_LAUNCH();
   return HPSI_OK;
 }
 
-template <typename T, int U, int RX, int RY, bool CPLX, int TY, int CB, bool TMA, bool MB, bool FLD>
-hpsi_status launch_blk_modes(const PassArgs &a, const CUtensorMap *tm, cudaStream_t st) {
+template <typename T, int U, int RX, int RY, bool CPLX, int TY, int CB, bool FLD>
+hpsi_status launch_blk_modes(const PassArgs &a, cudaStream_t st) {
   const bool horner = a.mode == PASS_HORNER, obs = a.obs != nullptr, rho = a.rho_part != nullptr;
-  if (horner && obs) return launch_blk_mode<T, true, true, false, U, RX, RY, CPLX, TY, CB, TMA, MB, FLD>(a, tm, st);
-  if (horner && rho) return launch_blk_mode<T, true, false, true, U, RX, RY, CPLX, TY, CB, TMA, MB, FLD>(a, tm, st);
-  if (horner) return launch_blk_mode<T, true, false, false, U, RX, RY, CPLX, TY, CB, TMA, MB, FLD>(a, tm, st);
-  if (obs) return launch_blk_mode<T, false, true, false, U, RX, RY, CPLX, TY, CB, TMA, MB, FLD>(a, tm, st);
-  return launch_blk_mode<T, false, false, false, U, RX, RY, CPLX, TY, CB, TMA, MB, FLD>(a, tm, st);
+  if (horner && obs) return launch_blk_mode<T, true, true, false, U, RX, RY, CPLX, TY, CB, FLD>(a, st);
+  if (horner && rho) return launch_blk_mode<T, true, false, true, U, RX, RY, CPLX, TY, CB, FLD>(a, st);
+  if (horner) return launch_blk_mode<T, true, false, false, U, RX, RY, CPLX, TY, CB, FLD>(a, st);
+  if (obs) return launch_blk_mode<T, false, true, false, U, RX, RY, CPLX, TY, CB, FLD>(a, st);
+  return launch_blk_mode<T, false, false, false, U, RX, RY, CPLX, TY, CB, FLD>(a, st);
 }
 
-template <typename T, int U, int RX, int RY, bool CPLX, int TY, int CB, bool TMA = false, bool MB = false>
-hpsi_status launch_blk_u(const PassArgs &a, const CUtensorMap *tm, cudaStream_t st) {
+template <typename T, int U, int RX, int RY, bool CPLX, int TY, int CB>
+hpsi_status launch_blk_u(const PassArgs &a, cudaStream_t st) {
   const bool horner = a.mode == PASS_HORNER, obs = a.obs != nullptr, rho = a.rho_part != nullptr;
   if (rho && (!horner || obs)) {
     set_error("launch_pass_blk: the density is fused into Horner passes without observables only");
@@ -884,11 +764,11 @@ hpsi_status launch_blk_u(const PassArgs &a, const CUtensorMap *tm, cudaStream_t 
   }
   // the default 16 x 8 shapes also come without the laser term, for passes
   // with no field set (fewer registers and branches per plane)
-  constexpr bool NOFLD = !TMA && !MB && U == 9 && RX == 2 && RY == 2 && TY == 8 && CB == 128;
+  constexpr bool NOFLD = U == 9 && RX == 2 && RY == 2 && TY == 8 && CB == 128;
   if constexpr (NOFLD)
     if (a.fld[0] == 0.0 && a.fld[1] == 0.0 && a.fld[2] == 0.0)
-      return launch_blk_modes<T, U, RX, RY, CPLX, TY, CB, TMA, MB, false>(a, tm, st);
-  return launch_blk_modes<T, U, RX, RY, CPLX, TY, CB, TMA, MB, true>(a, tm, st);
+      return launch_blk_modes<T, U, RX, RY, CPLX, TY, CB, false>(a, st);
+  return launch_blk_modes<T, U, RX, RY, CPLX, TY, CB, true>(a, st);
 }
 
 template <typename T, int U, int RX, int RY, bool CPLX, int TY, int CB, bool FLD>
