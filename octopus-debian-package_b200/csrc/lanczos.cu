@@ -313,14 +313,25 @@ extern "C" hpsi_status hpsi_lanczos_step(hpsi_hamiltonian *h, hpsi_batch *psi, d
   auto vec = [&](int j) { return j == 0 ? psi_d : U + (j - 1) * vstride; };
   const dim3 rgrid(nblk, (nst + 255) / 256);
 
-  // host copies: norms and scales of every vector, raw overlaps of this iteration
+  // host copies: norms and scales of every vector, raw overlaps of this
+  // iteration; they arrive through two pinned slots (the iteration under test
+  // and the next one, already queued)
   std::vector<double> hn(size_t(K + 1) * nst), hs(size_t(K + 1) * nst), hraw(4 * size_t(nst));
-  auto fetch = [&](int j, bool with_raw) -> hpsi_status {
-    HPSI_TRY_CUDA(cudaMemcpyAsync(hn.data() + size_t(j) * nst, nrm + size_t(j) * nst, nst * sizeof(double),
-                                  cudaMemcpyDeviceToHost, st));
+  const size_t pslot = 5 * size_t(nst);
+  s = h->lanczos_pinned(2 * pslot * sizeof(double));
+  if (s) return s;
+  auto slot = [&](int j) { return static_cast<double *>(h->lz_pin) + (j & 1) * pslot; };
+  auto send = [&](int j, bool with_raw) -> hpsi_status {
+    HPSI_TRY_CUDA(cudaMemcpyAsync(slot(j), nrm + size_t(j) * nst, nst * sizeof(double), cudaMemcpyDeviceToHost, st));
     if (with_raw)
-      HPSI_TRY_CUDA(cudaMemcpyAsync(hraw.data(), raw, hraw.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    HPSI_TRY_CUDA(cudaStreamSynchronize(st));
+      HPSI_TRY_CUDA(cudaMemcpyAsync(slot(j) + nst, raw, hraw.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+    HPSI_TRY_CUDA(cudaEventRecord(h->lz_ev[j & 1], st));
+    return HPSI_OK;
+  };
+  auto receive = [&](int j, bool with_raw) -> hpsi_status {
+    HPSI_TRY_CUDA(cudaEventSynchronize(h->lz_ev[j & 1]));
+    std::memcpy(hn.data() + size_t(j) * nst, slot(j), nst * sizeof(double));
+    if (with_raw) std::memcpy(hraw.data(), slot(j) + nst, hraw.size() * sizeof(double));
     for (int i = 0; i < nst; ++i) {
       const double n = hn[size_t(j) * nst + i];
       hs[size_t(j) * nst + i] = n >= 1e4 * 2.220446049250313e-16 ? n : 1.0;
@@ -334,7 +345,8 @@ extern "C" hpsi_status hpsi_lanczos_step(hpsi_hamiltonian *h, hpsi_batch *psi, d
   HPSI_CHECK_LAUNCH();
   lz_finalize<<<nst, 256, 0, st>>>(partial, nblk, nst, 1, dv, nullptr, nrm, sc);
   HPSI_CHECK_LAUNCH();
-  s = fetch(0, false);
+  s = send(0, false);
+  if (!s) s = receive(0, false);
   if (s) return s;
   bool all_null = true;
   for (int i = 0; i < nst; ++i) all_null = all_null && std::abs(hn[i]) <= 1e-12;
@@ -350,26 +362,47 @@ extern "C" hpsi_status hpsi_lanczos_step(hpsi_hamiltonian *h, hpsi_batch *psi, d
   std::vector<std::vector<cplx>> H(nst, std::vector<cplx>(size_t(K + 1) * (K + 1), 0.0));
   std::vector<std::vector<cplx>> expo(nst);
   std::vector<double> res(nst, 0.0);
-  int iter = 1;
-  for (; iter <= K; ++iter) {
-    // w = H u_{iter-1} into u_iter's slot, then CGS against v_l-1 .. v_iter-1, l = max(1, iter - 1)
-    s = apply_h_dev<double>(h, reinterpret_cast<const double *>(vec(iter - 1)), ld,
-                            reinterpret_cast<double *>(vec(iter)), ld, HPSI_TERM_ALL, 1, st);
-    if (s) return s;
-    const int l = std::max(1, iter - 1);
-    const bool two = iter - l == 1;
+  // device work of iteration `it`: w = H u_{it-1} into u_it's slot, then CGS
+  // against v_l-1 .. v_it-1, l = max(1, it - 1)
+  auto issue = [&](int it) -> hpsi_status {
+    hpsi_status r = apply_h_dev<double>(h, reinterpret_cast<const double *>(vec(it - 1)), ld,
+                                        reinterpret_cast<double *>(vec(it)), ld, HPSI_TERM_ALL, 1, st);
+    if (r) return r;
+    const int l = std::max(1, it - 1);
+    const bool two = it - l == 1;
     const double2 *ua = vec(l - 1), *ub = two ? vec(l) : nullptr;
-    lz_sum_kernel<1><<<rgrid, 256, 0, st>>>(vec(iter), ua, ub, ld, np, nst, none, partial);
+    lz_sum_kernel<1><<<rgrid, 256, 0, st>>>(vec(it), ua, ub, ld, np, nst, none, partial);
     HPSI_CHECK_LAUNCH();
     lz_finalize<<<nst, 256, 0, st>>>(partial, nblk, nst, 4, dv, raw, nullptr, nullptr);
     HPSI_CHECK_LAUNCH();
-    LzCoef cf{raw, sc + size_t(iter - 1) * nst, sc + size_t(l - 1) * nst, two ? sc + size_t(l) * nst : nullptr};
-    lz_sum_kernel<2><<<rgrid, 256, 0, st>>>(vec(iter), ua, ub, ld, np, nst, cf, partial);
+    LzCoef cf{raw, sc + size_t(it - 1) * nst, sc + size_t(l - 1) * nst, two ? sc + size_t(l) * nst : nullptr};
+    lz_sum_kernel<2><<<rgrid, 256, 0, st>>>(vec(it), ua, ub, ld, np, nst, cf, partial);
     HPSI_CHECK_LAUNCH();
-    lz_finalize<<<nst, 256, 0, st>>>(partial, nblk, nst, 1, dv, nullptr, nrm + size_t(iter) * nst,
-                                       sc + size_t(iter) * nst);
+    lz_finalize<<<nst, 256, 0, st>>>(partial, nblk, nst, 1, dv, nullptr, nrm + size_t(it) * nst, sc + size_t(it) * nst);
     HPSI_CHECK_LAUNCH();
-    s = fetch(iter, true);
+    return send(it, true);
+  };
+  int iter = 1, issued = 0;
+  double worst1 = 0.0, worst2 = 0.0;  // error estimates of the last two iterations
+  for (; iter <= K; ++iter) {
+    const int l = std::max(1, iter - 1);
+    if (issued < iter) {
+      s = issue(iter);
+      if (s) return s;
+      issued = iter;
+    }
+    // the next iteration is queued before this one's test, so that the GPU works
+    // while the host solves the small eigenproblems (R = 8 sphere, 32 states: 13.5 ms a
+    // step with the GPU waiting for every test); not where the trend of the
+    // estimates says that the test will stop (a queued iteration too many only
+    // costs its time: its vector is not used)
+    const bool stops = iter > 3 && worst1 * worst1 < 3.0 * tol * worst2;
+    if (!stops && iter < K) {
+      s = issue(iter + 1);
+      if (s) return s;
+      issued = iter + 1;
+    }
+    s = receive(iter, true);
     if (s) return s;
     const double *sp = hs.data() + size_t(iter - 1) * nst;
     std::vector<char> ok(nst, 1);
@@ -414,6 +447,8 @@ extern "C" hpsi_status hpsi_lanczos_step(hpsi_hamiltonian *h, hpsi_batch *psi, d
       worst = std::max(worst, res[i]);
       breakdown = breakdown && hn[size_t(iter) * nst + i] < 1e4 * 2.220446049250313e-16;
     }
+    worst2 = worst1;
+    worst1 = worst;
     if (breakdown) break;  // happy breakdown: the space is invariant
     if (iter > 3 && worst < tol) break;
   }
