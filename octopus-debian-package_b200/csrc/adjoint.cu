@@ -429,9 +429,12 @@ extern "C" hpsi_status hpsi_adjoint_gradient(hpsi_hamiltonian *h, const hpsi_bat
   const int nseg = (nsteps + ckpt - 1) / ckpt;
   const int seglen = std::min(ckpt, nsteps);
   // complex buffers: checkpoints nseg, segment seglen, lambda; then the step
-  // scratch; doubles: gv np, ov 2*ld, ov partial 4*ld, geps nsteps, gcont nsteps
+  // scratch; doubles: gv np, ov 2*ld, ov partials 4*ld per block, geps nsteps,
+  // gcont nsteps.  The overlaps with the targets take one block per SM (one
+  // block in all: 2.83 ms at 110,592 points, 16 states)
+  const int ovblk = std::max(1, std::min(m->num_sms, (m->np + 255) / 256));
   const size_t ncplx = batch * (size_t(nseg) + seglen + 1);
-  const size_t ndbl = size_t(m->np) + 6 * size_t(R.ld) + 2 * size_t(nsteps) + 8;
+  const size_t ndbl = size_t(m->np) + (2 + 4 * size_t(ovblk)) * size_t(R.ld) + 2 * size_t(nsteps) + 8;
   const size_t stepb = adj_step_bytes(m, R.ld, order);
   hpsi_status s = h->adjbuf.ensure(ncplx * sizeof(double2) + ndbl * sizeof(double) + 256 + stepb);
   if (s) return s;
@@ -440,8 +443,8 @@ extern "C" hpsi_status hpsi_adjoint_gradient(hpsi_hamiltonian *h, const hpsi_bat
   double2 *Lb = seg + batch * seglen;
   double *gv = reinterpret_cast<double *>(Lb + batch);
   double *ov = gv + m->np;           // 2*ld
-  double *ovpart = ov + 2 * R.ld;    // 4*ld (state_sum partial of one block)
-  double *geps = ovpart + 4 * R.ld;  // nsteps
+  double *ovpart = ov + 2 * R.ld;    // 4*ld per block (state_sum partials)
+  double *geps = ovpart + 4 * R.ld * ovblk;  // nsteps
   double *gcont = geps + nsteps;     // nsteps
   // the step scratch starts on the next 256-byte boundary (room reserved above)
   void *stepbase = reinterpret_cast<void *>((reinterpret_cast<uintptr_t>(gcont + nsteps + 8) + 255) &
@@ -470,7 +473,7 @@ extern "C" hpsi_status hpsi_adjoint_gradient(hpsi_hamiltonian *h, const hpsi_bat
   }
   // J and lambda_N
   s = launch_state_sum<double>(1, static_cast<const double *>(targets->ptr), targets->ld,
-                               reinterpret_cast<const double *>(cur), R.ld, m->np, R.nst, ovpart, 1, dv, 0, ov, st);
+                               reinterpret_cast<const double *>(cur), R.ld, m->np, R.nst, ovpart, ovblk, dv, 0, ov, st);
   if (s) return fail(s);
   std::vector<double> ovh(2 * size_t(R.nst));
   HPSI_TRY_CUDA(cudaMemcpyAsync(ovh.data(), ov, ovh.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
