@@ -470,8 +470,12 @@ hpsi_status hpsi_mesh_create(const hpsi_mesh_desc *d, hpsi_mesh **out) {
   up(&m->d_cell_row, cell_row);
   up(&m->d_src_raw, cell_row);
   if (s == HPSI_OK) {
+    // (the status words of the mesh's Hamiltonians follow the table, cleared)
+    const size_t ncol = col_z.size();
+    col_z.resize(ncol + MESH_STATUS_WORDS / 2, make_int2(0, 0));
     s = dev_alloc(reinterpret_cast<void **>(&m->d_col_z), col_z.size() * sizeof(int2));
     if (s == HPSI_OK) {
+      m->d_status = reinterpret_cast<int *>(m->d_col_z + ncol);
       cudaError_t e = cudaMemcpy(m->d_col_z, col_z.data(), col_z.size() * sizeof(int2), cudaMemcpyHostToDevice);
       if (e != cudaSuccess) {
         set_error(cudaGetErrorString(e));
@@ -536,19 +540,9 @@ hpsi_status hpsi_hamiltonian_create(hpsi_mesh *mesh, hpsi_hamiltonian **out) {
   // experiment override: HPSI_FUSED_DENSITY=1 fuses the density of
   // hpsi_taylor_step_density into the last pass
   if (const char *e = std::getenv("HPSI_FUSED_DENSITY")) h->fuse_density = std::atoi(e) != 0;
-  // status word of the passes' bounded waits (allocated here: a pass may first
-  // run inside a stream capture)
-  hpsi_status s = dev_alloc(reinterpret_cast<void **>(&h->d_err), sizeof(int));
-  if (s) {
-    delete h;
-    return s;
-  }
-  if (cudaMemset(h->d_err, 0, sizeof(int)) != cudaSuccess) {
-    set_error("hpsi_hamiltonian_create: cudaMemset failed");
-    dev_free(h->d_err);
-    delete h;
-    return HPSI_ERR_CUDA;
-  }
+  // status word of the passes' bounded waits: one of the mesh's (256 of them, taken
+  // in turn; no allocation of its own)
+  h->d_err = mesh->d_status + mesh->next_status.fetch_add(1u) % MESH_STATUS_WORDS;
   *out = h;
   return HPSI_OK;
 }
@@ -572,7 +566,6 @@ hpsi_status hpsi_hamiltonian_destroy(hpsi_hamiltonian *h) {
   h->adjstep.release();
   h->vjpbuf.release();
   h->rhobuf.release();
-  dev_free(h->d_err);
   h->lzsmall.release();
   if (h->lz_pin) cudaFreeHost(h->lz_pin);
   for (auto &e : h->lz_ev)
@@ -624,21 +617,9 @@ hpsi_status hpsi_hamiltonian::ensure_bra_stream() {
 }
 
 void hpsi_hamiltonian::proj_free() {
-  dev_free(d_mat);
-  dev_free(d_proj_row);
-  dev_free(d_map);
-  dev_free(d_pt);
-  dev_free(d_pt_f);
-  dev_free(d_scal);
-  dev_free(d_scal_f);
-  dev_free(d_krows);
-  dev_free(d_kidx);
+  dev_free(kb_tables);  // (holds every table below)
+  kb_tables = nullptr;
   d_kidx = nullptr;
-  dev_free(d_kptr);
-  dev_free(d_kb_ent);
-  dev_free(d_kblk);
-  dev_free(d_pk);
-  dev_free(d_pk_f);
   d_kblk = nullptr;
   d_pk = nullptr;
   d_pk_f = nullptr;
@@ -902,18 +883,14 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, c
   std::vector<float> pkf(pk.begin(), pk.end());
   int minp = 1 << 30;
   for (int i = 0; i < nmat; ++i) minp = std::min(minp, int(npoints[i]));
-  hpsi_status s = HPSI_OK;
-  auto up = [&](void **dp, const void *src, size_t bytes) {
-    if (s) return;
-    s = dev_alloc(dp, bytes);
-    if (!s && bytes) {
-      cudaError_t e = cudaMemcpy(*dp, src, bytes, cudaMemcpyHostToDevice);
-      if (e != cudaSuccess) {
-        set_error(cudaGetErrorString(e));
-        s = HPSI_ERR_CUDA;
-      }
-    }
+  // one allocation for all tables
+  struct Part {
+    void **dp;
+    const void *src;
+    size_t bytes;
   };
+  std::vector<Part> parts;
+  auto up = [&](void **dp, const void *src, size_t bytes) { parts.push_back({dp, src, bytes}); };
   up(reinterpret_cast<void **>(&h->d_mat), mat.data(), mat.size() * sizeof(int4));
   up(reinterpret_cast<void **>(&h->d_proj_row), prow.data(), prow.size() * sizeof(int));
   up(reinterpret_cast<void **>(&h->d_map), map, size_t(npts_tot) * sizeof(int));
@@ -922,16 +899,28 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, c
   up(reinterpret_cast<void **>(&h->d_scal), scal, size_t(nproj_tot) * sizeof(double));
   up(reinterpret_cast<void **>(&h->d_scal_f), scf.data(), scf.size() * sizeof(float));
   up(reinterpret_cast<void **>(&h->d_krows), krows.data(), krows.size() * sizeof(int));
-  {
-    std::vector<int> kidx(m->np, -1);
-    for (size_t i = 0; i < krows.size(); ++i) kidx[krows[i]] = int(i);
-    up(reinterpret_cast<void **>(&h->d_kidx), kidx.data(), kidx.size() * sizeof(int));
-  }
+  std::vector<int> kidx(m->np, -1);
+  for (size_t i = 0; i < krows.size(); ++i) kidx[krows[i]] = int(i);
+  up(reinterpret_cast<void **>(&h->d_kidx), kidx.data(), kidx.size() * sizeof(int));
   up(reinterpret_cast<void **>(&h->d_kptr), kptr.data(), kptr.size() * sizeof(int));
   up(reinterpret_cast<void **>(&h->d_kb_ent), ent.data(), ent.size() * sizeof(int4));
   up(reinterpret_cast<void **>(&h->d_kblk), blk.data(), blk.size() * sizeof(int4));
   up(reinterpret_cast<void **>(&h->d_pk), pk.data(), pk.size() * sizeof(double));
   up(reinterpret_cast<void **>(&h->d_pk_f), pkf.data(), pkf.size() * sizeof(float));
+  size_t total = 0;
+  for (const Part &q : parts) total += (q.bytes + 255) / 256 * 256;
+  hpsi_status s = dev_alloc(&h->kb_tables, std::max<size_t>(total, 256));
+  char *at = static_cast<char *>(h->kb_tables);
+  for (const Part &q : parts) {
+    if (s) break;
+    *q.dp = at;
+    at += (q.bytes + 255) / 256 * 256;
+    const cudaError_t e = q.bytes ? cudaMemcpy(*q.dp, q.src, q.bytes, cudaMemcpyHostToDevice) : cudaSuccess;
+    if (e != cudaSuccess) {
+      set_error(cudaGetErrorString(e));
+      s = HPSI_ERR_CUDA;
+    }
+  }
   if (s) {
     h->proj_free();
     return s;
@@ -1055,45 +1044,54 @@ static double pass_makespan(const hpsi_mesh *m, int ty, int zb, int chunks, int 
 // shallower ones balance the tail: on the R = 12 sphere (108 tile columns) the
 // choice is within 0.2 % of the best measured depth for 1 to 16 chunks, where
 // a fixed four-wave target was up to 9.5 % slower with one or two chunks.
-std::pair<int, double> choose_zb_single(const hpsi_mesh *m, int chunks, int ctas_per_sm) {
+int choose_zb_single(const hpsi_mesh *m, int chunks, int ctas_per_sm) {
   const int key = 4 * chunks + ctas_per_sm;
   auto it = m->zb_single.find(key);
   if (it != m->zb_single.end()) return it->second;
-  std::pair<int, double> best{16, 1e300};
+  int best = 16;
+  double best_t = 1e300;
   for (int zb : {1 << 20, 96, 64, 48, 32, 24, 16}) {
     const double t = pass_makespan(m, 8, zb, chunks, m->num_sms * ctas_per_sm, 8 + 4);
-    if (t < best.second) best = {zb, t};
+    if (t < best_t) best = zb, best_t = t;
   }
   m->zb_single[key] = best;
   return best;
 }
 
 // The same for the tensor-memory pass over 16 x 16 tiles, whose halo planes
-// cost less than output planes (their own cells only, no in-plane arms): the
-// candidates cut the tallest tile column into equal blocks.
-std::pair<int, double> choose_zb_tmem(const hpsi_mesh *m, int chunks) {
+// cost less than output planes (their own cells only, no in-plane arms): fixed
+// depths, and cuts of the tallest tile column into equal blocks.
+int choose_zb_tmem(const hpsi_mesh *m, int chunks) {
   const int key = 4 * chunks;
   auto it = m->zb_single.find(key);
   if (it != m->zb_single.end()) return it->second;
   int tall = 1;
   for (auto &t : m->tile_z)
     if (t.y >= 0) tall = std::max(tall, t.y - t.x + 1);
-  std::pair<int, double> best{1 << 20, 1e300};
-  for (int n = 1; n <= 16 && (tall + n - 1) / n >= 4; ++n) {
-    const int zb = n == 1 ? 1 << 20 : (tall + n - 1) / n;
+  int best = 1 << 20;
+  double best_t = 1e300;
+  // deepest first; no shallower ones once a depth gives four waves of units (they
+  // only add halo planes, and the first call on a mesh waits for this choice)
+  std::vector<int> cands = {1 << 20, 64, 48, 40, 32, 24, 20, 16, 12};
+  for (int n = 2; n <= 16 && (tall + n - 1) / n >= 4; ++n) cands.push_back((tall + n - 1) / n);
+  std::sort(cands.begin(), cands.end(), std::greater<int>());
+  cands.erase(std::unique(cands.begin(), cands.end()), cands.end());
+  for (int zb : cands) {
+    if (zb < (1 << 20) && zb > tall) continue;  // whole columns again
+    long long units = 0;
+    for (auto &t : m->tile_z)
+      if (t.y >= 0) units += (t.y - t.x + zb) / zb;
+    units *= chunks;
+    if (units >= 6LL * m->num_sms && zb == 1 << 20) {
+      best = zb;
+      break;
+    }
     const double t = pass_makespan(m, 16, zb, chunks, m->num_sms, TMEM_UNIT_EXTRA);
-    if (t < best.second) best = {zb, t};
+    if (t < best_t) best = zb, best_t = t;
+    if (units >= 4LL * m->num_sms) break;
   }
   m->zb_single[key] = best;
   return best;
-}
-
-// Whether the tensor-memory pass is expected to be faster than the pass
-// `other` would choose for this width.
-bool prefer_tmem(const hpsi_mesh *m, int dtype, long long ld, const PassShape &other) {
-  (void)dtype;
-  (void)other;
-  return m != nullptr && ld > 0;
 }
 
 // z block depth of a single-system pass of a shape: the simulated choice for
@@ -1102,9 +1100,9 @@ bool prefer_tmem(const hpsi_mesh *m, int dtype, long long ld, const PassShape &o
 int pass_zb(const hpsi_mesh *m, const PassShape &sh, int dtype, int chunks) {
   const int ty = sh.blk ? sh.ty : 16;
   const PassShape b = blk_shape(dtype);
-  if (sh.tmem) return choose_zb_tmem(m, chunks).first;
-  if (sh.blk && ty == 8 && sh.sc == b.sc) return choose_zb_single(m, chunks, 1).first;
-  if (sh.blk && ty == 8 && sh.sc == b.sc / 2 && sh.rx == 1 && sh.ry == 4) return choose_zb_single(m, chunks, 2).first;
+  if (sh.tmem) return choose_zb_tmem(m, chunks);
+  if (sh.blk && ty == 8 && sh.sc == b.sc) return choose_zb_single(m, chunks, 1);
+  if (sh.blk && ty == 8 && sh.sc == b.sc / 2 && sh.rx == 1 && sh.ry == 4) return choose_zb_single(m, chunks, 2);
   return choose_zb(m, chunks, ty);
 }
 
@@ -1373,16 +1371,23 @@ hpsi_status run_ket(hpsi_hamiltonian *h, const T *proj, long long ld, int nst, T
 }
 
 // Shape of the fused pass for a batch: the autotuned one when it matches, else
-// the tensor-memory pass or the default of the width, whichever is expected to
-// be faster on this mesh.
+// the tensor-memory pass wherever the rows are 16-byte pieces, but for batches of
+// at most a quarter of its chunk on large meshes, where it would work on empty
+// lanes.  Pass alone in us, the width's other shape / tensor-memory pass:
+//   width (FP64)     1          2          4          6           8           32
+//   48^3 box     26.2 / 17.1 28.8 / 17.2 27.2 / 17.2 28.8 / 17.3 37.2 / 17.1  49.9 / 34.8
+//   R = 8 sphere 25.8 / 31.6 29.1 / 31.8 37.1 / 31.9 78.7 / 32.8 49.1 / 32.4 147.5 / 94.8
+//   R = 12       51.3 / 80.4 81.7 / 81.1 87.2 / 82.6  178 / 84.4  131 / 82.7   406 / 273
+// (FP32 alike at twice the widths; below 48^3 points the tensor-memory pass takes
+// 16-17 us, the others 24-37.)
 PassShape pass_shape(const hpsi_hamiltonian *h, int dtype, long long ld) {
   const auto &t = h->tuned[dtype == HPSI_C128 ? 0 : 1];
   if (std::getenv(dtype == HPSI_C128 ? "HPSI_PASS_SHAPE64" : "HPSI_PASS_SHAPE32")) return default_shape(dtype, ld);
   if (t.ld == ld) return t.shape;
-  const PassShape s = default_shape(dtype, ld);
-  const bool rows16 = dtype == HPSI_C128 || ld % 2 == 0;  // 16-byte rows
-  if (rows16 && prefer_tmem(h->mesh, dtype, ld, s)) return tmem_shape(dtype);
-  return s;
+  const PassShape s = tmem_shape(dtype);
+  const bool rows16 = dtype == HPSI_C128 || ld % 2 == 0;
+  const bool narrow = 4 * ld <= s.sc && h->mesh->np > 200000;
+  return rows16 && !narrow ? s : default_shape(dtype, ld);
 }
 
 // Arguments of one fused pass (no launch).  in: rows to stencil; out: result

@@ -1,6 +1,7 @@
 // Handle layouts behind the opaque C types of hpsi.h.
 #pragma once
 
+#include <atomic>
 #include <map>
 #include <vector>
 
@@ -39,6 +40,8 @@ struct Workspace {
 
 }  // namespace hpsi
 
+constexpr int MESH_STATUS_WORDS = 256;
+
 struct hpsi_mesh {
   int np = 0, np_part = 0, order = 4, periodic = 0;
   hpsi::CellBox box{};
@@ -60,9 +63,9 @@ struct hpsi_mesh {
   // work list per (z block depth, tile height): key 2 * zb + (height == 8)
   std::map<int, std::pair<int4 *, int>> items;
   std::map<int, std::vector<int4>> items_h;  // the same lists on the host
-  // z block depth of a single-system pass and its simulated makespan, per state
-  // chunk count and kernel (4 * chunks + resident CTAs, 0: tensor-memory pass)
-  mutable std::map<int, std::pair<int, double>> zb_single;
+  // z block depth of a single-system pass, per state chunk count and kernel
+  // (4 * chunks + resident CTAs, 0: tensor-memory pass)
+  mutable std::map<int, int> zb_single;
   // domain-parallel meshes: rows [ghost_first, ghost_first + ghost_count) hold
   // other partitions' points; work lists split into the tiles/planes whose
   // stencil reads no ghost row (part 1) and the rest (part 2), per (zb, ty)
@@ -73,6 +76,9 @@ struct hpsi_mesh {
   std::vector<int> cell_row_h;
   std::map<const int *, unsigned long long *> seg_masks;
   int2 *d_col_z = nullptr;  // per (y, x) cell column: z range of its inner points
+  // status words of the Hamiltonians' bounded waits (after d_col_z's table)
+  int *d_status = nullptr;
+  std::atomic<unsigned> next_status{0};
 };
 
 struct hpsi_hamiltonian {
@@ -88,6 +94,7 @@ struct hpsi_hamiltonian {
   int *d_src_phase = nullptr;
   // KB projectors
   int nmat = 0, nprojections = 0, max_nproj = 0;
+  void *kb_tables = nullptr;  // one allocation for the tables of the projectors
   int4 *d_mat = nullptr;
   int *d_proj_row = nullptr, *d_map = nullptr;
   double *d_pt = nullptr, *d_scal = nullptr;

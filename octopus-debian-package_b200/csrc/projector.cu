@@ -157,17 +157,25 @@ __global__ void __launch_bounds__(128) bra_dmma_kernel(const ProjArgs p) {
   }
 }
 
-// proj[j][l] = scal[j] * sum_z partial[z][j][l]  (one thread per real lane;
-// FP64 sums, rounded once to the storage type)
+// proj[j][l] = scal[j] * sum_z partial[z][j][l]: block (32, 8), 32 real lanes by
+// 8 slices of the splits, folded in a fixed order (FP64 sums, rounded once to
+// the storage type).  One thread per lane waited for up to 32 loads in turn.
 template <typename T>
-__global__ void bra_reduce_kernel(const ProjArgs p, int ksplit) {
+__global__ void __launch_bounds__(256) bra_reduce_kernel(const ProjArgs p, int ksplit) {
+  __shared__ double red[8][32];
   const long long n = (long long)p.nprojections * 2 * p.proj_ld;
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int j = int(i / (2 * p.proj_ld));
+  const long long i = blockIdx.x * 32LL + threadIdx.x;
   double acc = 0.0;
-#pragma unroll 8
-  for (int z = 0; z < ksplit; ++z) acc += p.partial[(long long)z * n + i];
+  if (i < n) {
+#pragma unroll 4
+    for (int z = threadIdx.y; z < ksplit; z += 8) acc += p.partial[(long long)z * n + i];
+  }
+  red[threadIdx.y][threadIdx.x] = acc;
+  __syncthreads();
+  if (threadIdx.y != 0 || i >= n) return;
+#pragma unroll
+  for (int z = 1; z < 8; ++z) acc += red[z][threadIdx.x];
+  const int j = int(i / (2 * p.proj_ld));
   static_cast<T *>(p.proj)[i] = T(acc * p.scal64[j]);
 }
 
@@ -255,7 +263,7 @@ hpsi_status launch_bra(const ProjArgs &p, bool use_tensor, int ksplit, cudaStrea
       bra_dmma_kernel<T, false><<<grid, 128, 0, st>>>(p);
     HPSI_CHECK_LAUNCH();
     const long long n = (long long)p.nprojections * ld2;
-    bra_reduce_kernel<T><<<unsigned((n + 255) / 256), 256, 0, st>>>(p, ksplit);
+    bra_reduce_kernel<T><<<unsigned((n + 31) / 32), dim3(32, 8), 0, st>>>(p, ksplit);
     HPSI_CHECK_LAUNCH();
     return HPSI_OK;
   }
@@ -429,12 +437,13 @@ __global__ void __launch_bounds__(256) ket_kernel(const KetArgs k) {
 namespace {
 constexpr int KET_ROWS = 32;
 template <typename T, typename C2, bool PHASE, int SW>
-__global__ void __launch_bounds__(256) ket_block_kernel(const KetArgs k) {
-  constexpr int RPT = KET_ROWS * SW / 256;  // rows per thread
+__global__ void __launch_bounds__(256, PHASE ? 2 : 4) ket_block_kernel(const KetArgs k) {
+  constexpr int HALVES = SW >= 64 ? 2 : 1;           // sweeps over the block's rows: fewer registers, more CTAs per SM
+  constexpr int RPT = KET_ROWS * SW / 256 / HALVES;  // rows per thread and sweep
   extern __shared__ __align__(16) unsigned char ksm[];
   C2 *sp = reinterpret_cast<C2 *>(ksm);                  // [nproj][SW]
   T *sw = reinterpret_cast<T *>(sp + k.max_nproj * SW);  // [rows of the block][nproj]
-  const int t = threadIdx.x, sl = t % SW, r0 = (t / SW) * RPT;
+  const int t = threadIdx.x, sl = t % SW;
   const int sbase = blockIdx.x * SW, s = sbase + sl;
   const bool act = s < k.nst;
   const C2 *proj = static_cast<const C2 *>(k.proj);
@@ -446,6 +455,10 @@ __global__ void __launch_bounds__(256) ket_block_kernel(const KetArgs k) {
   for (int b = b0; b < b1; ++b) {
     const int4 D = __ldg(k.blk + b);  // {first covered row, rows + 256 * entries per row, first entry, value offset}
     const int cnt = D.y & 255, ne = D.y >> 8;
+#pragma unroll 1
+    for (int half = 0; half < HALVES; ++half) {
+    const int r0 = half * (KET_ROWS / HALVES) + (t / SW) * RPT;
+    if (half && cnt <= KET_ROWS / HALVES) break;  // (the same for the whole CTA)
     const T *w = static_cast<const T *>(k.pk) + D.w;
     int row[RPT];
     C2 y[RPT], h[RPT];
@@ -461,17 +474,20 @@ __global__ void __launch_bounds__(256) ket_block_kernel(const KetArgs k) {
     for (int e = 0; e < ne; ++e) {
       const int4 E = __ldg(k.ent + D.z + e);  // (the first row's entry: projection row and count of the matrix)
       const int np = E.z;
-      __syncthreads();  // the matrix before has been read
-      for (int i = t; i < cnt * np; i += 256) sw[i] = w[i];
-      for (int i = t; i < np * SW; i += 256) {
-        const int c = sbase + i % SW;
-        C2 v;
-        v.x = 0;
-        v.y = 0;
-        if (c < k.nst) v = proj[(long long)(E.y + i / SW) * k.proj_ld + c];
-        sp[i] = v;
+      // one matrix: the second sweep finds it staged
+      if (half == 0 || ne > 1) {
+        __syncthreads();  // the matrix before has been read
+        for (int i = t; i < cnt * np; i += 256) sw[i] = w[i];
+        for (int i = t; i < np * SW; i += 256) {
+          const int c = sbase + i % SW;
+          C2 v;
+          v.x = 0;
+          v.y = 0;
+          if (c < k.nst) v = proj[(long long)(E.y + i / SW) * k.proj_ld + c];
+          sp[i] = v;
+        }
+        __syncthreads();
       }
-      __syncthreads();
       if (row[0] >= 0) {
         const T *wr = sw + r0 * np;
         C2 g[RPT];
@@ -522,6 +538,7 @@ __global__ void __launch_bounds__(256) ket_block_kernel(const KetArgs k) {
         const C2 x = psi0[(long long)row[q] * k.psi0_ld + s];
         kadd(ke, double(x.x) * double(h[q].x) + double(x.y) * double(h[q].y));
       }
+    }
     }
   }
   if (k.obs) {
@@ -585,8 +602,12 @@ hpsi_status launch_ket(const KetArgs &k, cudaStream_t st) {
   const int rb = k.row_blocks > 0 ? std::min(k.row_blocks, ket_row_blocks(k.nk)) : ket_row_blocks(k.nk);
   // the fused density needs the row's states in one warp (the form above); so
   // do matrices whose projections would not fit shared memory
-  if (!k.rho_ket && k.blk && size_t(k.max_nproj) * (64 * sizeof(C2) + KET_ROWS * sizeof(T)) <= 200 * 1024)
-    return k.phase ? launch_ket_blocks_w<T, C2, true>(k, rb, st) : launch_ket_blocks_w<T, C2, false>(k, rb, st);
+  if (!k.rho_ket && k.blk && size_t(k.max_nproj) * (64 * sizeof(C2) + KET_ROWS * sizeof(T)) <= 200 * 1024) {
+    // a CTA per block, but where the energy partials count the CTA rows or the
+    // launch shares the GPU
+    const int rows = k.obs || k.row_blocks > 0 ? rb : std::min(k.nblk, 65535);
+    return k.phase ? launch_ket_blocks_w<T, C2, true>(k, rows, st) : launch_ket_blocks_w<T, C2, false>(k, rows, st);
+  }
   dim3 grid((k.nst + 63) / 64, rb);  // two states per thread
   // narrow batches: several rows per warp
   const int rpw = k.nst <= 8 ? 4 : k.nst <= 16 ? 2 : 1;

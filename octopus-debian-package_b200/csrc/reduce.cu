@@ -315,19 +315,27 @@ __global__ void __launch_bounds__(512) cholesky_inverse_smem_kernel(const double
     for (int i = lane; i <= j; i += 32)
       M[at(i, j)] = make_double2(S[2 * ((long long)i * nst + j)], S[2 * ((long long)i * nst + j) + 1]);
   __syncthreads();
+  double2 *v = M + nst * (nst + 1) / 2;               // a new column of the inverse
+  double *rinv = reinterpret_cast<double *>(v + nst);  // 1 / U(j, j)
   for (int j = 0; j < nst; ++j) {
-    double d = M[at(j, j)].x;
-    __syncthreads();
-    if (!(d > 0.0)) {
-      if (t == 0) err[0] = 1;
-      d = 1.0;
+    // one thread takes the root and the reciprocal (every warp's square root
+    // would occupy the FP64 pipe for longer than the step's updates)
+    if (t == 0) {
+      double d = M[at(j, j)].x;
+      if (!(d > 0.0)) {
+        err[0] = 1;
+        d = 1.0;
+      }
+      const double r = sqrt(d);
+      M[at(j, j)] = make_double2(r, 0.0);
+      rinv[j] = 1.0 / r;
     }
-    const double r = sqrt(d);
-    if (t == 0) M[at(j, j)] = make_double2(r, 0.0);
+    __syncthreads();
+    const double ri = rinv[j];
     for (int c = j + 1 + t; c < nst; c += blockDim.x) {
       double2 &x = M[at(j, c)];
-      x.x /= r;
-      x.y /= r;
+      x.x *= ri;
+      x.y *= ri;
     }
     __syncthreads();
     // trailing update: M(i, c) -= conj(U(j, i)) U(j, c)
@@ -351,9 +359,8 @@ __global__ void __launch_bounds__(512) cholesky_inverse_smem_kernel(const double
   __syncthreads();
   // column j of the inverse: -X(0..j-1, 0..j-1) U(0..j-1, j) / U(j, j), X the
   // inverse of the leading block (four lanes per row: all rows at once)
-  double2 *v = M + nst * (nst + 1) / 2;  // the new column
   for (int j = 0; j < nst; ++j) {
-    const double d = M[at(j, j)].x;
+    const double ri = rinv[j];
     for (int i0 = 0; i0 < j; i0 += blockDim.x / 4) {
       const int i = i0 + t / 4;
       double sr = 0.0, si = 0.0;
@@ -370,11 +377,11 @@ __global__ void __launch_bounds__(512) cholesky_inverse_smem_kernel(const double
         sr += __shfl_xor_sync(0xffffffffu, sr, o);
         si += __shfl_xor_sync(0xffffffffu, si, o);
       }
-      if (i < j && (t & 3) == 0) v[i] = make_double2(-sr / d, -si / d);
+      if (i < j && (t & 3) == 0) v[i] = make_double2(-sr * ri, -si * ri);
     }
     __syncthreads();
     for (int i = t; i < j; i += blockDim.x) M[at(i, j)] = v[i];
-    if (t == 0) M[at(j, j)] = make_double2(1.0 / d, 0.0);
+    if (t == 0) M[at(j, j)] = make_double2(ri, 0.0);
     __syncthreads();
   }
   for (int j = warp; j < nst; j += nw)
@@ -592,7 +599,7 @@ hpsi_status launch_gram(const T *a, long long lda, const T *b, long long ldb, in
 }
 
 hpsi_status launch_cholesky_inverse(const double *S, int nst, double *U, double *Uinv, int *err, cudaStream_t st) {
-  const size_t smem = (size_t(nst) * (nst + 1) / 2 + nst) * sizeof(double2);
+  const size_t smem = (size_t(nst) * (nst + 1) / 2 + nst) * sizeof(double2) + size_t(nst) * sizeof(double);
   if (smem <= 226 * 1024) {
     static std::once_flag once;
     static cudaError_t attr = cudaSuccess;

@@ -47,16 +47,26 @@ constexpr int TM_SIDE = 2 * TM_HAL * TM_TY;           // cells left and right of
 constexpr int TM_SC = TM_BAND + TM_SIDE;              // star cells of a plane
 constexpr int TM_NC = 256, TM_NP = 128;               // consumer, producer threads
 // registers a thread: at launch (the whole CTA's share), after the split
-constexpr int TM_LREG = 168, TM_CREG = 216, TM_PREG = 72;
+constexpr int TM_LREG = 168, TM_CREG = 208, TM_PREG = 88;
+// (the grouped pass, whose arguments are indexed by system, needs more registers
+// in its consumers)
+constexpr int TM_GCREG = 216, TM_GPREG = 72;
 static_assert(TM_NC * TM_CREG + TM_NP * TM_PREG <= (TM_NC + TM_NP) * TM_LREG, "registers of the split");
+static_assert(TM_NC * TM_GCREG + TM_NP * TM_GPREG <= (TM_NC + TM_NP) * TM_LREG, "registers of the grouped split");
 constexpr int TM_NBUF = 3;
 constexpr size_t TM_OV = size_t(TM_SC) * TM_CELLB;              // centre weights of the plane
-constexpr size_t TM_OROW = TM_OV + TM_TX * TM_TY * sizeof(double);  // output rows four planes below
-constexpr size_t TM_STAGE = TM_OROW + TM_TX * TM_TY * sizeof(int);
+constexpr size_t TM_STAGE = TM_OV + TM_TX * TM_TY * sizeof(double);
 constexpr size_t TM_OBS = TM_NBUF * TM_STAGE;                   // observable sums of the consumers
 constexpr size_t TM_OBSB = size_t(TM_NC) * 3 * sizeof(double);
 constexpr size_t TM_MAP = TM_OBS + TM_OBSB;                     // load map entries of the producers
-constexpr size_t TM_BAR = TM_MAP + 3 * TM_SC * sizeof(int);     // (rows, and two planes of entries with Bloch phases)
+constexpr size_t TM_PH = TM_MAP + 3 * TM_SC * sizeof(int);       // (rows, two planes of entries), phases of a plane's images
+// output rows four planes below, in a ring of their own: they are read after the
+// stage has been handed back.  Four slots: a plane's rows are overwritten by those
+// of the fourth plane after it, whose copies wait for every warp to hand back the
+// next plane's stage, that is to be done with this plane
+constexpr size_t TM_ROWB = TM_TX * TM_TY * sizeof(int);
+constexpr size_t TM_OROW = TM_PH + size_t(TM_SC) * 16;
+constexpr size_t TM_BAR = TM_OROW + 4 * TM_ROWB;
 constexpr size_t TM_BYTES = TM_BAR + 2 * TM_NBUF * 8 + 16;
 static_assert(TM_BYTES <= 232448, "shared memory per CTA");
 static_assert(TM_STAGE % 128 == 0 && TM_BAR % 16 == 0, "alignment");
@@ -124,8 +134,13 @@ __device__ __forceinline__ float2 escale(float w, float2 v) { return make_float2
 struct TmemRing {
   int slot = 0;
   unsigned phase = 0;
+  unsigned n = 0;     // planes so far (rows ring)
   bool dead = false;  // a wait has given up: no further waits
+  __device__ __forceinline__ int *rows(unsigned char *smem) const {
+    return reinterpret_cast<int *>(smem + TM_OROW + (n & 3u) * TM_ROWB);
+  }
   __device__ __forceinline__ void next() {
+    ++n;
     if (++slot == TM_NBUF) {
       slot = 0;
       phase ^= 1u;
@@ -157,7 +172,8 @@ __device__ __forceinline__ uint64_t *smem_bar(unsigned char *smem, int b) {
 // TMA: a run of eight cells of a halo row that are eight consecutive rows of
 // the batch (bit of p.seg_mask; segments of the tile's columns only) arrives as
 // one box copy of 8 rows x 128 bytes on the stage's full barrier.
-template <typename T, bool TMA = false>
+// PH: the pass has Bloch phases.
+template <typename T, bool TMA, bool PH>
 __device__ __forceinline__ void tmem_produce(const PassArgs &p, const int ih, const int chunk, unsigned char *smem,
                                              TmemRing &ring, const CUtensorMap *tm = nullptr) {
   constexpr int HAL = TM_HAL;
@@ -190,6 +206,7 @@ __device__ __forceinline__ void tmem_produce(const PassArgs &p, const int ih, co
   constexpr int EPP = 16 / int(sizeof(T));
   // pieces past the batch width are zero-filled
   const bool pok = piece * EPP < left;
+  const int csize = pok ? 16 : 0;
   const T *in_base = static_cast<const T *>(p.in) + (pok ? col + piece * EPP : 0);
   const char *in_bytes = reinterpret_cast<const char *>(in_base);
   const unsigned in_rb = unsigned(2 * p.in_ld) * unsigned(sizeof(T));
@@ -209,14 +226,33 @@ __device__ __forceinline__ void tmem_produce(const PassArgs &p, const int ih, co
   // copied like any other row; the copy is multiplied by the point's phase in
   // shared memory once it has landed, one plane after it was issued, before the
   // stage is handed over (`ent`: the plane's entries, double-buffered)
-  const bool phased = p.phase_corr != nullptr;
   int4 *mapw = reinterpret_cast<int4 *>(smem + TM_MAP) + 32 * pw;  // this warp's rows of the plane
-  int4 *ent = mapw + TM_SC / 4;
+  [[maybe_unused]] int4 *ent = mapw + TM_SC / 4;
   auto image = [&](int e) { return e >= -1 ? e : __ldg(p.per_inner - (e + 2)); };
-  int pslot = -1, pq0 = 0, pq1 = 0, pent = 0;  // plane waiting for its phases
-  auto finish = [&]() {
+  [[maybe_unused]] auto images4 = [&](const int4 &e) { return PH ? make_int4(image(e.x), image(e.y), image(e.z), image(e.w)) : e; };
+  // phases of this warp's images, staged before the plane is finished
+  using C = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+  [[maybe_unused]] C *phw = reinterpret_cast<C *>(smem + TM_PH) + 128 * pw;
+  [[maybe_unused]] auto phase_of = [&](int e) {
+    C c;
+    c.x = 1;
+    c.y = 0;
+    return e >= -1 ? c : __ldg(static_cast<const C *>(p.phase_corr) - ((long long)e + 2));
+  };
+  [[maybe_unused]] int pslot = -1, pq0 = 0, pq1 = 0, pent = 0;  // plane waiting for its phases
+  [[maybe_unused]] auto finish = [&]() {
     unsigned char *d0 = smem + size_t(pslot) * TM_STAGE + (size_t(128 * pw) + 4 * sub) * TM_CELLB + piece * 16;
     const int4 *pe = ent + pent * (TM_SC / 4);
+    if (pq1 > pq0) {
+      const int4 e = pe[lane];
+      const C c0 = phase_of(e.x), c1 = phase_of(e.y), c2 = phase_of(e.z), c3 = phase_of(e.w);
+      __syncwarp();
+      phw[4 * lane] = c0;
+      phw[4 * lane + 1] = c1;
+      phw[4 * lane + 2] = c2;
+      phw[4 * lane + 3] = c3;
+      __syncwarp();
+    }
     for (int g = pq0; g < pq1; ++g) {
       const int4 m4 = pe[4 * g + sub];
       const int src[4] = {m4.x, m4.y, m4.z, m4.w};
@@ -224,14 +260,12 @@ __device__ __forceinline__ void tmem_produce(const PassArgs &p, const int ih, co
       for (int j = 0; j < 4; ++j) {
         if (src[j] >= -1 || !pok) continue;
         T *e = reinterpret_cast<T *>(d0 + size_t(16 * g + j) * TM_CELLB);
-        const long long bp = -((long long)src[j] + 2);
-        const T pr = static_cast<const T *>(p.phase_corr)[2 * bp];
-        const T pi = static_cast<const T *>(p.phase_corr)[2 * bp + 1];
+        const C ph = phw[16 * g + 4 * sub + j];
 #pragma unroll
         for (int i = 0; i < EPP; i += 2) {
           const T xr = e[i], xi = e[i + 1];
-          e[i] = xr * pr - xi * pi;
-          e[i + 1] = xr * pi + xi * pr;
+          e[i] = xr * ph.x - xi * ph.y;
+          e[i + 1] = xr * ph.y + xi * ph.x;
         }
       }
     }
@@ -240,8 +274,24 @@ __device__ __forceinline__ void tmem_produce(const PassArgs &p, const int ih, co
   };
 
   auto entries = [&](int q) { return *reinterpret_cast<const int4 *>(map + (long long)q * planeN); };
-  int4 nxt = entries(zbeg);
-  double2 vnxt = v_load(zbeg);
+  // The loads of the next planes: an arrival (release) waits for the thread's
+  // loads in flight.  In the first planes they are issued after it, so that the
+  // ring fills at once; later before it, which holds the next plane's copies back
+  // until the consumers are past their shared-memory loads (R = 12 sphere, 128
+  // states, FP64: 0.98 ms; issued after it throughout: 1.14 ms, and in the small
+  // boxes of 6-plane units 0.026 -> 0.024 ms).
+  int4 cur = entries(zbeg), nxt = nplanes > 1 ? entries(zbeg + 1) : cur;
+  int4 rows = images4(cur);
+  double2 v = v_load(zbeg), vnxt = v_load(zbeg + 1);
+  auto advance = [&](int k) {
+    cur = nxt;
+    rows = images4(cur);
+    v = vnxt;
+    if (k + 2 < nplanes) {
+      nxt = entries(zbeg + k + 2);
+      vnxt = v_load(zbeg + k + 2);
+    }
+  };
   for (int k = 0; k < nplanes; ++k) {
     const int q = zbeg + k;
     const bool inner = q >= zs && q < ze;  // the in-plane halo is read for output planes only
@@ -249,21 +299,16 @@ __device__ __forceinline__ void tmem_produce(const PassArgs &p, const int ih, co
     const int q0 = inner ? 0 : pw == 0 ? 4 : pw == 3 ? 8 : 0;
     const int q1 = inner ? 8 : pw == 2 ? 4 : 8;
     __syncwarp();  // the plane before has read its entries
-    if (phased) {
-      ent[(k & 1) * (TM_SC / 4) + lane] = nxt;
-      mapw[lane] = make_int4(image(nxt.x), image(nxt.y), image(nxt.z), image(nxt.w));
-    } else {
-      mapw[lane] = nxt;
+    mapw[lane] = PH ? rows : cur;
+    [[maybe_unused]] bool images = false;  // whether the plane's rounds hold an image (uniform in the warp)
+    if constexpr (PH) {
+      ent[(k & 1) * (TM_SC / 4) + lane] = cur;
+      images = __any_sync(0xffffffffu, lane >= 4 * q0 && lane < 4 * q1 &&
+                                           (cur.x < -1 || cur.y < -1 || cur.z < -1 || cur.w < -1));
     }
-    // whether the plane's rounds hold an image (uniform in the warp)
-    const bool mine = lane >= 4 * q0 && lane < 4 * q1 && (nxt.x < -1 || nxt.y < -1 || nxt.z < -1 || nxt.w < -1);
-    const bool images = phased && __any_sync(0xffffffffu, mine);
     __syncwarp();
-    const double2 v = vnxt;
-    if (k + 1 < nplanes) {
-      nxt = entries(q + 1);
-      vnxt = v_load(q + 1);
-    }
+    const double2 vk = v;
+    if (k >= TM_NBUF) advance(k);
     const int b = ring.slot;
     ring.wait<true>(smem_bar<true>(smem, b), ring.phase ^ 1u, p.err);  // the first round passes at once
     unsigned char *st = smem + size_t(b) * TM_STAGE;
@@ -283,15 +328,14 @@ __device__ __forceinline__ void tmem_produce(const PassArgs &p, const int ih, co
       if constexpr (TMA)
         if ((boxes >> (2 * g + (sub >> 1))) & 1u) continue;  // these cells arrive with their segment's box
       const int4 m4 = mapw[4 * g + sub];
-      int src[4] = {m4.x, m4.y, m4.z, m4.w};
-      if (!pok) src[0] = src[1] = src[2] = src[3] = -1;
+      const int src[4] = {m4.x, m4.y, m4.z, m4.w};
       unsigned char *d = dst + size_t(16 * g) * TM_CELLB;
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        cp_async16_zfill(d + j * TM_CELLB, in_bytes + size_t(unsigned(max(src[j], 0))) * in_rb, src[j] >= 0 ? 16 : 0);
+        cp_async16_zfill(d + j * TM_CELLB, in_bytes + size_t(unsigned(max(src[j], 0))) * in_rb, src[j] >= 0 ? csize : 0);
     }
     if (inner) {
-      double2 c = v;
+      double2 c = vk;
       if (has_field) {
         const double f = fxy + fz * double(q + B.lo[2]);
         c.x += f;
@@ -303,8 +347,8 @@ __device__ __forceinline__ void tmem_produce(const PassArgs &p, const int ih, co
       cw[1] = w0 + static_cast<T>(c.y);
     }
     if (pt < 64 && q - HAL >= zs)
-      cp_async16(reinterpret_cast<int *>(st + TM_OROW) + 4 * pt, p.cell_row + (long long)(q - HAL) * planeN + r_src);
-    if (phased) {
+      cp_async16(ring.rows(smem) + 4 * pt, p.cell_row + (long long)(q - HAL) * planeN + r_src);
+    if constexpr (PH) {
       cp_async_commit();
       if (pslot >= 0) {
         cp_async_wait<1>();
@@ -319,10 +363,13 @@ __device__ __forceinline__ void tmem_produce(const PassArgs &p, const int ih, co
       if (!TMA || lane != 0) mbar_arrive(smem_bar<false>(smem, b));
     }
     ring.next();
+    if (k < TM_NBUF) advance(k);
   }
-  if (phased && pslot >= 0) {
-    cp_async_wait<0>();
-    finish();
+  if constexpr (PH) {
+    if (pslot >= 0) {
+      cp_async_wait<0>();
+      finish();
+    }
   }
 }
 
@@ -330,10 +377,11 @@ __device__ __forceinline__ void tmem_produce(const PassArgs &p, const int ih, co
 // CROSS: Horner pass on real lanes with a purely imaginary factor: the lane
 // that holds one part of H psi writes the other part of the output, so the
 // lanes exchange nothing.
+// pw: the arguments that hold the weights (at a fixed parameter address).
 // RHO: also the density of the outputs, per row and chunk (p.rho_part).
 template <typename T, bool HORNER, bool OBS, bool CROSS, bool RHO>
-__device__ __forceinline__ void tmem_consume(const PassArgs &p, const int ih, const int chunk, unsigned char *smem,
-                                             const uint32_t tm_base, TmemRing &ring) {
+__device__ __forceinline__ void tmem_consume(const PassArgs &p, const PassArgs &pw, const int ih, const int chunk,
+                                             unsigned char *smem, const uint32_t tm_base, TmemRing &ring) {
   constexpr bool CPLX = sizeof(T) == 4;
   constexpr bool X0 = HORNER || OBS;
   using E = typename BlkElem<T, CPLX>::E;
@@ -402,6 +450,7 @@ __device__ __forceinline__ void tmem_consume(const PassArgs &p, const int ih, co
     const int pz = zbeg + k;
     ring.wait<false>(smem_bar<false>(smem, b), ring.phase, p.err);
     const unsigned char *st = smem + size_t(b) * TM_STAGE;
+    const int *rows = ring.rows(smem);
     const bool need = pz >= ws - HAL && pz < we + HAL;  // warp-uniform
     const bool work = need && pz >= ws;
     const bool emit = work && pz - HAL >= ws;  // output plane pz - 4 completes here
@@ -416,8 +465,7 @@ __device__ __forceinline__ void tmem_consume(const PassArgs &p, const int ih, co
     }
     if (emit) {
       // rows of the output plane
-      [[maybe_unused]] const int *rows = reinterpret_cast<const int *>(st + TM_OROW);
-      if constexpr (X0) {
+            if constexpr (X0) {
         // lane i of a cell group fetches cell i's psi0 line to L2: it is read
         // after the in-plane arms (a load in flight across the hand-over of
         // the stage would delay it)
@@ -431,7 +479,57 @@ __device__ __forceinline__ void tmem_consume(const PassArgs &p, const int ih, co
 #pragma unroll
       for (int i = 0; i < 16; ++i) a[i] = ezero<E>();
       if (pz < we) {
-        // centre, potential and the arms inside the 4 x 4 block
+        // the arms inside the 4 x 4 block
+#pragma unroll
+        for (int i = 0; i < R * R; ++i)
+          a[i] = escale(wsel_t<T>(pw.wx, pw.wxf, (i & 1) ? 3 : 5), c[i ^ 1]);
+#pragma unroll
+        for (int d = 1; d < R; ++d)
+#pragma unroll
+          for (int i = 0; i < R; ++i)
+#pragma unroll
+            for (int j = 0; j + d < R; ++j) {
+              // cells j and j + d of a row / column i
+              if (d > 1 || j % 2 == 1) {  // (the others came first)
+                a[i * R + j] = fmae(wsel_t<T>(pw.wx, pw.wxf, 4 + d), c[i * R + j + d], a[i * R + j]);
+                a[i * R + j + d] = fmae(wsel_t<T>(pw.wx, pw.wxf, 4 - d), c[i * R + j], a[i * R + j + d]);
+              }
+              a[j * R + i] = fmae(wsel_t<T>(pw.wy, pw.wyf, 4 + d), c[(j + d) * R + i], a[j * R + i]);
+              a[(j + d) * R + i] = fmae(wsel_t<T>(pw.wy, pw.wyf, 4 - d), c[j * R + i], a[(j + d) * R + i]);
+            }
+        // y arms from above and below the block
+#pragma unroll
+        for (int i = 0; i < HAL; ++i)
+#pragma unroll
+          for (int cx = 0; cx < R; ++cx) {
+            const E lo = *reinterpret_cast<const E *>(st + own + ((i - HAL) * TM_TX + cx) * TM_CELLB);
+            const E hi = *reinterpret_cast<const E *>(st + own + ((i + R) * TM_TX + cx) * TM_CELLB);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              if (i - HAL - r >= -HAL)
+                a[r * R + cx] = fmae(wsel_t<T>(pw.wy, pw.wyf, i - r), lo, a[r * R + cx]);
+              if (i + R - r <= HAL)
+                a[r * R + cx] = fmae(wsel_t<T>(pw.wy, pw.wyf, i + R - r + 4), hi, a[r * R + cx]);
+            }
+          }
+        // x arms from left and right of the block
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int i = 0; i < HAL; ++i) {
+            const E lo = *reinterpret_cast<const E *>(st + lefto + r * lstep + i * TM_CELLB);
+            const E hi = *reinterpret_cast<const E *>(st + righto + r * rstep + i * TM_CELLB);
+#pragma unroll
+            for (int cx = 0; cx < R; ++cx) {
+              if (i - HAL - cx >= -HAL)
+                a[r * R + cx] = fmae(wsel_t<T>(pw.wx, pw.wxf, i - cx), lo, a[r * R + cx]);
+              if (i + R - cx <= HAL)
+                a[r * R + cx] = fmae(wsel_t<T>(pw.wx, pw.wxf, i + R - cx + 4), hi, a[r * R + cx]);
+            }
+          }
+        // the centre after the in-plane arms: it cancels most of their sum, so the
+        // z arms are added to a small number (FP32: a third less rounding error than
+        // with the centre first)
         const T *cw = reinterpret_cast<const T *>(st + TM_OV) + by * TM_TX + bx;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -445,53 +543,17 @@ __device__ __forceinline__ void tmem_consume(const PassArgs &p, const int ih, co
             w[0] = t.x, w[1] = t.y, w[2] = u.x, w[3] = u.y;
           }
 #pragma unroll
-          for (int cx = 0; cx < R; ++cx) a[r * R + cx] = escale(w[cx], c[r * R + cx]);
+          for (int cx = 0; cx < R; ++cx) a[r * R + cx] = fmae(w[cx], c[r * R + cx], a[r * R + cx]);
         }
-#pragma unroll
-        for (int d = 1; d < R; ++d)
-#pragma unroll
-          for (int i = 0; i < R; ++i)
-#pragma unroll
-            for (int j = 0; j + d < R; ++j) {
-              // cells j and j + d of a row / column i
-              a[i * R + j] = fmae(wsel_t<T>(p.wx, p.wxf, 4 + d), c[i * R + j + d], a[i * R + j]);
-              a[i * R + j + d] = fmae(wsel_t<T>(p.wx, p.wxf, 4 - d), c[i * R + j], a[i * R + j + d]);
-              a[j * R + i] = fmae(wsel_t<T>(p.wy, p.wyf, 4 + d), c[(j + d) * R + i], a[j * R + i]);
-              a[(j + d) * R + i] = fmae(wsel_t<T>(p.wy, p.wyf, 4 - d), c[j * R + i], a[(j + d) * R + i]);
-            }
-        // y arms from above and below the block
-#pragma unroll
-        for (int i = 0; i < HAL; ++i)
-#pragma unroll
-          for (int cx = 0; cx < R; ++cx) {
-            const E lo = *reinterpret_cast<const E *>(st + own + ((i - HAL) * TM_TX + cx) * TM_CELLB);
-            const E hi = *reinterpret_cast<const E *>(st + own + ((i + R) * TM_TX + cx) * TM_CELLB);
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-              if (i - HAL - r >= -HAL)
-                a[r * R + cx] = fmae(wsel_t<T>(p.wy, p.wyf, i - r), lo, a[r * R + cx]);
-              if (i + R - r <= HAL)
-                a[r * R + cx] = fmae(wsel_t<T>(p.wy, p.wyf, i + R - r + 4), hi, a[r * R + cx]);
-            }
-          }
-        // x arms from left and right of the block
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-#pragma unroll
-          for (int i = 0; i < HAL; ++i) {
-            const E lo = *reinterpret_cast<const E *>(st + lefto + r * lstep + i * TM_CELLB);
-            const E hi = *reinterpret_cast<const E *>(st + righto + r * rstep + i * TM_CELLB);
-#pragma unroll
-            for (int cx = 0; cx < R; ++cx) {
-              if (i - HAL - cx >= -HAL)
-                a[r * R + cx] = fmae(wsel_t<T>(p.wx, p.wxf, i - cx), lo, a[r * R + cx]);
-              if (i + R - cx <= HAL)
-                a[r * R + cx] = fmae(wsel_t<T>(p.wx, p.wxf, i + R - cx + 4), hi, a[r * R + cx]);
-            }
-          }
       }
 
     }
+    // the stage has been read: it is handed back before the z arms, so that the
+    // producers' copies overlap the z arms and not the next plane's loads from
+    // shared memory
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_bar<true>(smem, b));
+
     const uint32_t slot = uint32_t(k & 3) * 32u;
     uint32_t buf[32], buf2[32];
     tm_wait_store();  // of the plane before
@@ -501,7 +563,7 @@ __device__ __forceinline__ void tmem_consume(const PassArgs &p, const int ih, co
           // rows outside the mesh read row 0 (not used)
 #pragma unroll
           for (int r = 0; r < R; ++r) {
-            const int4 v = *reinterpret_cast<const int4 *>(st + TM_OROW + ((by + r) * TM_TX + bx) * 4);
+            const int4 v = *reinterpret_cast<const int4 *>(rows + (by + r) * TM_TX + bx);
             const int row[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int i = 0; i < R; ++i)
@@ -519,13 +581,13 @@ __device__ __forceinline__ void tmem_consume(const PassArgs &p, const int ih, co
       tm_wait_load(buf2);
       unpack(buf, o);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) o[i] = fmae(wsel_t<T>(p.wz, p.wzf, 8), c[i], o[i]);
+      for (int i = 0; i < 16; ++i) o[i] = fmae(wsel_t<T>(pw.wz, pw.wzf, 8), c[i], o[i]);
       auto zarm = [&](auto Jc, const E (&v)[16]) {
         constexpr int J = decltype(Jc)::value;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          a[i] = fmae(wsel_t<T>(p.wz, p.wzf, 4 - J), v[i], a[i]);
-          if (J < HAL) o[i] = fmae(wsel_t<T>(p.wz, p.wzf, 8 - J), v[i], o[i]);
+          a[i] = fmae(wsel_t<T>(pw.wz, pw.wzf, 4 - J), v[i], a[i]);
+          if (J < HAL) o[i] = fmae(wsel_t<T>(pw.wz, pw.wzf, 8 - J), v[i], o[i]);
         }
       };
       tm_load(tm + uint32_t((k - 2) & 3) * 32u, buf);
@@ -553,7 +615,7 @@ __device__ __forceinline__ void tmem_consume(const PassArgs &p, const int ih, co
         int4 rv;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          if (i % R == 0) rv = *reinterpret_cast<const int4 *>(st + TM_OROW + ((by + i / R) * TM_TX + bx) * 4);
+          if (i % R == 0) rv = *reinterpret_cast<const int4 *>(rows + (by + i / R) * TM_TX + bx);
           const int row = i % R == 0 ? rv.x : i % R == 1 ? rv.y : i % R == 2 ? rv.z : rv.w;
           const E h = o[i];
           E val = h;
@@ -608,7 +670,7 @@ __device__ __forceinline__ void tmem_consume(const PassArgs &p, const int ih, co
             }
             if (hi) cell += half;
           }
-          const int row = *reinterpret_cast<const int *>(st + TM_OROW + ((by + cell / R) * TM_TX + bx + cell % R) * 4);
+          const int row = rows[(by + cell / R) * TM_TX + bx + cell % R];
           if (unsigned(row) < unsigned(p.np)) p.rho_part[(long long)chunk * p.np + row] = rc[0];
         }
         if constexpr (OBS) {
@@ -621,9 +683,6 @@ __device__ __forceinline__ void tmem_consume(const PassArgs &p, const int ih, co
       pack(c, buf);
       tm_store(tm + slot, buf);
     }
-    // the stage has been read
-    __syncwarp();
-    if (lane == 0) mbar_arrive(smem_bar<true>(smem, b));
     ring.next();
   }
   tm_wait_store();
@@ -682,7 +741,7 @@ __device__ __forceinline__ void tmem_end(uint32_t tm_base) {
 }
 
 // grid: nitems * chunks
-template <typename T, bool HORNER, bool OBS, bool CROSS, bool RHO, bool TMA>
+template <typename T, bool HORNER, bool OBS, bool CROSS, bool RHO, bool TMA, bool PH>
 __global__ void __launch_bounds__(TM_NC + TM_NP, 1) pass_tmem_kernel(const __grid_constant__ PassArgs p,
                                                                     const __grid_constant__ CUtensorMap tm) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -691,13 +750,13 @@ __global__ void __launch_bounds__(TM_NC + TM_NP, 1) pass_tmem_kernel(const __gri
   TmemRing ring;
   if (threadIdx.x >= TM_NC) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(TM_PREG));
-    tmem_produce<T, TMA>(p, ih, chunk, smem, ring, &tm);
+    tmem_produce<T, TMA, PH>(p, ih, chunk, smem, ring, &tm);
     // the copies have landed before the CTA ends
     cp_async_commit();
     cp_async_wait<0>();
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(TM_CREG));
-    tmem_consume<T, HORNER, OBS, CROSS, RHO>(p, ih, chunk, smem, tm_base, ring);
+    tmem_consume<T, HORNER, OBS, CROSS, RHO>(p, p, ih, chunk, smem, tm_base, ring);
   }
   tmem_end(tm_base);
 }
@@ -705,25 +764,28 @@ __global__ void __launch_bounds__(TM_NC + TM_NP, 1) pass_tmem_kernel(const __gri
 // Many systems in one launch (Horner passes): CTA i takes the units
 // first[i] .. first[i + 1] - 1 of the list; the producers run on into the next
 // unit while the consumers finish one.
-template <typename T>
+// WEQ: every system has the weights of the first (equal spacings): they are
+// read at a fixed parameter address instead of through the system's index.
+template <typename T, bool PH, bool WEQ>
 __global__ void __launch_bounds__(TM_NC + TM_NP, 1) pass_tmem_group_kernel(const __grid_constant__ GroupArgs g) {
   extern __shared__ __align__(128) unsigned char smem[];
   const uint32_t tm_base = tmem_begin(smem);
   const int u0 = g.first[blockIdx.x], u1 = g.first[blockIdx.x + 1];
   TmemRing ring;
   if (threadIdx.x >= TM_NC) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(TM_PREG));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(TM_GPREG));
     for (int u = u0; u < u1; ++u) {
       const int4 W = g.units[u];  // {system, item, chunk, -}
-      tmem_produce<T>(g.sys[W.x], W.y, W.z, smem, ring);
+      tmem_produce<T, false, PH>(g.sys[W.x], W.y, W.z, smem, ring);
     }
     cp_async_commit();
     cp_async_wait<0>();
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(TM_CREG));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(TM_GCREG));
     for (int u = u0; u < u1; ++u) {
       const int4 W = g.units[u];
-      tmem_consume<T, true, false, sizeof(T) == 8, false>(g.sys[W.x], W.y, W.z, smem, tm_base, ring);
+      tmem_consume<T, true, false, sizeof(T) == 8, false>(g.sys[W.x], WEQ ? g.sys[0] : g.sys[W.x], W.y, W.z, smem,
+                                                            tm_base, ring);
     }
   }
   tmem_end(tm_base);
@@ -744,9 +806,9 @@ hpsi_status tmem_regs_ok(int regs) {
   return HPSI_ERR_UNSUPPORTED;
 }
 
-template <typename T, bool HORNER, bool OBS, bool CROSS, bool RHO, bool TMA>
+template <typename T, bool HORNER, bool OBS, bool CROSS, bool RHO, bool TMA, bool PH>
 hpsi_status launch_tmem_mode(const PassArgs &a, const CUtensorMap *tm, cudaStream_t st) {
-  auto kern = pass_tmem_kernel<T, HORNER, OBS, CROSS, RHO, TMA>;
+  auto kern = pass_tmem_kernel<T, HORNER, OBS, CROSS, RHO, TMA, PH>;
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
   static int regs = 0;
@@ -761,7 +823,7 @@ hpsi_status launch_tmem_mode(const PassArgs &a, const CUtensorMap *tm, cudaStrea
   return HPSI_OK;
 }
 
-template <typename T, bool TMA>
+template <typename T, bool TMA, bool PH>
 hpsi_status launch_tmem_f(const PassArgs &a, const CUtensorMap *tm, cudaStream_t st) {
   constexpr bool REAL = sizeof(T) == 8;
   const bool horner = a.mode == PASS_HORNER, obs = a.obs != nullptr, rho = a.rho_part != nullptr;
@@ -770,19 +832,19 @@ hpsi_status launch_tmem_f(const PassArgs &a, const CUtensorMap *tm, cudaStream_t
       set_error("launch_pass_tmem: the density is fused into Horner passes without observables only");
       return HPSI_ERR_UNSUPPORTED;
     }
-    if (REAL && a.a_re == 0.0) return launch_tmem_mode<T, true, false, REAL, true, TMA>(a, tm, st);
-    return launch_tmem_mode<T, true, false, false, true, TMA>(a, tm, st);
+    if (REAL && a.a_re == 0.0) return launch_tmem_mode<T, true, false, REAL, true, TMA, PH>(a, tm, st);
+    return launch_tmem_mode<T, true, false, false, true, TMA, PH>(a, tm, st);
   }
-  if (horner && obs) return launch_tmem_mode<T, true, true, false, false, TMA>(a, tm, st);
-  if (horner && REAL && a.a_re == 0.0) return launch_tmem_mode<T, true, false, REAL, false, TMA>(a, tm, st);
-  if (horner) return launch_tmem_mode<T, true, false, false, false, TMA>(a, tm, st);
-  if (obs) return launch_tmem_mode<T, false, true, false, false, TMA>(a, tm, st);
-  return launch_tmem_mode<T, false, false, false, false, TMA>(a, tm, st);
+  if (horner && obs) return launch_tmem_mode<T, true, true, false, false, TMA, PH>(a, tm, st);
+  if (horner && REAL && a.a_re == 0.0) return launch_tmem_mode<T, true, false, REAL, false, TMA, PH>(a, tm, st);
+  if (horner) return launch_tmem_mode<T, true, false, false, false, TMA, PH>(a, tm, st);
+  if (obs) return launch_tmem_mode<T, false, true, false, false, TMA, PH>(a, tm, st);
+  return launch_tmem_mode<T, false, false, false, false, TMA, PH>(a, tm, st);
 }
 
-template <typename T>
+template <typename T, bool PH, bool WEQ>
 hpsi_status launch_tmem_group_f(const GroupArgs &g, int grid, cudaStream_t st) {
-  auto kern = pass_tmem_group_kernel<T>;
+  auto kern = pass_tmem_group_kernel<T, PH, WEQ>;
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
   static int regs = 0;
@@ -799,14 +861,20 @@ hpsi_status launch_tmem_group_f(const GroupArgs &g, int grid, cudaStream_t st) {
 template <typename T>
 hpsi_status launch_pass_tmem_group(const GroupArgs &g, int grid, cudaStream_t st) {
   if (g.nunits == 0) return HPSI_OK;
+  bool phased = false, weq = true;
   for (int s = 0; s < GROUP_MAX && g.sys[s].in != nullptr; ++s) {
     if (!blk_strides_ok<T>(g.sys[s])) return HPSI_ERR_ARG;
+    phased = phased || g.sys[s].phase_corr != nullptr;
+    weq = weq && std::memcmp(g.sys[s].wx, g.sys[0].wx, sizeof(g.sys[0].wx)) == 0 &&
+          std::memcmp(g.sys[s].wy, g.sys[0].wy, sizeof(g.sys[0].wy)) == 0 &&
+          std::memcmp(g.sys[s].wz, g.sys[0].wz, sizeof(g.sys[0].wz)) == 0;
     if (g.sys[s].a_re != 0.0 && sizeof(T) == 8) {
       set_error("launch_pass_tmem_group: purely imaginary Horner factors only");
       return HPSI_ERR_UNSUPPORTED;
     }
   }
-  return launch_tmem_group_f<T>(g, grid, st);
+  if (phased) return launch_tmem_group_f<T, true, false>(g, grid, st);
+  return weq ? launch_tmem_group_f<T, false, true>(g, grid, st) : launch_tmem_group_f<T, false, false>(g, grid, st);
 }
 template hpsi_status launch_pass_tmem_group<double>(const GroupArgs &, int, cudaStream_t);
 template hpsi_status launch_pass_tmem_group<float>(const GroupArgs &, int, cudaStream_t);
@@ -818,7 +886,8 @@ hpsi_status launch_pass_tmem(const PassArgs &a, const CUtensorMap *tm, cudaStrea
     set_error("launch_pass_tmem: TMA fill without its segment masks, or with Bloch phases");
     return HPSI_ERR_ARG;
   }
-  return tm ? launch_tmem_f<T, true>(a, tm, st) : launch_tmem_f<T, false>(a, tm, st);
+  if (a.phase_corr) return launch_tmem_f<T, false, true>(a, nullptr, st);
+  return tm ? launch_tmem_f<T, true, false>(a, tm, st) : launch_tmem_f<T, false, false>(a, tm, st);
 }
 template hpsi_status launch_pass_tmem<double>(const PassArgs &, const CUtensorMap *, cudaStream_t);
 template hpsi_status launch_pass_tmem<float>(const PassArgs &, const CUtensorMap *, cudaStream_t);
