@@ -167,8 +167,8 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *ham, int32_t nmat,
  *                   ld_points = max_npoints (the compiler copies the section
  *                   into a contiguous temporary).
  * ld_points below the largest sphere gives HPSI_ERR_ARG.  NULL removes the
- * phases; setting new projectors removes them too.  With phases the bra runs
- * on the SIMT kernel (at most 32 projectors per matrix). */
+ * phases; setting new projectors removes them too (at most 32 projectors per
+ * matrix with or without phases). */
 hpsi_status hpsi_hamiltonian_set_projector_phases(hpsi_hamiltonian *ham,
                                                   const double *phases,
                                                   int32_t ld_points);
@@ -299,7 +299,7 @@ hpsi_status hpsi_group_taylor_steps(hpsi_group *group, hpsi_batch *psis,
  * width, z block depth) on scratch batches of width ld and storage dtype and
  * keeps the fastest for this Hamiltonian's later calls with that width.
  * shape_out (optional): {state chunk, rows per thread, z block, tile height
- * (16: one-complex-per-thread pass, 8: register-blocked pass)};
+ * (16: tensor-memory or one-complex-per-thread pass, 8: register-blocked pass)};
  * ms_out: time of one pass with that shape. */
 hpsi_status hpsi_autotune(hpsi_hamiltonian *ham, int32_t dtype, int64_t ld,
                           int32_t shape_out[4], double *ms_out, void *stream);
@@ -520,7 +520,7 @@ hpsi_status hpsi_apply_h_horner_points(hpsi_hamiltonian *ham, const hpsi_batch *
 /* ------------------------------------------------------------------ */
 /* Library-wide controls and diagnostics. */
 /* Status word of the kernels of a Hamiltonian that wait on the hardware with a
- * bound (the TMA fill of the stencil pass): HPSI_OK, or HPSI_ERR_TIMEOUT when a
+ * bound (the stages of the stencil pass): HPSI_OK, or HPSI_ERR_TIMEOUT when a
  * wait gave up (its pass's results are then invalid).  Waits for the device,
  * returns the word and clears it. */
 hpsi_status hpsi_hamiltonian_status(hpsi_hamiltonian *ham, int32_t *status);

@@ -567,6 +567,8 @@ hpsi_status hpsi_hamiltonian_destroy(hpsi_hamiltonian *h) {
   h->vjpbuf.release();
   h->rhobuf.release();
   h->lzsmall.release();
+  for (auto &e : h->lz_ev)
+    if (e) cudaEventSynchronize(e);  // (a queued copy may still write to the pinned slots)
   if (h->lz_pin) cudaFreeHost(h->lz_pin);
   for (auto &e : h->lz_ev)
     if (e) cudaEventDestroy(e);
