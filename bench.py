@@ -69,7 +69,7 @@ def peaks():
         return 6650.0, "fallback"
 
 
-def profile_traffic(path="profiles/pass_blk_fp64_sphere64.md"):
+def profile_traffic(path="profiles/pass_tmem_box128x128x64.md"):
     """dram bytes per launch of the pass kernel from the committed ncu summary."""
     try:
         with open(os.path.join(ROOT, path)) as f:
@@ -749,7 +749,7 @@ def main():
                          "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
                          "traffic_kind": "ncu DRAM bytes (read + write) of one full-size launch of the same "
                                          "kernel (committed profile summary)",
-                         "kernel": "pass_blk_kernel FP64 (fused stencil + local potential)",
+                         "kernel": "pass_tmem_kernel FP64 (fused stencil + local potential)",
                          "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": pass_avg_ms,
                          "timing": "pass alone (apply without the KB term), CUDA events over the launches"},
             "kernels": {"pass_fp64": {"launches": npass, "ms": pass_ms,
