@@ -118,47 +118,60 @@ static hpsi_status group_build_tmem(hpsi_group *g, int dtype, const std::vector<
     hpsi_group::Launch L;
     L.first = first;
     L.end = std::min(n, first + GROUP_MAX);
+    using Slot = std::pair<double, int>;
+    using Slots = std::priority_queue<Slot, std::vector<Slot>, std::greater<Slot>>;
+    // depth: from the tile columns' extents alone (the lists of the chosen depth
+    // are the only ones built); no shallower one after four waves of units
     double best_t = 1e300;
     int best_blocks = 1;
-    std::vector<std::vector<int4>> plan;
     for (int blocks = 1; blocks <= 8; ++blocks) {
-      std::vector<std::pair<double, int4>> units;
+      std::vector<double> cost;
       for (int s = L.first; s < L.end; ++s) {
-        const hpsi_mesh *m = g->hams[s]->mesh;
         const int zb = depth(s, blocks), chunks = pass_chunks(shape, ld[s]);
-        const int4 *items;
-        int nitems = 0;
-        hpsi_status st = mesh_items(g->hams[s]->mesh, zb, 16, &items, &nitems);
-        if (st) return st;
-        // the list on the device, in its own order, from the same construction
-        const std::vector<int4> &hi = m->items_h.at(2 * zb);
-        for (int i = 0; i < nitems; ++i)
-          for (int c = 0; c < chunks; ++c)
-            units.push_back({double(hi[i].w - hi[i].z) + TMEM_UNIT_EXTRA, make_int4(s - L.first, i, c, 0)});
+        for (auto &t : g->hams[s]->mesh->tile_z)
+          for (int z = t.x; t.y >= 0 && z <= t.y; z += zb)
+            cost.insert(cost.end(), chunks, double(std::min(zb, t.y + 1 - z)) + TMEM_UNIT_EXTRA);
       }
-      std::stable_sort(units.begin(), units.end(), [](const auto &a, const auto &b) { return a.first > b.first; });
-      const int grid = std::max(1, std::min<int>(g->num_sms, int(units.size())));
-      std::vector<std::vector<int4>> lists(grid);
-      std::priority_queue<std::pair<double, int>, std::vector<std::pair<double, int>>, std::greater<std::pair<double, int>>> q;
-      for (int i = 0; i < grid; ++i) q.push({0.0, i});
+      std::sort(cost.begin(), cost.end(), std::greater<double>());
+      Slots q;
+      for (int i = 0; i < g->num_sms; ++i) q.push({0.0, i});
       double end = 0.0;
-      for (auto &u : units) {
-        auto [t, i] = q.top();
+      for (double u : cost) {
+        const Slot t = q.top();
         q.pop();
-        t += u.first;
-        lists[i].push_back(u.second);
-        end = std::max(end, t);
-        q.push({t, i});
+        q.push({t.first + u, t.second});
+        end = std::max(end, t.first + u);
       }
       if (end < best_t) {
         best_t = end;
         best_blocks = blocks;
-        plan.swap(lists);
       }
+      if (cost.size() >= 4 * size_t(g->num_sms)) break;
     }
+    std::vector<std::pair<double, int4>> units;
     for (int s = L.first; s < L.end; ++s) {
       g->shapes[s] = shape;
       g->shapes[s].zb = depth(s, best_blocks);
+      hpsi_mesh *m = g->hams[s]->mesh;
+      const int zb = g->shapes[s].zb, chunks = pass_chunks(shape, ld[s]);
+      const int4 *items;
+      int nitems = 0;
+      hpsi_status st = mesh_items(m, zb, 16, &items, &nitems);
+      if (st) return st;
+      const std::vector<int4> &hi = m->items_h.at(2 * zb);  // the list on the device
+      for (int i = 0; i < nitems; ++i)
+        for (int c = 0; c < chunks; ++c)
+          units.push_back({double(hi[i].w - hi[i].z) + TMEM_UNIT_EXTRA, make_int4(s - L.first, i, c, 0)});
+    }
+    std::stable_sort(units.begin(), units.end(), [](const auto &a, const auto &b) { return a.first > b.first; });
+    std::vector<std::vector<int4>> plan(std::max(1, std::min<int>(g->num_sms, int(units.size()))));
+    Slots q;
+    for (int i = 0; i < int(plan.size()); ++i) q.push({0.0, i});
+    for (auto &u : units) {
+      const Slot t = q.top();
+      q.pop();
+      plan[t.second].push_back(u.second);
+      q.push({t.first + u.first, t.second});
     }
     std::vector<int4> u;
     std::vector<int> fst(1, 0);
