@@ -91,8 +91,8 @@ bool blk_pass_eligible(const PassArgs &a, long long ld, int sc) {
 //   64-byte chunks, 16 x 8 tiles, 1 x 4 cells, 256 threads and two CTAs per
 //     SM (faster on small meshes: twice the CTAs per state chunk).
 // Tensor map of a pass input for the TMA fill: [in_rows][2 in_ld] elements of
-// the storage type, box 8 rows x one 128-byte chunk, no swizzle, zero fill
-// outside (never reached: only runs of eight existing rows are copied).
+// the storage type, box 8 rows x one 128-byte chunk, no swizzle, zero fill past
+// the batch width (a partial last chunk); the rows are runs of eight existing ones.
 // cuTensorMapEncodeTiled comes through the runtime's driver entry point.
 template <typename T>
 static hpsi_status encode_input_map(const PassArgs &a, CUtensorMap *tm) {

@@ -170,9 +170,11 @@ __device__ __forceinline__ void mbar_init_fence() {
   asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
 }
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, unsigned bytes) {
+// bytes of copies that the current phase also waits for; no arrival (the caller's
+// own arrival comes later, which holds the phase open)
+__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, unsigned bytes) {
   const unsigned a = static_cast<unsigned>(__cvta_generic_to_shared(bar));
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(a), "r"(bytes) : "memory");
+  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;\n" ::"r"(a), "r"(bytes) : "memory");
 }
 // true once the phase of the given parity has completed
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, unsigned parity) {

@@ -332,8 +332,9 @@ __device__ __forceinline__ void tmem_produce(const PassArgs &p, const int ih, co
     if constexpr (TMA) {
       const unsigned long long m = __ldg(p.seg_mask + (size_t(it.y) * p.seg_tiles_x + it.x) * B.NZ + q);
       boxes = pw < 3 && q1 > q0 ? unsigned(m >> (16 * pw)) & ((0xffffu >> (16 - 2 * (q1 - q0))) << (2 * q0)) : 0u;
-      // the bytes of the boxes, expected with this warp's plain arrival
-      if (lane == 0) mbar_arrive_expect_tx(smem_bar<false>(smem, b), unsigned(__popc(boxes)) * 8u * TM_CELLB);
+      // the bytes of the boxes; the warp's plain arrivals all come after its stores of
+      // centre weights (a release: the asynchronous arrivals order copies only)
+      if (lane == 0 && boxes) mbar_expect_tx(smem_bar<false>(smem, b), unsigned(__popc(boxes)) * 8u * TM_CELLB);
       __syncwarp();
       if (lane < 16 && ((boxes >> lane) & 1u))
         tma_load_rows(st + (size_t(128 * pw) + 8 * lane) * TM_CELLB, tm, col, mapw[2 * lane].x, smem_bar<false>(smem, b));
@@ -375,7 +376,7 @@ __device__ __forceinline__ void tmem_produce(const PassArgs &p, const int ih, co
       pent = k & 1;
     } else {
       cp_async_arrive_noinc(smem_bar<false>(smem, b));
-      if (!TMA || lane != 0) mbar_arrive(smem_bar<false>(smem, b));
+      mbar_arrive(smem_bar<false>(smem, b));
     }
     ring.next();
     if (k < TM_NBUF) advance(k);

@@ -16,7 +16,7 @@ bounded wait gave up)."""
 import numpy as np
 import pytest
 
-from helpers import small_sphere_system
+from helpers import rel_maxnorm_per_state, small_sphere_system
 
 pytestmark = pytest.mark.gpu
 
@@ -84,3 +84,43 @@ def test_fill_variant_box_mesh_default_order(cuda, variant, monkeypatch):
     H.apply(x, y1)
     assert H.status() == 0
     assert torch.equal(y0, y1)
+
+
+@pytest.mark.parametrize("dtype,nst", [("c128", 5), ("c128", 13), ("c64", 6), ("c64", 22)])
+def test_tma_fill_of_a_partial_chunk(cuda, dtype, nst, monkeypatch):
+    """Widths whose last chunk is partial (its boxes are zero-filled past the
+    width), with a potential and a laser field in the centre weights, which the
+    producers store between issuing the boxes and handing the stage over."""
+    import torch
+    from hpsi import fixtures, lib
+    from hpsi.mesh import index_box_mesh
+    from hpsi.stencil import laplacian_weights, star_points
+    from oracle import oracle as O
+    tdt, var, shape, tol = {
+        "c128": (torch.complex128, "HPSI_PASS_SHAPE64", "8,2,0,9,1,2,0,8,1,0,0,1", 1e-12),
+        "c64": (torch.complex64, "HPSI_PASS_SHAPE32", "16,2,0,9,1,2,1,8,1,0,0,1", 2e-5)}[dtype]
+    rng = np.random.default_rng(85)
+    m = index_box_mesh((34, 20, 18), 0.3)
+    v = fixtures.soft_coulomb(m, rng)
+    psi = fixtures.random_states(m, nst, rng, orthonormal=False)
+    pol, amp = np.array([0.4, -0.2, 0.9]), 0.05
+    w, pts = laplacian_weights(m.spacing), star_points()
+    H = lib.Hamiltonian(lib.DeviceMesh(m), w, pts, v=v)
+    H.set_field(pol, amp)
+    x = torch.from_numpy(psi).to(cuda).to(tdt)
+    got = []
+    for s in (None, shape):
+        if s:
+            monkeypatch.setenv(var, s)
+        else:
+            monkeypatch.delenv(var, raising=False)
+        y = torch.full((m.np, nst), float("nan"), dtype=tdt, device=cuda)
+        H.apply(x, y)
+        z = torch.full_like(y, float("nan"))
+        H.apply_horner(x, x[: m.np].clone(), z, -0.01j)
+        got.append((y, z))
+    assert H.status() == 0
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    ref = O.Hamiltonian(m, w, pts, v=v + amp * (m.x[: m.np] @ pol), bc="zero").apply(psi)
+    assert rel_maxnorm_per_state(got[1][0].cpu().numpy(), ref) <= tol
