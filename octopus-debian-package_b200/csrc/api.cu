@@ -470,12 +470,13 @@ hpsi_status hpsi_mesh_create(const hpsi_mesh_desc *d, hpsi_mesh **out) {
   up(&m->d_cell_row, cell_row);
   up(&m->d_src_raw, cell_row);
   if (s == HPSI_OK) {
-    // (the status words of the mesh's Hamiltonians follow the table, cleared)
+    // (the first status words of the mesh's Hamiltonians follow the table, cleared)
     const size_t ncol = col_z.size();
-    col_z.resize(ncol + MESH_STATUS_WORDS / 2, make_int2(0, 0));
+    col_z.resize(ncol + hpsi_status_words::BLOCK / 2, make_int2(0, 0));
     s = dev_alloc(reinterpret_cast<void **>(&m->d_col_z), col_z.size() * sizeof(int2));
     if (s == HPSI_OK) {
-      m->d_status = reinterpret_cast<int *>(m->d_col_z + ncol);
+      m->status = std::make_shared<hpsi_status_words>();
+      m->status->add(m->d_col_z, reinterpret_cast<int *>(m->d_col_z + ncol));
       cudaError_t e = cudaMemcpy(m->d_col_z, col_z.data(), col_z.size() * sizeof(int2), cudaMemcpyHostToDevice);
       if (e != cudaSuccess) {
         set_error(cudaGetErrorString(e));
@@ -505,7 +506,6 @@ hpsi_status hpsi_mesh_destroy(hpsi_mesh *m) {
   dev_free(m->d_src_per);
   dev_free(m->d_per_inner);
   dev_free(m->d_cell_of_row);
-  dev_free(m->d_col_z);
   m->scratch.release();
   m->scratch2.release();
   for (auto &kv : m->items) dev_free(kv.second.first);
@@ -531,8 +531,12 @@ hpsi_status hpsi_mesh_info(const hpsi_mesh *m, int32_t dims[6]) {
 // ---------------------------------------------------------------------------
 hpsi_status hpsi_hamiltonian_create(hpsi_mesh *mesh, hpsi_hamiltonian **out) {
   if (!mesh || !out) return HPSI_ERR_ARG;
+  int *word = nullptr;
+  if (hpsi_status s = mesh->status->take(&word)) return s;
   hpsi_hamiltonian *h = new hpsi_hamiltonian();
   h->mesh = mesh;
+  h->status = mesh->status;
+  h->d_err = word;
   // experiment override: HPSI_BRA_OVERLAP=0 runs the KB bra on the caller's
   // stream before the pass
   if (const char *e = std::getenv("HPSI_BRA_OVERLAP")) h->overlap_bra = std::atoi(e) != 0;
@@ -540,9 +544,6 @@ hpsi_status hpsi_hamiltonian_create(hpsi_mesh *mesh, hpsi_hamiltonian **out) {
   // experiment override: HPSI_FUSED_DENSITY=1 fuses the density of
   // hpsi_taylor_step_density into the last pass
   if (const char *e = std::getenv("HPSI_FUSED_DENSITY")) h->fuse_density = std::atoi(e) != 0;
-  // status word of the passes' bounded waits: one of the mesh's (256 of them, taken
-  // in turn; no allocation of its own)
-  h->d_err = mesh->d_status + mesh->next_status.fetch_add(1u) % MESH_STATUS_WORDS;
   *out = h;
   return HPSI_OK;
 }
@@ -586,8 +587,47 @@ hpsi_status hpsi_hamiltonian_destroy(hpsi_hamiltonian *h) {
   h->slab_in.release();
   h->slab_out.release();
   h->small.release();
+  h->status->give(h->d_err);
   delete h;
   return HPSI_OK;
+}
+
+void hpsi_status_words::add(void *alloc, int *words) {
+  blocks.push_back(alloc);
+  for (int i = BLOCK - 1; i >= 0; --i) fresh.push_back(words + i);
+}
+
+hpsi_status hpsi_status_words::take(int **word) {
+  std::lock_guard<std::mutex> lk(mu);
+  if (fresh.empty() && !used.empty()) {
+    HPSI_TRY_CUDA(cudaMemset(used.back(), 0, sizeof(int)));
+    *word = used.back();
+    used.pop_back();
+    return HPSI_OK;
+  }
+  if (fresh.empty()) {
+    void *p = nullptr;
+    hpsi_status s = dev_alloc(&p, BLOCK * sizeof(int));
+    if (s) return s;
+    const cudaError_t e = cudaMemset(p, 0, BLOCK * sizeof(int));
+    if (e != cudaSuccess) {
+      dev_free(p);
+      HPSI_TRY_CUDA(e);
+    }
+    add(p, static_cast<int *>(p));
+  }
+  *word = fresh.back();
+  fresh.pop_back();
+  return HPSI_OK;
+}
+
+void hpsi_status_words::give(int *word) {
+  std::lock_guard<std::mutex> lk(mu);
+  used.push_back(word);
+}
+
+hpsi_status_words::~hpsi_status_words() {
+  for (void *p : blocks) dev_free(p);
 }
 
 hpsi_status hpsi_hamiltonian::lanczos_pinned(size_t bytes) {
@@ -2321,10 +2361,17 @@ hpsi_status hpsi_apply_h_horner_points(hpsi_hamiltonian *h, const hpsi_batch *ps
                          ld, a_re, a_im, nullptr, nullptr, st, nullptr, points);
 }
 
+// For the tests (not in hpsi.h): records what a kernel records whose wait gave up.
+hpsi_status hpsi_test_record_timeout(hpsi_hamiltonian *h) {
+  if (!h) return HPSI_ERR_ARG;
+  const int v = HPSI_ERR_TIMEOUT;
+  HPSI_TRY_CUDA(cudaMemcpy(h->d_err, &v, sizeof(int), cudaMemcpyHostToDevice));
+  return HPSI_OK;
+}
+
 hpsi_status hpsi_hamiltonian_status(hpsi_hamiltonian *h, int32_t *status) {
   if (!h || !status) return HPSI_ERR_ARG;
   *status = HPSI_OK;
-  if (!h->d_err) return HPSI_OK;
   int v = 0;
   HPSI_TRY_CUDA(cudaMemcpy(&v, h->d_err, sizeof(int), cudaMemcpyDeviceToHost));
   HPSI_TRY_CUDA(cudaMemset(h->d_err, 0, sizeof(int)));

@@ -1,8 +1,9 @@
 // Handle layouts behind the opaque C types of hpsi.h.
 #pragma once
 
-#include <atomic>
 #include <map>
+#include <memory>
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -40,7 +41,21 @@ struct Workspace {
 
 }  // namespace hpsi
 
-constexpr int MESH_STATUS_WORDS = 256;
+// Status words of the bounded waits, one for each Hamiltonian of a mesh, in blocks of
+// 256 (the first block follows the mesh's column table).  Held by the mesh and by its
+// Hamiltonians: the memory goes with the last of them, so that a Hamiltonian's
+// word outlives a mesh destroyed before it.
+struct hpsi_status_words {
+  static constexpr int BLOCK = 256;
+  std::mutex mu;
+  std::vector<void *> blocks;  // device allocations
+  std::vector<int *> fresh;    // cleared words nobody has had
+  std::vector<int *> used;     // returned words: cleared when they are handed out again
+  void add(void *alloc, int *words);
+  hpsi_status take(int **word);
+  void give(int *word);
+  ~hpsi_status_words();
+};
 
 struct hpsi_mesh {
   int np = 0, np_part = 0, order = 4, periodic = 0;
@@ -76,9 +91,7 @@ struct hpsi_mesh {
   std::vector<int> cell_row_h;
   std::map<const int *, unsigned long long *> seg_masks;
   int2 *d_col_z = nullptr;  // per (y, x) cell column: z range of its inner points
-  // status words of the Hamiltonians' bounded waits (after d_col_z's table)
-  int *d_status = nullptr;
-  std::atomic<unsigned> next_status{0};
+  std::shared_ptr<hpsi_status_words> status;  // owns d_col_z's allocation
 };
 
 struct hpsi_hamiltonian {
@@ -152,6 +165,7 @@ struct hpsi_hamiltonian {
   hpsi::Workspace vstage;  // host potential staged for hpsi_hamiltonian_update_vloc
   hpsi::Workspace adjstep, vjpbuf;  // per-step adjoint scratch, field VJP partials
   hpsi::Workspace rhobuf;  // fused density: weights, pass and ket partials
-  int *d_err = nullptr;     // status word of the passes' bounded waits  // Lanczos: Krylov vectors, reductions and coefficients
+  int *d_err = nullptr;     // status word of the passes' bounded waits, one of `status`
+  std::shared_ptr<hpsi_status_words> status;
   void proj_free();
 };
