@@ -522,7 +522,11 @@ hpsi_status hpsi_apply_h_horner_points(hpsi_hamiltonian *ham, const hpsi_batch *
 /* Status word of the kernels of a Hamiltonian that wait on the hardware with a
  * bound (the stages of the stencil pass): HPSI_OK, or HPSI_ERR_TIMEOUT when a
  * wait gave up (its pass's results are then invalid).  Waits for the device,
- * returns the word and clears it. */
+ * returns the word and clears it.  Calls that wait for the device themselves
+ * (host batches, observables, hpsi_td_propagate*, hpsi_lanczos_step,
+ * hpsi_adjoint_gradient, hpsi_adjoint_step with host results, hpsi_autotune)
+ * return HPSI_ERR_TIMEOUT while it is set; the others are queued, and
+ * a program reads the word where it waits for their results. */
 hpsi_status hpsi_hamiltonian_status(hpsi_hamiltonian *ham, int32_t *status);
 const char *hpsi_last_error_string(void);
 /* Number of this library's kernels launched since load (diagnostic). */

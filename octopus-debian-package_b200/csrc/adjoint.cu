@@ -508,9 +508,12 @@ extern "C" hpsi_status hpsi_adjoint_gradient(hpsi_hamiltonian *h, const hpsi_bat
   if (grad_eps_cont)
     HPSI_TRY_CUDA(cudaMemcpyAsync(grad_eps_cont, gcont, nsteps * sizeof(double), cudaMemcpyDeviceToHost, st));
   if (grad_v) HPSI_TRY_CUDA(cudaMemcpyAsync(grad_v, gv, size_t(m->np) * sizeof(double), cudaMemcpyDeviceToHost, st));
+  int word = 0;
+  s = h->send_status(&word, st);
+  if (s) return fail(s);
   HPSI_TRY_CUDA(cudaStreamSynchronize(st));
   for (int a = 0; a < 3; ++a) h->fld[a] = save_fld[a];
-  return HPSI_OK;
+  return h->waits_ok(word, "hpsi_adjoint_gradient");
 }
 
 // ---------------------------------------------------------------------------
@@ -572,7 +575,13 @@ extern "C" hpsi_status hpsi_adjoint_step(hpsi_hamiltonian *h, hpsi_batch *lambda
       HPSI_TRY_CUDA(cudaMemcpyAsync(o, o == grad_eps ? g2 : g2 + 1, sizeof(double), cudaMemcpyDefault, st));
       host_out = host_out || !is_device_ptr(o);
     }
-  if (host_out) HPSI_TRY_CUDA(cudaStreamSynchronize(st));
+  if (host_out) {
+    int word = 0;
+    s = h->send_status(&word, st);
+    if (s) return s;
+    HPSI_TRY_CUDA(cudaStreamSynchronize(st));
+    return h->waits_ok(word, "hpsi_adjoint_step");
+  }
   return HPSI_OK;
 }
 

@@ -646,6 +646,17 @@ hpsi_status hpsi_hamiltonian::lanczos_pinned(size_t bytes) {
   return HPSI_OK;
 }
 
+hpsi_status hpsi_hamiltonian::send_status(int *word, cudaStream_t st) const {
+  HPSI_TRY_CUDA(cudaMemcpyAsync(word, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+  return HPSI_OK;
+}
+
+hpsi_status hpsi_hamiltonian::waits_ok(int word, const char *who) {
+  if (word == HPSI_OK) return HPSI_OK;
+  set_error(std::string(who) + ": a bounded device wait gave up, the results are invalid");
+  return word;
+}
+
 hpsi_status hpsi_hamiltonian::ensure_bra_stream() {
   if (bra_stream) return HPSI_OK;
   HPSI_TRY_CUDA(cudaStreamCreateWithFlags(&bra_stream, cudaStreamNonBlocking));
@@ -1642,7 +1653,7 @@ hpsi_status prepare_taylor_workspaces(hpsi_hamiltonian *h, long long ld, size_t 
   if (obs) {
     hpsi_status s = h->obsbuf.ensure(obs_partial_bytes(h, ld));
     if (s) return s;
-    s = h->small.ensure(3 * size_t(ld) * sizeof(double));
+    s = h->small.ensure((3 * size_t(ld) + 1) * sizeof(double));
     if (s) return s;
   }
   if (h->nmat > 0) {
@@ -1713,7 +1724,7 @@ hpsi_status taylor_dev_impl(hpsi_hamiltonian *h, T *psi, long long ld, int nst, 
     const bool nl = h->nmat > 0 && h->nk > 0;
     hpsi_status s = launch_obs_finalize(obs_partial, ncta, int(ld), nst, m->box.h[0] * m->box.h[1] * m->box.h[2],
                                         nl ? static_cast<const double *>(h->ketobs.ptr) : nullptr,
-                                        nl ? ket_row_blocks(h->nk) : 0, obs_dev, st);
+                                        nl ? ket_row_blocks(h->nk) : 0, h->d_err, obs_dev, st);
     if (s) return s;
   }
   return HPSI_OK;
@@ -1796,8 +1807,11 @@ hpsi_status apply_h_host_pipelined(hpsi_hamiltonian *h, const hpsi_batch *psi, h
     HPSI_TRY_CUDA(cudaEventRecord(out_done[b], h->xfer_out));
   }
   HPSI_TRY_CUDA(cudaStreamSynchronize(h->xfer_out));
+  int word = 0;
+  s = h->send_status(&word, st);
+  if (s) return s;
   HPSI_TRY_CUDA(cudaStreamSynchronize(st));
-  return HPSI_OK;
+  return h->waits_ok(word, "hpsi_apply_h");
 }
 
 // State slabs of the host pipeline (widths in states, each a multiple of the
@@ -1892,7 +1906,13 @@ hpsi_status hpsi_apply_h(hpsi_hamiltonian *h, const hpsi_batch *psi, hpsi_batch 
     const size_t esz = hpsi->dtype == HPSI_C128 ? 16 : 8;
     HPSI_TRY_CUDA(cudaMemcpyAsync(hpsi->ptr, pout, size_t(m->np) * ldo * esz, cudaMemcpyDeviceToHost, st));
   }
-  if (!din || !dout) HPSI_TRY_CUDA(cudaStreamSynchronize(st));
+  if (!din || !dout) {
+    int word = 0;
+    s = h->send_status(&word, st);
+    if (s) return s;
+    HPSI_TRY_CUDA(cudaStreamSynchronize(st));
+    return h->waits_ok(word, "hpsi_apply_h");
+  }
   return HPSI_OK;
 }
 
@@ -1938,7 +1958,7 @@ hpsi_status hpsi_taylor_step(hpsi_hamiltonian *h, hpsi_batch *psi, double dt_re,
   const bool want_obs = energy || dipole || norm2;
   double *obs_dev = nullptr;
   if (want_obs) {
-    s = h->small.ensure(3 * size_t(psi->nst) * sizeof(double));
+    s = h->small.ensure((3 * size_t(psi->nst) + 1) * sizeof(double));
     if (s) return s;
     obs_dev = static_cast<double *>(h->small.ptr);
   }
@@ -1958,9 +1978,11 @@ hpsi_status hpsi_taylor_step(hpsi_hamiltonian *h, hpsi_batch *psi, double dt_re,
     HPSI_TRY_CUDA(cudaMemcpyAsync(psi->ptr, p, size_t(m->np) * psi->ld * esz, cudaMemcpyDeviceToHost, st));
   }
   if (want_obs) {
-    std::vector<double> hv(3 * size_t(psi->nst));
+    std::vector<double> hv(3 * size_t(psi->nst) + 1);  // (the last one: the status word)
     HPSI_TRY_CUDA(cudaMemcpyAsync(hv.data(), obs_dev, hv.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     HPSI_TRY_CUDA(cudaStreamSynchronize(st));
+    s = h->waits_ok(int(hv.back()), "hpsi_taylor_step");
+    if (s) return s;
     bool finite = true;
     for (double x : hv) finite = finite && std::isfinite(x);
     const int n = psi->nst;
@@ -1972,7 +1994,11 @@ hpsi_status hpsi_taylor_step(hpsi_hamiltonian *h, hpsi_batch *psi, double dt_re,
       return HPSI_ERR_NONFINITE;
     }
   } else if (!dev) {
+    int word = 0;
+    s = h->send_status(&word, st);
+    if (s) return s;
     HPSI_TRY_CUDA(cudaStreamSynchronize(st));
+    return h->waits_ok(word, "hpsi_taylor_step");
   }
   return HPSI_OK;
 }

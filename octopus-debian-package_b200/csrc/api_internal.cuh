@@ -166,6 +166,11 @@ struct hpsi_hamiltonian {
   hpsi::Workspace adjstep, vjpbuf;  // per-step adjoint scratch, field VJP partials
   hpsi::Workspace rhobuf;  // fused density: weights, pass and ket partials
   int *d_err = nullptr;     // status word of the passes' bounded waits, one of `status`
+  // For calls that wait for the device anyway: the word into *word after the work of
+  // `st`, and, once it has arrived, HPSI_ERR_TIMEOUT if it is set (it stays set
+  // until hpsi_hamiltonian_status).
+  hpsi_status send_status(int *word, cudaStream_t st) const;
+  static hpsi_status waits_ok(int word, const char *who);
   std::shared_ptr<hpsi_status_words> status;
   void proj_free();
 };

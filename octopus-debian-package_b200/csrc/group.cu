@@ -540,9 +540,12 @@ static hpsi_status autotune_t(hpsi_hamiltonian *h, int dtype, long long ld, cuda
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  int word = 0;
+  if (!r) r = h->send_status(&word, st);
   cudaStreamSynchronize(st);
   dev_free(in);
   dev_free(out);
+  if (!r) r = h->waits_ok(word, "hpsi_autotune");
   if (r) return r;
   auto &t = h->tuned[dtype == HPSI_C128 ? 0 : 1];
   t.ld = ld;

@@ -318,7 +318,7 @@ extern "C" hpsi_status hpsi_lanczos_step(hpsi_hamiltonian *h, hpsi_batch *psi, d
   // and the next one, already queued)
   std::vector<double> hn(size_t(K + 1) * nst), hs(size_t(K + 1) * nst), hraw(4 * size_t(nst));
   const size_t pslot = 5 * size_t(nst);
-  s = h->lanczos_pinned(2 * pslot * sizeof(double));
+  s = h->lanczos_pinned((2 * pslot + 1) * sizeof(double));  // (and the status word)
   if (s) return s;
   auto slot = [&](int j) { return static_cast<double *>(h->lz_pin) + (j & 1) * pslot; };
   auto send = [&](int j, bool with_raw) -> hpsi_status {
@@ -463,7 +463,12 @@ extern "C" hpsi_status hpsi_lanczos_step(hpsi_hamiltonian *h, hpsi_batch *psi, d
   HPSI_TRY_CUDA(cudaMemcpyAsync(coef, cc.data(), cc.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
   lz_combine<<<grid_for(nel), 256, 0, st>>>(psi_d, U, vstride, mdim, ld, nel, nst, coef);
   HPSI_CHECK_LAUNCH();
+  int *word = reinterpret_cast<int *>(static_cast<double *>(h->lz_pin) + 2 * pslot);
+  s = h->send_status(word, st);
+  if (s) return s;
   HPSI_TRY_CUDA(cudaStreamSynchronize(st));
+  s = h->waits_ok(*word, "hpsi_lanczos_step");
+  if (s) return s;
   if (iters_out) *iters_out = mdim;
   if (res_out) *res_out = worst;  // > tol: not converged (the reference only warns)
   return HPSI_OK;

@@ -474,13 +474,15 @@ __global__ void __launch_bounds__(256) trsm_apply_kernel(T *psi, long long ld, i
   }
 }
 
-// observables: partial [ncta][ld][3][2] -> out[3][nst] (energy, norm2, dipole) * dv.
+// observables: partial [ncta][ld][3][2] -> out[3][nst] (energy, norm2, dipole) * dv,
+// then the status word of the passes, so that one copy brings both to the host.
 // One CTA per state: its threads take strided slices of the CTA partials
 // (compensated sums), then fold them in shared memory.
 __global__ void __launch_bounds__(128) obs_finalize_kernel(const double *partial, int ncta, int ld, int nst,
                                                            double dv, const double *ket_partial, int nket,
-                                                           double *out) {
+                                                           const int *status, double *out) {
   const int s = blockIdx.x;
+  if (s == 0 && threadIdx.x == 0) out[3 * nst] = double(*status);
   __shared__ double red[3][2][128];
   Kahan a[3] = {{0, 0}, {0, 0}, {0, 0}};
   for (int c = threadIdx.x; c < ncta; c += blockDim.x) {
@@ -636,9 +638,10 @@ hpsi_status launch_trsm_apply(T *psi, long long ld, int np, int nst, const doubl
 }
 
 hpsi_status launch_obs_finalize(const double *partial, int ncta, int ld, int nst, double dv,
-                                const double *ket_partial, int nket, double *out, cudaStream_t st) {
+                                const double *ket_partial, int nket, const int *status, double *out,
+                                cudaStream_t st) {
   if (nst < 1) return HPSI_OK;
-  obs_finalize_kernel<<<nst, 128, 0, st>>>(partial, ncta, ld, nst, dv, ket_partial, nket, out);
+  obs_finalize_kernel<<<nst, 128, 0, st>>>(partial, ncta, ld, nst, dv, ket_partial, nket, status, out);
   HPSI_CHECK_LAUNCH();
   return HPSI_OK;
 }

@@ -26,14 +26,16 @@ hpsi_status launch_cholesky_inverse(const double *S, int nst, double *U, double 
 template <typename T>
 hpsi_status launch_trsm_apply(T *psi, long long ld, int np, int nst, const double *Uinv, cudaStream_t st);
 
-// partial [ncta][ld][3][2] -> out[3][nst] = (energy, norm2, dipole) * dv;
-// ket_partial [nket][ld][2] (may be null) adds the KB part of the energy
 // rho[ip] (+)= sum_s w[s] |psi_s(ip)|^2 (w on the device, nst entries)
 template <typename T>
 hpsi_status launch_density(const T *psi, long long ld, int np, int nst, const double *w, double *rho, int accumulate,
                            cudaStream_t st);
 
+// partial [ncta][ld][3][2] -> out[3][nst] = (energy, norm2, dipole) * dv;
+// ket_partial [nket][ld][2] (may be null) adds the KB part of the energy;
+// out[3 nst] = *status
 hpsi_status launch_obs_finalize(const double *partial, int ncta, int ld, int nst, double dv,
-                                const double *ket_partial, int nket, double *out, cudaStream_t st);
+                                const double *ket_partial, int nket, const int *status, double *out,
+                                cudaStream_t st);
 
 }  // namespace hpsi

@@ -32,9 +32,11 @@ namespace {
 
 // Sums the per-state observables of the current step over the states and
 // advances the device step counter and the field amplitude of the next step.
-// tables: amp_mid[nsteps+1], amp_n[nsteps+1]; state: {cur_amp, step}.
+// tables: amp_mid[nsteps+1], amp_n[nsteps+1]; state: {cur_amp, step, status word
+// of the passes so far}.
 __global__ void td_step_finalize(const double *obs_state, int nst, const double *amp_mid, const double *amp_n,
-                                 double *cur_amp, int *step, double *energy, double *dipole, double *norm2) {
+                                 double *cur_amp, int *step, double *energy, double *dipole, double *norm2,
+                                 const int *status) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   const int s = *step;
   Kahan e = {0, 0}, n = {0, 0}, d = {0, 0};
@@ -48,6 +50,7 @@ __global__ void td_step_finalize(const double *obs_state, int nst, const double 
   dipole[s] = D;
   norm2[s] = n.s + n.c;
   *step = s + 1;
+  step[1] = *status;
   *cur_amp = amp_mid[s + 1];
 }
 
@@ -71,18 +74,18 @@ hpsi_status td_run(hpsi_hamiltonian *h, T *psi, long long ld, int nst, int nstep
                    const hpsi_laser *las, double t0, bool graph, double *e_out, double *d_out, double *n_out,
                    cudaStream_t st, int propagator = 0) {
   // device layout of the driver buffer (doubles):
-  // amp_mid[nsteps+1] amp_n[nsteps+1] cur_amp step(int) E[nsteps] D[nsteps] N[nsteps] obs_state[3*nst]
-  // amp_b[nsteps+1]
+  // amp_mid[nsteps+1] amp_n[nsteps+1] cur_amp {step, status word}(ints) E[nsteps] D[nsteps] N[nsteps]
+  // obs_state[3*nst+1] amp_b[nsteps+1]
   // (ETRS: amp_mid = amp_n = E(t_n), the first half step; amp_b = E(t_n+1))
   const bool etrs = propagator == 1;
-  const size_t nd = 2 * size_t(nsteps + 1) + 2 + 3 * size_t(nsteps) + 3 * size_t(nst) + size_t(nsteps + 1);
+  const size_t nd = 2 * size_t(nsteps + 1) + 2 + 3 * size_t(nsteps) + 3 * size_t(nst) + 1 + size_t(nsteps + 1);
   hpsi_status s = h->tdbuf.ensure(nd * sizeof(double));
   if (s) return s;
   double *base = static_cast<double *>(h->tdbuf.ptr);
   double *amp_mid = base, *amp_n = base + (nsteps + 1), *cur_amp = amp_n + (nsteps + 1);
   int *step = reinterpret_cast<int *>(cur_amp + 1);
   double *E = cur_amp + 2, *D = E + nsteps, *N = D + nsteps, *obs_state = N + nsteps;
-  double *amp_b = obs_state + 3 * size_t(nst);
+  double *amp_b = obs_state + 3 * size_t(nst) + 1;
   std::vector<double> host(2 * size_t(nsteps + 1) + 2, 0.0), hostb(size_t(nsteps + 1), 0.0);
   const hpsi_laser none = {0.0, 0.0, 0.0, {0.0, 0.0, 1.0}};
   const hpsi_laser &L = las ? *las : none;
@@ -92,8 +95,8 @@ hpsi_status td_run(hpsi_hamiltonian *h, T *psi, long long ld, int nst, int nstep
     hostb[i] = laser_field(L, t0 + (i + 1) * dt);
   }
   host[2 * size_t(nsteps + 1)] = host[0];  // cur_amp
-  int zero = 0;
-  std::memcpy(&host[2 * size_t(nsteps + 1) + 1], &zero, sizeof(int));
+  const int zero[2] = {0, 0};
+  std::memcpy(&host[2 * size_t(nsteps + 1) + 1], zero, sizeof(zero));
   HPSI_TRY_CUDA(cudaMemcpyAsync(base, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice, st));
   if (etrs)
     HPSI_TRY_CUDA(cudaMemcpyAsync(amp_b, hostb.data(), hostb.size() * sizeof(double), cudaMemcpyHostToDevice, st));
@@ -118,7 +121,7 @@ hpsi_status td_run(hpsi_hamiltonian *h, T *psi, long long ld, int nst, int nstep
       r = taylor_dev<T>(h, psi, ld, nst, 0.5 * dt, 0.0, order, nullptr, st);
       if (r) return r;
     }
-    td_step_finalize<<<1, 32, 0, st>>>(obs_state, nst, amp_mid, amp_n, cur_amp, step, E, D, N);
+    td_step_finalize<<<1, 32, 0, st>>>(obs_state, nst, amp_mid, amp_n, cur_amp, step, E, D, N, h->d_err);
     HPSI_CHECK_LAUNCH();
     return HPSI_OK;
   };
@@ -182,10 +185,15 @@ hpsi_status td_run(hpsi_hamiltonian *h, T *psi, long long ld, int nst, int nstep
   }
   h->have_pol = save_have;
   if (r) return r;
-  std::vector<double> out(3 * size_t(nsteps));
+  std::vector<double> out(3 * size_t(nsteps) + 1);  // {step, status word}, then the tables
   if (nsteps > 0)
-    HPSI_TRY_CUDA(cudaMemcpyAsync(out.data(), E, out.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+    HPSI_TRY_CUDA(cudaMemcpyAsync(out.data(), step, out.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
   HPSI_TRY_CUDA(cudaStreamSynchronize(st));
+  int words[2] = {0, 0};
+  std::memcpy(words, out.data(), sizeof(words));
+  r = hpsi_hamiltonian::waits_ok(words[1], etrs ? "hpsi_td_propagate_etrs" : "hpsi_td_propagate");
+  if (r) return r;
+  out.erase(out.begin());
   bool finite = true;
   for (double x : out) finite = finite && std::isfinite(x);
   if (e_out) std::memcpy(e_out, out.data(), nsteps * sizeof(double));

@@ -59,3 +59,41 @@ def test_a_word_outlives_its_mesh(cuda):
     assert H.status() == 0
     _record_timeout(H)
     assert other.status() == 0 and H.status() == TIMEOUT
+
+
+def test_calls_that_wait_for_the_device_report_a_timeout(cuda):
+    """Every call that brings results to the host answers with the timeout as long as
+    the word is set, and works again once it has been read."""
+    import torch
+    from hpsi import lib
+    m, dm = _mesh()
+    H = _ham(m, dm)
+    rng = np.random.default_rng(3)
+    host = np.zeros((m.np_part, 4), dtype=np.complex128)
+    host[: m.np] = rng.standard_normal((m.np, 4)) + 1j * rng.standard_normal((m.np, 4))
+    wide = np.zeros((m.np_part, 16), dtype=np.complex128)  # (two slabs of the host pipeline)
+    x = torch.from_numpy(host).to(cuda)
+    dm.orthonormalize_cholesky(x)
+    eps = np.linspace(0.0, 0.01, 3)
+    calls = {
+        "host batch": lambda: H.apply(host, np.zeros((m.np, 4), dtype=np.complex128)),
+        "host batch in slabs": lambda: H.apply(wide, np.zeros((m.np, 16), dtype=np.complex128)),
+        "host step": lambda: H.taylor_step(host.copy(), 1e-3),
+        "observables": lambda: H.taylor_step(x.clone(), 1e-3, observables=True),
+        "propagation": lambda: H.td_propagate(x.clone(), 2, 1e-3),
+        "propagation, no graph": lambda: H.td_propagate(x.clone(), 2, 1e-3, graph=False),
+        "etrs": lambda: H.td_propagate(x.clone(), 2, 1e-3, propagator="etrs"),
+        "lanczos": lambda: H.lanczos_step(x.clone(), 1e-3),
+        "adjoint": lambda: H.adjoint_gradient(x, x.clone(), eps, 1e-3),
+        "adjoint step": lambda: H.adjoint_step(x.clone(), x, 0.01, 1e-3),
+        "autotune": lambda: H.autotune(ld=4),
+    }
+    for name, call in calls.items():
+        call()
+        _record_timeout(H)
+        with pytest.raises(lib.HpsiError) as e:
+            call()
+        assert e.value.status == TIMEOUT, name
+        assert H.status() == TIMEOUT, name
+        call()
+    assert H.status() == 0
