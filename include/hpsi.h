@@ -390,7 +390,8 @@ hpsi_status hpsi_vjp_vloc(hpsi_hamiltonian *ham, const hpsi_batch *lambda,
  *                    column j fastest) X(mesh_batch_dotp_matrix), :20-263
  *   hpsi_orthonormalize_cholesky   S = U^H U, psi <- psi U^-1 in place,
  *                    X(states_elec_orthogonalization_full) cholesky_serial,
- *                    src/states/states_elec_calc_inc.F90:66-98 */
+ *                    src/states/states_elec_calc_inc.F90:66-98; at most 3072
+ *                    states */
 hpsi_status hpsi_nrm2(hpsi_mesh *mesh, const hpsi_batch *psi, double *out,
                       void *stream);
 hpsi_status hpsi_dotp_matrix(hpsi_mesh *mesh, const hpsi_batch *a,

@@ -2172,6 +2172,10 @@ hpsi_status hpsi_orthonormalize_cholesky(hpsi_mesh *m, hpsi_batch *psi, void *st
     set_error("hpsi_orthonormalize_cholesky: device batch expected");
     return HPSI_ERR_ARG;
   }
+  if (psi->nst > ORTHO_MAX_STATES) {
+    set_error("hpsi_orthonormalize_cholesky: at most " + std::to_string(ORTHO_MAX_STATES) + " states");
+    return HPSI_ERR_UNSUPPORTED;
+  }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int nst = psi->nst, splits = gram_splits(m->np, nst, true);
   const size_t pbytes = size_t(splits) * 4 * nst * nst * sizeof(double);

@@ -622,10 +622,6 @@ hpsi_status launch_cholesky_inverse(const double *S, int nst, double *U, double 
 template <typename T>
 hpsi_status launch_trsm_apply(T *psi, long long ld, int np, int nst, const double *Uinv, cudaStream_t st) {
   constexpr size_t smem = size_t(2) * GK * (GT + 4) * sizeof(double) + size_t(GST) * GT * (GK + 4) * sizeof(T);
-  if (nst > 1536) {
-    set_error("orthonormalisation supports at most 1536 states");
-    return HPSI_ERR_UNSUPPORTED;
-  }
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
   std::call_once(once, [&] {

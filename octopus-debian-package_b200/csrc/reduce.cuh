@@ -5,6 +5,9 @@
 
 namespace hpsi {
 
+// Most states of an orthonormalisation.
+constexpr int ORTHO_MAX_STATES = 3072;
+
 int reduce_blocks(int np);
 int gram_splits(int np, int nst, bool sym);
 

@@ -56,3 +56,29 @@ def test_indefinite_overlap_is_refused(cuda):
     with pytest.raises(lib.HpsiError):
         dm.orthonormalize_cholesky(x, nst=2)  # a zero state
     assert torch.equal(x, keep)
+
+
+def test_orthonormalisation_of_many_states(cuda):
+    """1537 states: the triangular update has no limit of its own."""
+    import torch
+    from hpsi import lib
+    from hpsi.mesh import index_box_mesh
+    m = index_box_mesh((17, 17, 17), 0.4)
+    dm = lib.DeviceMesh(m)
+    nst = 1537
+    g = torch.Generator(device=cuda).manual_seed(7)
+    x = torch.randn((m.np, nst), dtype=torch.complex128, device=cuda, generator=g)
+    dm.orthonormalize_cholesky(x)
+    S = dm.dotp_matrix(x, x)
+    # condition of the overlap about (1.56 / 0.44)^2 = 13 (np / nst = 3.2): the
+    # overlap of the result is the unit matrix to condition * nst * eps at most
+    assert np.max(np.abs(S - np.eye(nst))) <= 13 * nst * np.finfo(float).eps
+
+
+def test_too_many_states_are_refused(cuda):
+    import torch
+    from hpsi import lib
+    m = _mesh()
+    x = torch.zeros((m.np, 3074), dtype=torch.complex64, device=cuda)
+    with pytest.raises(lib.HpsiError, match="3072"):
+        lib.DeviceMesh(m).orthonormalize_cholesky(x, nst=3073)
