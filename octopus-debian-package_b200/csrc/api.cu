@@ -2145,12 +2145,12 @@ hpsi_status hpsi_dotp_matrix(hpsi_mesh *m, const hpsi_batch *a, const hpsi_batch
     return HPSI_ERR_ARG;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int nst = a->nst, splits = gram_splits(m->np, nst, a->ptr == b->ptr && a->ld == b->ld);
-  const size_t pbytes = size_t(splits) * 4 * nst * nst * sizeof(double);
+  const int nst = a->nst, splits = gram_splits(m->np, nst, a->ptr == b->ptr && a->ld == b->ld, m->num_sms);
+  const size_t pn = gram_partial_doubles(m->np, nst, splits), pbytes = pn * sizeof(double);
   s = m->scratch.ensure(pbytes + 2 * size_t(nst) * nst * sizeof(double));
   if (s) return s;
   double *partial = static_cast<double *>(m->scratch.ptr);
-  double *S = partial + size_t(splits) * 4 * nst * nst;
+  double *S = partial + pn;
   const double dv = m->box.h[0] * m->box.h[1] * m->box.h[2];
   if (a->dtype == HPSI_C128)
     s = launch_gram<double>(static_cast<const double *>(a->ptr), a->ld, static_cast<const double *>(b->ptr), b->ld,
@@ -2177,13 +2177,13 @@ hpsi_status hpsi_orthonormalize_cholesky(hpsi_mesh *m, hpsi_batch *psi, void *st
     return HPSI_ERR_UNSUPPORTED;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int nst = psi->nst, splits = gram_splits(m->np, nst, true);
-  const size_t pbytes = size_t(splits) * 4 * nst * nst * sizeof(double);
+  const int nst = psi->nst, splits = gram_splits(m->np, nst, true, m->num_sms);
+  const size_t pn = gram_partial_doubles(m->np, nst, splits), pbytes = pn * sizeof(double);
   const size_t mbytes = 2 * size_t(nst) * nst * sizeof(double);
   s = m->scratch.ensure(pbytes + 3 * mbytes + 16);
   if (s) return s;
   double *partial = static_cast<double *>(m->scratch.ptr);
-  double *S = partial + size_t(splits) * 4 * nst * nst;
+  double *S = partial + pn;
   double *U = S + 2 * size_t(nst) * nst;
   double *Uinv = U + 2 * size_t(nst) * nst;
   int *err = reinterpret_cast<int *>(Uinv + 2 * size_t(nst) * nst);

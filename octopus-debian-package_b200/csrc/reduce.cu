@@ -107,6 +107,7 @@ __global__ void state_sum_finalize(const double *partial, int nblk, int nst, dou
 constexpr int GT = 64;   // tile edge (real lanes, rows)
 constexpr int GK = 16;   // K step staged at once
 constexpr int GST = 4;   // staged steps
+constexpr int GFOLD = 8192 / GK;  // K steps summed before they are folded with compensation
 
 __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -130,15 +131,30 @@ constexpr int gram_pitch() {
   return sizeof(T) == 8 ? GT + 4 : GT + 8;
 }
 
+// Two sums into the partials at `at`, their remainders (Kahan) into oc.
+__device__ __forceinline__ void gram_fold(double *o, double *oc, long long at, bool first, const double (&c)[2]) {
+  double2 &s = *reinterpret_cast<double2 *>(o + at), &r = *reinterpret_cast<double2 *>(oc + at);
+  Kahan x = {0, 0}, y = {0, 0};
+  if (!first) x = {s.x, r.x}, y = {s.y, r.y};
+  kadd(x, c[0]);
+  kadd(y, c[1]);
+  s = make_double2(x.s, y.s);
+  r = make_double2(x.c, y.c);
+}
+
 // Gram matrix of the real views: G[u][v] = sum_p Ar[p][u] Br[p][v], u, v over
 // n = 2 nst lanes.  grid (tile pairs, splits over the points); block 256.
 // sym: a is b, only the tiles on and above the diagonal are listed (the matrix
 // is Hermitian).  Partials [splits][n][n].
+// FOLD: for splits of more than 8192 points (many tiles: 3 splits for 512 states,
+// one from 660 on): after every GFOLD steps the sums go into the partials with
+// compensation, whose remainders follow them ([splits][n][n] again), so that no plain sum
+// runs over more than 8192 points.
 // 96 states, 267,761 points, FP64: 0.468 ms (one triangle; 78 % of the FP64 rate),
 // the update below 0.50 ms; orthonormalisation and overlap together 9.5 -> 1.72 ms
 // (before: 2 x 2 register blocks per thread over 32 x 32 tiles, one output of the
 // update per thread).
-template <typename T>
+template <typename T, bool FOLD>
 __global__ void __launch_bounds__(256) gram_kernel(const T *a, long long lda, const T *b, long long ldb, int np,
                                                   int n, int tiles, int sym, double *partial) {
   constexpr int PITCH = gram_pitch<T>();
@@ -177,9 +193,23 @@ __global__ void __launch_bounds__(256) gram_kernel(const T *a, long long lda, co
     }
     cp_async_commit();
   };
+  double *o = partial + (long long)blockIdx.y * n * n;
   double c[2][4][2] = {};
   for (int k = 0; k < GST - 1; ++k) stage(k);
   for (int k = 0; k < nk; ++k) {
+    if constexpr (FOLD) {
+      if (k && k % GFOLD == 0) {
+        double *oc = o + (long long)gridDim.y * n * n;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int u = u0 + wu + 8 * i + (lane >> 2), v = v0 + wv + 8 * j + 2 * (lane & 3);
+            if (u < n && v < n) gram_fold(o, oc, (long long)u * n + v, k == GFOLD, c[i][j]);
+            c[i][j][0] = c[i][j][1] = 0.0;
+          }
+      }
+    }
     cp_async_wait<GST - 2>();
     __syncthreads();
     stage(k + GST - 1);
@@ -198,21 +228,25 @@ __global__ void __launch_bounds__(256) gram_kernel(const T *a, long long lda, co
     }
   }
   cp_async_wait<0>();
-  double *o = partial + (long long)blockIdx.y * n * n;
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int u = u0 + wu + 8 * i + (lane >> 2), v = v0 + wv + 8 * j + 2 * (lane & 3);
-      if (u < n && v < n) *reinterpret_cast<double2 *>(o + (long long)u * n + v) = make_double2(c[i][j][0], c[i][j][1]);
+      if (u >= n || v >= n) continue;
+      if constexpr (FOLD)
+        gram_fold(o, o + (long long)gridDim.y * n * n, (long long)u * n + v, nk <= GFOLD, c[i][j]);
+      else
+        *reinterpret_cast<double2 *>(o + (long long)u * n + v) = make_double2(c[i][j][0], c[i][j][1]);
     }
 }
 
 // S[i][j] = dV * (conj(a_i) . b_j) from the real Gram G (n = 2 * nst); sym:
 // G holds the tiles on and above the diagonal, entries below it are conjugates.
 // block (32, 8): 8 slices of the splits per entry, folded in a fixed order.
+// rest: the partials' remainders follow them.
 __global__ void __launch_bounds__(256) gram_finalize(const double *partial, int splits, int nst, double dv, int sym,
-                                                     double *S) {
+                                                     int rest, double *S) {
   __shared__ double red[8][32][4];
   const int i = blockIdx.y, j = blockIdx.x * 32 + threadIdx.x;
   const int n = 2 * nst;
@@ -228,6 +262,11 @@ __global__ void __launch_bounds__(256) gram_finalize(const double *partial, int 
       kadd(re, g1.y);
       kadd(im, g0.y);
       kadd(im, -g1.x);
+      if (rest) {
+        const double2 *R0 = G0 + (long long)splits * n * nst;
+        re.c += R0[0].x + R0[nst].y;
+        im.c += R0[0].y - R0[nst].x;
+      }
     }
   }
   red[threadIdx.y][threadIdx.x][0] = re.s;
@@ -572,13 +611,20 @@ hpsi_status launch_state_sum(int mode, const T *a, long long lda, const T *b, lo
 }
 
 // Splits of the points: as many CTAs as the SMs hold at once (three each), at
-// least 64 points each, and partial matrices of at most 64 MB.
-int gram_splits(int np, int nst, bool sym) {
+// least 64 points each, and partial matrices of at most 64 MB (but for one split).
+int gram_splits(int np, int nst, bool sym, int num_sms) {
   const long long tiles = (2LL * nst + GT - 1) / GT, pairs = sym ? tiles * (tiles + 1) / 2 : tiles * tiles;
-  long long s = std::max<long long>(1, 3LL * 148 / pairs);
+  long long s = std::max<long long>(1, 3LL * num_sms / pairs);
   s = std::min<long long>(s, (np + 63) / 64);
   s = std::min<long long>(s, std::max<long long>(1, (64LL << 20) / (4LL * nst * nst * 8)));
   return int(std::max<long long>(1, std::min<long long>(s, 65535)));
+}
+
+// Points of a split: more than 8192 are folded in pieces.
+static bool gram_folds(int np, int splits) { return (np + splits - 1) / splits > GFOLD * GK; }
+
+size_t gram_partial_doubles(int np, int nst, int splits) {
+  return size_t(splits) * 4 * nst * nst * (gram_folds(np, splits) ? 2 : 1);
 }
 
 template <typename T>
@@ -590,14 +636,17 @@ hpsi_status launch_gram(const T *a, long long lda, const T *b, long long ldb, in
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
   std::call_once(once, [&] {
-    attr = cudaFuncSetAttribute(gram_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    attr = cudaFuncSetAttribute(gram_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (attr == cudaSuccess)
+      attr = cudaFuncSetAttribute(gram_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   });
   HPSI_TRY_CUDA(attr);
   const long long pairs = sym ? (long long)tiles * (tiles + 1) / 2 : (long long)tiles * tiles;
-  gram_kernel<T><<<dim3(unsigned(pairs), unsigned(splits)), 256, smem, st>>>(a, lda, b, ldb, np, n, tiles, sym,
-                                                                             partial);
+  const bool fold = gram_folds(np, splits);
+  auto kern = fold ? gram_kernel<T, true> : gram_kernel<T, false>;
+  kern<<<dim3(unsigned(pairs), unsigned(splits)), 256, smem, st>>>(a, lda, b, ldb, np, n, tiles, sym, partial);
   HPSI_CHECK_LAUNCH();
-  gram_finalize<<<dim3((nst + 31) / 32, nst), dim3(32, 8), 0, st>>>(partial, splits, nst, dv, sym, S);
+  gram_finalize<<<dim3((nst + 31) / 32, nst), dim3(32, 8), 0, st>>>(partial, splits, nst, dv, sym, fold, S);
   HPSI_CHECK_LAUNCH();
   return HPSI_OK;
 }

@@ -9,7 +9,8 @@ namespace hpsi {
 constexpr int ORTHO_MAX_STATES = 3072;
 
 int reduce_blocks(int np);
-int gram_splits(int np, int nst, bool sym);
+int gram_splits(int np, int nst, bool sym, int num_sms);
+size_t gram_partial_doubles(int np, int nst, int splits);
 
 // mode 0: out[2*s] = scale * sum |a_s|^2 (sqrt if sqrt_first); mode 1:
 // out[2*s], out[2*s+1] = scale * sum conj(a_s) b_s.  partial: nblk*nst*4 doubles.
@@ -18,7 +19,7 @@ hpsi_status launch_state_sum(int mode, const T *a, long long lda, const T *b, lo
                              double *partial, int nblk, double scale, int sqrt_first, double *out,
                              cudaStream_t st);
 
-// S (complex nst x nst, interleaved) = dv * a^H b.  partial: splits*(2nst)^2 doubles,
+// S (complex nst x nst, interleaved) = dv * a^H b.  partial: gram_partial_doubles,
 // splits from gram_splits (sym: a and b are the same batch).
 template <typename T>
 hpsi_status launch_gram(const T *a, long long lda, const T *b, long long ldb, int np, int nst, double *partial,

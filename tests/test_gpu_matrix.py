@@ -82,3 +82,24 @@ def test_too_many_states_are_refused(cuda):
     x = torch.zeros((m.np, 3074), dtype=torch.complex64, device=cuda)
     with pytest.raises(lib.HpsiError, match="3072"):
         lib.DeviceMesh(m).orthonormalize_cholesky(x, nst=3073)
+
+
+@pytest.mark.parametrize("dtype", ["c128", "c64"])
+@pytest.mark.parametrize("nst,same", [(641, True), (480, False), (512, True)])
+def test_long_sums_are_folded(cuda, dtype, nst, same):
+    """One split (641 states, or two batches of 480) or few over 216,000 points.  The
+    first row is so large that every later product is lost when it is added to a
+    plain running sum: a sum in one chain is off by 5e-12."""
+    import torch
+    from hpsi import lib
+    from hpsi.mesh import index_box_mesh
+    m = index_box_mesh((60, 60, 60), 0.25)
+    tdt = torch.complex128 if dtype == "c128" else torch.complex64
+    ld = nst + nst % 2
+    x = torch.full((m.np, ld), 0.66, dtype=tdt, device=cuda)
+    x[0] = 2.0 ** 27
+    small = float(x[1, 0].real.item()) ** 2
+    S = lib.DeviceMesh(m).dotp_matrix(x, x if same else x.clone(), nst=nst)
+    ref = m.vol_pp * (2.0 ** 54 + (m.np - 1) * small)
+    # plain sums run over 8192 points at most: 8192 roundings of half an eps each
+    assert np.max(np.abs(S - ref)) <= 8192 * np.finfo(float).eps / 2 * ref
