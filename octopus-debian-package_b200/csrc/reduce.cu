@@ -124,6 +124,13 @@ __device__ __forceinline__ void copy_state(float *d, const float *g, bool ok) {
   const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(d));
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(g), "r"(ok ? 8 : 0));
 }
+// The same in pieces of one real.
+__device__ __forceinline__ void copy_state_reals(float *d, const float *g, bool ok) {
+  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(d));
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s + 4 * i), "l"(g + i), "r"(ok ? 4 : 0));
+}
 // Row pitch of a staged K x 64 block: the four K rows of a fragment read fall
 // into different bank groups (FP64 pitch = 4 mod 16, FP32 = 8 mod 32).
 template <typename T>
@@ -154,7 +161,9 @@ __device__ __forceinline__ void gram_fold(double *o, double *oc, long long at, b
 // the update below 0.50 ms; orthonormalisation and overlap together 9.5 -> 1.72 ms
 // (before: 2 x 2 register blocks per thread over 32 x 32 tiles, one output of the
 // update per thread).
-template <typename T, bool FOLD>
+// REALS: rows that start on 4-byte boundaries only (FP32 batches of width 1, the only
+// ones whose alignment nothing checks).
+template <typename T, bool FOLD, bool REALS = false>
 __global__ void __launch_bounds__(256) gram_kernel(const T *a, long long lda, const T *b, long long ldb, int np,
                                                   int n, int tiles, int sym, double *partial) {
   constexpr int PITCH = gram_pitch<T>();
@@ -187,8 +196,14 @@ __global__ void __launch_bounds__(256) gram_kernel(const T *a, long long lda, co
         const long long row = p0 + (long long)k * GK + pp;
         const bool in = row < p1;
         const bool ua = in && u0 + l < n, vb = in && v0 + l < n;
-        copy_state(sa + (s * GK + pp) * PITCH + l, ua ? a + row * 2 * lda + u0 + l : a, ua);
-        if (!same) copy_state(sb + (s * GK + pp) * PITCH + l, vb ? b + row * 2 * ldb + v0 + l : b, vb);
+        auto copy = [](T *d, const T *g, bool ok) {
+          if constexpr (REALS)
+            copy_state_reals(d, g, ok);
+          else
+            copy_state(d, g, ok);
+        };
+        copy(sa + (s * GK + pp) * PITCH + l, ua ? a + row * 2 * lda + u0 + l : a, ua);
+        if (!same) copy(sb + (s * GK + pp) * PITCH + l, vb ? b + row * 2 * ldb + v0 + l : b, vb);
       }
     }
     cp_async_commit();
@@ -644,6 +659,11 @@ hpsi_status launch_gram(const T *a, long long lda, const T *b, long long ldb, in
   const long long pairs = sym ? (long long)tiles * (tiles + 1) / 2 : (long long)tiles * tiles;
   const bool fold = gram_folds(np, splits);
   auto kern = fold ? gram_kernel<T, true> : gram_kernel<T, false>;
+  if constexpr (sizeof(T) == 4) {
+    static_assert(smem <= 48 * 1024, "no opt-in shared memory");
+    if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) % 8 != 0)
+      kern = fold ? gram_kernel<T, true, true> : gram_kernel<T, false, true>;
+  }
   kern<<<dim3(unsigned(pairs), unsigned(splits)), 256, smem, st>>>(a, lda, b, ldb, np, n, tiles, sym, partial);
   HPSI_CHECK_LAUNCH();
   gram_finalize<<<dim3((nst + 31) / 32, nst), dim3(32, 8), 0, st>>>(partial, splits, nst, dv, sym, fold, S);

@@ -103,3 +103,24 @@ def test_long_sums_are_folded(cuda, dtype, nst, same):
     ref = m.vol_pp * (2.0 ** 54 + (m.np - 1) * small)
     # plain sums run over 8192 points at most: 8192 roundings of half an eps each
     assert np.max(np.abs(S - ref)) <= 8192 * np.finfo(float).eps / 2 * ref
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2])
+def test_overlap_of_an_unaligned_single_state(cuda, offset):
+    """FP32 batches of width 1 may start on any 4-byte boundary."""
+    import ctypes as C
+    import torch
+    from hpsi import lib
+    m = _mesh()
+    dm = lib.DeviceMesh(m)
+    g = torch.Generator(device=cuda).manual_seed(5)
+    buf = torch.randn(2 * m.np + 4, device=cuda, generator=g)
+    b = lib.Batch()
+    b.dtype, b.ptr, b.ld, b.npts, b.nst = lib.HPSI_C64, buf.data_ptr() + 4 * offset, 1, m.np, 1
+    out = np.zeros(2)
+    lib.check(lib.load().hpsi_dotp_matrix(dm.handle, C.byref(b), C.byref(b), out.ctypes.data_as(C.POINTER(C.c_double)),
+                                          None))
+    x = buf[offset: offset + 2 * m.np].double().cpu().numpy()
+    torch.cuda.synchronize()
+    ref = m.vol_pp * float(x @ x)
+    assert abs(out[0] - ref) <= 4 * m.np * np.finfo(float).eps * ref and out[1] == 0.0
