@@ -674,6 +674,7 @@ void hpsi_hamiltonian::proj_free() {
   kb_tables = nullptr;
   d_kidx = nullptr;
   d_kblk = nullptr;
+  d_brow = nullptr;
   d_pk = nullptr;
   d_pk_f = nullptr;
   nkblk = 0;
@@ -881,8 +882,9 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, c
       const int row = map[mat[i].z + k];
       ent[fill[row]++] = make_int4(mat[i].w + k * nprojs[i], prow[i], nprojs[i], mat[i].z + k);
     }
-  // compress to the covered rows (entries stay in matrix order per row), rows
-  // with the same list of matrices together: each list's rows in mesh order
+  // compress to the covered rows (entries stay in matrix order per row); for the
+  // blocks rows with the same list of matrices together, each list's rows in
+  // mesh order
   std::vector<std::vector<int>> lists;
   {
     std::unordered_map<unsigned long long, int> by_hash;
@@ -912,27 +914,26 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, c
     }
   }
   std::vector<int> krows, kptr(1, 0);
-  std::vector<int4> ent_row, blk;
+  for (int r = 0; r < m->np; ++r)
+    if (cnt[r + 1] > cnt[r]) {
+      krows.push_back(r);
+      kptr.push_back(cnt[r + 1]);
+    }
+  std::vector<int4> blk;
+  std::vector<int2> brow;
   std::vector<double> pk;
-  ent_row.reserve(ent.size());
   pk.reserve(nval);
   for (const auto &l : lists)
     for (size_t i = 0; i < l.size(); i += 32) {
       const int n = int(std::min<size_t>(32, l.size() - i)), ne = cnt[l[i] + 1] - cnt[l[i]];
-      blk.push_back(make_int4(int(krows.size()), n + 256 * ne, int(ent_row.size()), int(pk.size())));
+      blk.push_back(make_int4(int(brow.size()), n + 256 * ne, cnt[l[i]], int(pk.size())));
       for (int e = 0; e < ne; ++e)
         for (int q = 0; q < n; ++q) {
           const int4 E = ent[cnt[l[i + q]] + e];
           pk.insert(pk.end(), pt.begin() + E.x, pt.begin() + E.x + E.z);
         }
-      for (int q = 0; q < n; ++q) {
-        const int r = l[i + q];
-        krows.push_back(r);
-        ent_row.insert(ent_row.end(), ent.begin() + cnt[r], ent.begin() + cnt[r + 1]);
-        kptr.push_back(int(ent_row.size()));
-      }
+      for (int q = 0; q < n; ++q) brow.push_back(make_int2(l[i + q], cnt[l[i + q]]));
     }
-  ent.swap(ent_row);
   std::vector<float> pkf(pk.begin(), pk.end());
   int minp = 1 << 30;
   for (int i = 0; i < nmat; ++i) minp = std::min(minp, int(npoints[i]));
@@ -958,6 +959,7 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, c
   up(reinterpret_cast<void **>(&h->d_kptr), kptr.data(), kptr.size() * sizeof(int));
   up(reinterpret_cast<void **>(&h->d_kb_ent), ent.data(), ent.size() * sizeof(int4));
   up(reinterpret_cast<void **>(&h->d_kblk), blk.data(), blk.size() * sizeof(int4));
+  up(reinterpret_cast<void **>(&h->d_brow), brow.data(), brow.size() * sizeof(int2));
   up(reinterpret_cast<void **>(&h->d_pk), pk.data(), pk.size() * sizeof(double));
   up(reinterpret_cast<void **>(&h->d_pk_f), pkf.data(), pkf.size() * sizeof(float));
   size_t total = 0;
@@ -983,6 +985,7 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, c
   h->max_nproj = maxp;
   h->nk = int(krows.size());
   h->nkblk = int(blk.size());
+  h->kb_nproj = double(nval) / double(std::max(1LL, npts_tot));
   h->min_npoints = minp;
   h->kb_npts = npts_tot;
   h->kb_npoints_h.assign(npoints, npoints + nmat);
@@ -1398,6 +1401,9 @@ hpsi_status run_ket(hpsi_hamiltonian *h, const T *proj, long long ld, int nst, T
   k.nk = h->nk;
   k.nblk = h->nkblk;
   k.blk = h->d_kblk;
+  k.brow = h->d_brow;
+  k.rows_per_block = h->nkblk > 0 ? double(h->nk) / h->nkblk : 0.0;
+  k.nproj_per_point = h->kb_nproj;
   k.pk = sizeof(T) == 8 ? static_cast<const void *>(h->d_pk) : static_cast<const void *>(h->d_pk_f);
   k.max_nproj = h->max_nproj;
   k.krows = h->d_krows;

@@ -121,6 +121,8 @@ struct hpsi_hamiltonian {
   // their projector values in block order
   int nkblk = 0;
   int4 *d_kblk = nullptr;
+  int2 *d_brow = nullptr;
+  double kb_nproj = 0.0;  // projectors per sphere point, on average
   double *d_pk = nullptr;
   float *d_pk_f = nullptr;
   // projector phases (k != 0): one complex number per sphere point, or null

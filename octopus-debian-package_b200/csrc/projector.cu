@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(256, PHASE ? 2 : 4) ket_block_kernel(const Ket
   const int per = (k.nblk + gridDim.y - 1) / gridDim.y;
   const int b0 = blockIdx.y * per, b1 = min(k.nblk, b0 + per);
   for (int b = b0; b < b1; ++b) {
-    const int4 D = __ldg(k.blk + b);  // {first covered row, rows + 256 * entries per row, first entry, value offset}
+    const int4 D = __ldg(k.blk + b);  // {first row, rows + 256 * entries per row, its first entry, value offset}
     const int cnt = D.y & 255, ne = D.y >> 8;
 #pragma unroll 1
     for (int half = 0; half < HALVES; ++half) {
@@ -461,10 +461,13 @@ __global__ void __launch_bounds__(256, PHASE ? 2 : 4) ket_block_kernel(const Ket
     if (half && cnt <= KET_ROWS / HALVES) break;  // (the same for the whole CTA)
     const T *w = static_cast<const T *>(k.pk) + D.w;
     int row[RPT];
+    [[maybe_unused]] int ent0[RPT];  // the rows' first entries
     C2 y[RPT], h[RPT];
 #pragma unroll
     for (int q = 0; q < RPT; ++q) {
-      row[q] = r0 + q < cnt ? __ldg(k.krows + D.x + r0 + q) : -1;
+      const int2 R = r0 + q < cnt ? __ldg(k.brow + D.x + r0 + q) : make_int2(-1, 0);
+      row[q] = R.x;
+      if constexpr (PHASE) ent0[q] = R.y;
       h[q].x = 0;
       h[q].y = 0;
     }
@@ -512,7 +515,7 @@ __global__ void __launch_bounds__(256, PHASE ? 2 : 4) ket_block_kernel(const Ket
 #pragma unroll
           for (int q = 0; q < RPT; ++q) {
             if (row[q] < 0) continue;
-            const int pnt = __ldg(k.ent + D.z + (long long)(r0 + q) * ne + e).w;
+            const int pnt = __ldg(k.ent + ent0[q] + e).w;
             const T *ph = static_cast<const T *>(k.phase) + 2 * (long long)pnt;
             const T c = ph[0], sn = ph[1];
             h[q].x += g[q].x * c + g[q].y * sn;
@@ -584,6 +587,35 @@ hpsi_status launch_ket_blocks_w(const KetArgs &k, int rb, cudaStream_t st) {
 }
 }  // namespace
 
+// Whether the blocks are the faster form.  They gain where a block is well filled
+// (rows_per_block of at most 32: many overlapping spheres make many lists of a few
+// rows each) and where the rows above wait for many projections (wide batches,
+// many projectors); with phases their registers halve the CTAs per SM.  Kernel
+// alone on a 60^3 mesh at 0.25 bohr, us, rows / blocks (spheres of 2 bohr with 9
+// projectors: 32 of them 29.6 rows per block; 400 of 1.2 bohr 9.6; 32 with 18
+// projectors 30.4):
+//                                   FP64 8 states    32       128     FP32 8     32       128
+//   29.6 rows, 9 projectors           25 / 16    44 / 23   94 / 75   18 / 15  34 / 19   60 / 48
+//   9.6 rows, 9 projectors            43 / 66   111 / 101 253 / 299  33 / 64  77 / 78  164 / 228
+//   29.6 rows, 9 projectors, phases   25 / 24    47 / 32  103 / 130  21 / 19  37 / 29   70 / 91
+//   30.4 rows, 18 projectors, phases  26 / 26    71 / 37  168 / 152  23 / 18  55 / 33  108 / 106
+//   9.6 rows, 9 projectors, phases    45 / 136  121 / 185 281 / 607  35 / 92  90 / 160 210 / 526
+// The lines below lie between measured sides of 24 such sets (1 to 32 projectors, 9.6 to
+// 31.6 rows, 2 to 128 states).
+template <typename T>
+static bool ket_blocks_better(const KetArgs &k) {
+  const double rows = k.rows_per_block, q = k.nproj_per_point;
+  const bool f64 = sizeof(T) == 8;
+  if (k.phase) {
+    if (k.nst > 16 && k.nst <= 32) return rows >= 25;
+    return rows >= 28 && q >= (f64 || k.nst <= 64 ? 16 : 24);
+  }
+  if (k.nst > 32) return rows >= 20;
+  if (k.nst > 16) return rows >= 14;
+  if (k.nst > 8) return rows >= (q >= 8 ? 20 : 28);
+  return q >= 8 && rows >= (f64 ? 20 : 29);
+}
+
 // At most 1024 CTA rows, each over a contiguous range of covered rows: one
 // row per thread (up to 65535 CTA rows) measured 45 % slower on the R = 12
 // sphere, the projections of neighbouring rows no longer sharing L1.
@@ -602,7 +634,7 @@ hpsi_status launch_ket(const KetArgs &k, cudaStream_t st) {
   const int rb = k.row_blocks > 0 ? std::min(k.row_blocks, ket_row_blocks(k.nk)) : ket_row_blocks(k.nk);
   // the fused density needs the row's states in one warp (the form above); so
   // do matrices whose projections would not fit shared memory
-  if (!k.rho_ket && k.blk && size_t(k.max_nproj) * (64 * sizeof(C2) + KET_ROWS * sizeof(T)) <= 200 * 1024) {
+  if (!k.rho_ket && k.blk && ket_blocks_better<T>(k) && size_t(k.max_nproj) * (64 * sizeof(C2) + KET_ROWS * sizeof(T)) <= 200 * 1024) {
     // a CTA per block, but where the energy partials count the CTA rows or the
     // launch shares the GPU
     const int rows = k.obs || k.row_blocks > 0 ? rb : std::min(k.nblk, 65535);

@@ -31,13 +31,16 @@ struct KetArgs {
   const int *krows;      // covered row -> mesh row
   const int *kptr;       // nk + 1 offsets into ent
   const int4 *ent;       // {projector value offset, projection row, nproj, 0}
-  // blocks of at most 32 consecutive covered rows with the same list of
-  // matrices: {first covered row, rows + 256 * entries per row, first entry,
-  // offset into pk}; pk: per block and matrix the rows' projector values
+  // blocks of at most 32 covered rows with the same list of matrices: {first
+  // row in brow, rows + 256 * entries per row, the first row's first entry,
+  // offset into pk}; brow: {row, its first entry} in block order; pk: per
+  // block and matrix the rows' projector values
   int nblk = 0;
   const int4 *blk = nullptr;
+  const int2 *brow = nullptr;
   const void *pk = nullptr;
   int max_nproj = 0;
+  double rows_per_block = 0.0, nproj_per_point = 0.0;  // averages, for the choice of the form
   const void *pt;        // projector values
   const void *proj;      // projections [nprojections][proj_ld] complex
   long long proj_ld;

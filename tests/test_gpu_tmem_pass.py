@@ -147,18 +147,26 @@ def test_group_of_unequal_spacings_and_phases(cuda, dtype, phases):
 @pytest.mark.parametrize("dtype", ["c128", "c64"])
 @pytest.mark.parametrize("nst", [2, 8, 10, 16, 18, 32, 34, 66])
 @pytest.mark.parametrize("phased", [False, True])
-def test_ket_widths(cuda, dtype, nst, phased):
-    """Overlapping spheres (rows of one to three matrices) of unequal projector counts."""
+@pytest.mark.parametrize("spheres", ["few", "many projectors", "many spheres"])
+def test_ket_widths(cuda, dtype, nst, phased, spheres):
+    """Overlapping spheres of unequal projector counts: three (rows of one to three
+    matrices in well-filled blocks), three with 18 projectors on average, and forty
+    small ones (lists of a few rows each: one row at a time at every width)."""
     import torch
     from hpsi.mesh import sphere_mesh
     rng = np.random.default_rng(31)
     m = sphere_mesh(3.0, 0.3)
     x = m.x[: m.np]
+    atoms = [((0.0, 0.1, 0.2), 1.3, 9), ((0.9, 0.0, 0.0), 1.2, 4), ((0.3, 0.8, 0.1), 1.0, 1)]
+    if spheres == "many projectors":
+        atoms = [(c, r, q + 14) for c, r, q in atoms]
+    if spheres == "many spheres":
+        atoms = [(rng.uniform(-1.4, 1.4, 3), 0.9, 1 + i % 9) for i in range(40)]
 
     class P:
         maps, mats, scals = [], [], []
     P.maps, P.mats, P.scals = [], [], []
-    for c, r, q in [((0.0, 0.1, 0.2), 1.3, 9), ((0.9, 0.0, 0.0), 1.2, 4), ((0.3, 0.8, 0.1), 1.0, 1)]:
+    for c, r, q in atoms:
         sel = np.nonzero(np.sum((x - np.array(c)) ** 2, axis=1) <= r * r)[0].astype(np.int32)
         P.maps.append(sel)
         P.mats.append(rng.standard_normal((len(sel), q)))
