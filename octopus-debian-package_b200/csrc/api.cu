@@ -6,9 +6,9 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <string>
-#include <unordered_map>
 #include <queue>
 #include <vector>
 
@@ -73,6 +73,30 @@ namespace {
 __global__ void scatter_cells_kernel(const double *v, const int *cell_of_row, int n, double *vcell) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) vcell[cell_of_row[i]] = v[i];
+}
+
+// Tables of the projectors that the device makes itself: the values in FP32,
+// the covered rows' numbers (kidx, -1 before) and the values in block order (KetArgs::pk).
+__global__ void __launch_bounds__(256) kb_layout_kernel(const double *pt, long long nval, const int *krows, int nk,
+                                                        const int4 *blk, int nblk, const int2 *brow, const int4 *ent,
+                                                        float *ptf, int *kidx, double *pk, float *pkf) {
+  const long long t0 = blockIdx.x * 256LL + threadIdx.x, step = gridDim.x * 256LL;
+  for (long long i = t0; i < nval; i += step) ptf[i] = float(pt[i]);
+  for (long long i = t0; i < nk; i += step) kidx[krows[i]] = int(i);
+  for (int b = blockIdx.x; b < nblk; b += gridDim.x) {
+    const int4 D = blk[b];
+    const int n = D.y & 255, ne = D.y >> 8;
+    int w = D.w;
+    for (int e = 0; e < ne; ++e) {
+      const int q = ent[D.z + e].z;
+      for (int i = threadIdx.x; i < n * q; i += 256) {
+        const double v = pt[ent[brow[D.x + i / q].y + e].x + i % q];
+        pk[w + i] = v;
+        pkf[w + i] = float(v);
+      }
+      w += n * q;
+    }
+  }
 }
 
 // rho[r] (+)= the density of row r from the fused partials: the KB ket's row
@@ -828,6 +852,72 @@ hpsi_status hpsi_hamiltonian_set_phase_corr(hpsi_hamiltonian *h, const double *p
   return HPSI_OK;
 }
 
+// Covered rows of the projector spheres, in mesh order: krows[nk], kptr[nk + 1],
+// ent their entries in matrix order; and in blocks of rows with the same list of
+// matrices (KetArgs::blk, brow; lists in the order of their first row).  A
+// row's list is a number: matrix i leads from a list to the list with i at its
+// end, so that one pass over the points finds them all.
+struct KbRows {
+  std::vector<int> krows, kptr;
+  std::vector<int4> ent, blk;
+  std::vector<int2> brow;
+};
+static void kb_rows(int np, const std::vector<int4> &mat, const std::vector<int> &prow, const int *map, KbRows &o) {
+  struct List {
+    int len, nproj;   // matrices, projectors of all of them
+    int from, next;   // last matrix seen at this list, the list it leads to
+    int rows, first;  // rows of the list, place of the next one
+  };
+  std::vector<List> lists(1, List{0, 0, -1, 0, 0, 0});  // list 0: no matrix
+  std::vector<int> id(np, 0);
+  for (int i = 0; i < int(mat.size()); ++i)
+    for (int k = 0; k < mat[i].x; ++k) {
+      int &at = id[map[mat[i].z + k]];
+      if (lists[at].from != i) {
+        lists[at].from = i;
+        lists[at].next = int(lists.size());
+        lists.push_back(List{lists[at].len + 1, lists[at].nproj + mat[i].y, -1, 0, 0, 0});
+      }
+      at = lists[at].next;
+    }
+  std::vector<int> order;  // lists by their first row
+  int nk = 0;
+  for (int r = 0; r < np; ++r)
+    if (id[r]) {
+      if (lists[id[r]].rows++ == 0) order.push_back(id[r]);
+      ++nk;
+    }
+  int at = 0, npk = 0;
+  for (int l : order) {
+    List &L = lists[l];
+    L.first = at;
+    for (int i = 0; i < L.rows; i += 32) {
+      const int n = std::min(32, L.rows - i);
+      o.blk.push_back(make_int4(at + i, n + 256 * L.len, 0, npk));
+      npk += n * L.nproj;
+    }
+    at += L.rows;
+  }
+  o.krows.reserve(nk);
+  o.kptr.reserve(size_t(nk) + 1);
+  o.kptr.push_back(0);
+  o.brow.resize(nk);
+  for (int r = 0; r < np; ++r)
+    if (id[r]) {
+      List &L = lists[id[r]];
+      const int e = o.kptr.back();
+      o.brow[L.first++] = make_int2(r, e);
+      o.krows.push_back(r);
+      o.kptr.push_back(e + L.len);
+      id[r] = e;  // place of the row's next entry
+    }
+  for (int4 &b : o.blk) b.z = o.brow[b.x].y;
+  o.ent.resize(o.kptr.back());
+  for (int i = 0; i < int(mat.size()); ++i)
+    for (int k = 0; k < mat[i].x; ++k)
+      o.ent[id[map[mat[i].z + k]]++] = make_int4(mat[i].w + k * mat[i].y, prow[i], mat[i].y, mat[i].z + k);
+}
+
 hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, const int32_t *npoints,
                                             const int32_t *nprojs, const int32_t *map, const double *matrices,
                                             const double *scal) {
@@ -853,12 +943,13 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, c
     maxp = std::max(maxp, int(nprojs[i]));
   }
   if (nval > (1LL << 31) - 1) return HPSI_ERR_UNSUPPORTED;
-  std::vector<double> pt(nval);
-  std::vector<float> ptf(nval), scf(nproj_tot);
-  std::vector<int> cnt(m->np + 1, 0);
+  // values by point (a point's projectors together), read by the bra and the ket
+  std::unique_ptr<double[]> pt(new double[nval]);
+  std::vector<float> scf(scal, scal + nproj_tot);
   for (int i = 0; i < nmat; ++i) {
     const int n = npoints[i], q = nprojs[i];
     const double *src = matrices + mat[i].w;
+    double *dst = pt.get() + mat[i].w;
     for (int k = 0; k < n; ++k) {
       const int row = map[mat[i].z + k];
       if (row < 0 || row >= m->np) {
@@ -866,102 +957,42 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, c
                   " is not an inner point");
         return HPSI_ERR_INDEX;
       }
-      cnt[row + 1]++;
-      for (int j = 0; j < q; ++j) {
-        pt[mat[i].w + (long long)k * q + j] = src[(long long)j * n + k];
-        ptf[mat[i].w + (long long)k * q + j] = float(src[(long long)j * n + k]);
-      }
+      for (int j = 0; j < q; ++j) *dst++ = src[(long long)j * n + k];
     }
   }
-  for (int i = 0; i < nproj_tot; ++i) scf[i] = float(scal[i]);
-  for (int r = 0; r < m->np; ++r) cnt[r + 1] += cnt[r];
-  std::vector<int4> ent(npts_tot);
-  std::vector<int> fill(cnt.begin(), cnt.end() - 1);
-  for (int i = 0; i < nmat; ++i)
-    for (int k = 0; k < npoints[i]; ++k) {
-      const int row = map[mat[i].z + k];
-      ent[fill[row]++] = make_int4(mat[i].w + k * nprojs[i], prow[i], nprojs[i], mat[i].z + k);
-    }
-  // compress to the covered rows (entries stay in matrix order per row); for the
-  // blocks rows with the same list of matrices together, each list's rows in
-  // mesh order
-  std::vector<std::vector<int>> lists;
-  {
-    std::unordered_map<unsigned long long, int> by_hash;
-    for (int r = 0; r < m->np; ++r) {
-      const int e0 = cnt[r], e1 = cnt[r + 1];
-      if (e1 == e0) continue;
-      unsigned long long hash = 1469598103934665603ull;
-      for (int e = e0; e < e1; ++e) hash = (hash ^ (unsigned long long)(ent[e].y + 1)) * 1099511628211ull;
-      auto same = [&](int q) {
-        if (cnt[q + 1] - cnt[q] != e1 - e0) return false;
-        for (int e = 0; e < e1 - e0; ++e)
-          if (ent[cnt[q] + e].y != ent[e0 + e].y) return false;
-        return true;
-      };
-      for (;; ++hash) {  // (a list that shares another's hash takes the next free one)
-        auto it = by_hash.find(hash);
-        if (it == by_hash.end()) {
-          by_hash.emplace(hash, int(lists.size()));
-          lists.emplace_back(1, r);
-          break;
-        }
-        if (same(lists[it->second][0])) {
-          lists[it->second].push_back(r);
-          break;
-        }
-      }
-    }
-  }
-  std::vector<int> krows, kptr(1, 0);
-  for (int r = 0; r < m->np; ++r)
-    if (cnt[r + 1] > cnt[r]) {
-      krows.push_back(r);
-      kptr.push_back(cnt[r + 1]);
-    }
-  std::vector<int4> blk;
-  std::vector<int2> brow;
-  std::vector<double> pk;
-  pk.reserve(nval);
-  for (const auto &l : lists)
-    for (size_t i = 0; i < l.size(); i += 32) {
-      const int n = int(std::min<size_t>(32, l.size() - i)), ne = cnt[l[i] + 1] - cnt[l[i]];
-      blk.push_back(make_int4(int(brow.size()), n + 256 * ne, cnt[l[i]], int(pk.size())));
-      for (int e = 0; e < ne; ++e)
-        for (int q = 0; q < n; ++q) {
-          const int4 E = ent[cnt[l[i + q]] + e];
-          pk.insert(pk.end(), pt.begin() + E.x, pt.begin() + E.x + E.z);
-        }
-      for (int q = 0; q < n; ++q) brow.push_back(make_int2(l[i + q], cnt[l[i + q]]));
-    }
-  std::vector<float> pkf(pk.begin(), pk.end());
+  KbRows R;
+  kb_rows(m->np, mat, prow, map, R);
+  const int nk = int(R.krows.size());
+  // lists of a few rows each: no block form (ket_blocks_better)
+  const int nblk = (long long)R.blk.size() * KET_BLOCK_ROWS <= nk ? int(R.blk.size()) : 0;
+  const int npk = nblk ? int(nval) : 0;
   int minp = 1 << 30;
   for (int i = 0; i < nmat; ++i) minp = std::min(minp, int(npoints[i]));
-  // one allocation for all tables
+  // one allocation for all tables; those without a source are made on the device
   struct Part {
     void **dp;
     const void *src;
     size_t bytes;
   };
   std::vector<Part> parts;
-  auto up = [&](void **dp, const void *src, size_t bytes) { parts.push_back({dp, src, bytes}); };
-  up(reinterpret_cast<void **>(&h->d_mat), mat.data(), mat.size() * sizeof(int4));
-  up(reinterpret_cast<void **>(&h->d_proj_row), prow.data(), prow.size() * sizeof(int));
-  up(reinterpret_cast<void **>(&h->d_map), map, size_t(npts_tot) * sizeof(int));
-  up(reinterpret_cast<void **>(&h->d_pt), pt.data(), pt.size() * sizeof(double));
-  up(reinterpret_cast<void **>(&h->d_pt_f), ptf.data(), ptf.size() * sizeof(float));
-  up(reinterpret_cast<void **>(&h->d_scal), scal, size_t(nproj_tot) * sizeof(double));
-  up(reinterpret_cast<void **>(&h->d_scal_f), scf.data(), scf.size() * sizeof(float));
-  up(reinterpret_cast<void **>(&h->d_krows), krows.data(), krows.size() * sizeof(int));
-  std::vector<int> kidx(m->np, -1);
-  for (size_t i = 0; i < krows.size(); ++i) kidx[krows[i]] = int(i);
-  up(reinterpret_cast<void **>(&h->d_kidx), kidx.data(), kidx.size() * sizeof(int));
-  up(reinterpret_cast<void **>(&h->d_kptr), kptr.data(), kptr.size() * sizeof(int));
-  up(reinterpret_cast<void **>(&h->d_kb_ent), ent.data(), ent.size() * sizeof(int4));
-  up(reinterpret_cast<void **>(&h->d_kblk), blk.data(), blk.size() * sizeof(int4));
-  up(reinterpret_cast<void **>(&h->d_brow), brow.data(), brow.size() * sizeof(int2));
-  up(reinterpret_cast<void **>(&h->d_pk), pk.data(), pk.size() * sizeof(double));
-  up(reinterpret_cast<void **>(&h->d_pk_f), pkf.data(), pkf.size() * sizeof(float));
+  auto up = [&](auto **dp, const void *src, size_t n) {
+    parts.push_back({reinterpret_cast<void **>(dp), src, n * sizeof(**dp)});
+  };
+  up(&h->d_mat, mat.data(), mat.size());
+  up(&h->d_proj_row, prow.data(), prow.size());
+  up(&h->d_map, map, npts_tot);
+  up(&h->d_pt, pt.get(), nval);
+  up(&h->d_pt_f, nullptr, nval);
+  up(&h->d_scal, scal, nproj_tot);
+  up(&h->d_scal_f, scf.data(), scf.size());
+  up(&h->d_krows, R.krows.data(), nk);
+  up(&h->d_kidx, nullptr, m->np);
+  up(&h->d_kptr, R.kptr.data(), R.kptr.size());
+  up(&h->d_kb_ent, R.ent.data(), R.ent.size());
+  up(&h->d_kblk, R.blk.data(), nblk);
+  up(&h->d_brow, R.brow.data(), nblk ? nk : 0);
+  up(&h->d_pk, nullptr, npk);
+  up(&h->d_pk_f, nullptr, npk);
   size_t total = 0;
   for (const Part &q : parts) total += (q.bytes + 255) / 256 * 256;
   hpsi_status s = dev_alloc(&h->kb_tables, std::max<size_t>(total, 256));
@@ -970,9 +1001,22 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, c
     if (s) break;
     *q.dp = at;
     at += (q.bytes + 255) / 256 * 256;
-    const cudaError_t e = q.bytes ? cudaMemcpy(*q.dp, q.src, q.bytes, cudaMemcpyHostToDevice) : cudaSuccess;
+    const cudaError_t e =
+        q.bytes && q.src ? cudaMemcpy(*q.dp, q.src, q.bytes, cudaMemcpyHostToDevice) : cudaSuccess;
     if (e != cudaSuccess) {
       set_error(cudaGetErrorString(e));
+      s = HPSI_ERR_CUDA;
+    }
+  }
+  if (!s) {
+    cudaError_t e = cudaMemsetAsync(h->d_kidx, 0xff, size_t(m->np) * sizeof(int), nullptr);
+    kb_layout_kernel<<<4 * m->num_sms, 256>>>(h->d_pt, nval, h->d_krows, nk, h->d_kblk, nblk, h->d_brow, h->d_kb_ent,
+                                              h->d_pt_f, h->d_kidx, h->d_pk, h->d_pk_f);
+    g_launches++;
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // the set-up call returns with its tables in place
+    if (e != cudaSuccess) {
+      set_error(std::string("hpsi_hamiltonian_set_projectors: ") + cudaGetErrorString(e));
       s = HPSI_ERR_CUDA;
     }
   }
@@ -983,8 +1027,8 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, c
   h->nmat = nmat;
   h->nprojections = nproj_tot;
   h->max_nproj = maxp;
-  h->nk = int(krows.size());
-  h->nkblk = int(blk.size());
+  h->nk = nk;
+  h->nkblk = nblk;
   h->kb_nproj = double(nval) / double(std::max(1LL, npts_tot));
   h->min_npoints = minp;
   h->kb_npts = npts_tot;

@@ -611,7 +611,7 @@ static bool ket_blocks_better(const KetArgs &k) {
     return rows >= 28 && q >= (f64 || k.nst <= 64 ? 16 : 24);
   }
   if (k.nst > 32) return rows >= 20;
-  if (k.nst > 16) return rows >= 14;
+  if (k.nst > 16) return rows >= KET_BLOCK_ROWS;
   if (k.nst > 8) return rows >= (q >= 8 ? 20 : 28);
   return q >= 8 && rows >= (f64 ? 20 : 29);
 }

@@ -26,6 +26,10 @@ struct ProjArgs {
   const void *phase64 = nullptr;  // the same phases in FP64 (tensor-core path)
 };
 
+// Rows per block, on average, from which on the block form of the ket is ever the better
+// one (no blocks are made below).
+constexpr int KET_BLOCK_ROWS = 14;
+
 struct KetArgs {
   int nk;                // covered rows
   const int *krows;      // covered row -> mesh row

@@ -150,8 +150,8 @@ def test_group_of_unequal_spacings_and_phases(cuda, dtype, phases):
 @pytest.mark.parametrize("spheres", ["few", "many projectors", "many spheres"])
 def test_ket_widths(cuda, dtype, nst, phased, spheres):
     """Overlapping spheres of unequal projector counts: three (rows of one to three
-    matrices in well-filled blocks), three with 18 projectors on average, and forty
-    small ones (lists of a few rows each: one row at a time at every width)."""
+    matrices in well-filled blocks), three with 18 projectors on average whose points
+    come in any order, and forty small ones (lists of a few rows each: one row at a time at every width)."""
     import torch
     from hpsi.mesh import sphere_mesh
     rng = np.random.default_rng(31)
@@ -168,6 +168,8 @@ def test_ket_widths(cuda, dtype, nst, phased, spheres):
     P.maps, P.mats, P.scals = [], [], []
     for c, r, q in atoms:
         sel = np.nonzero(np.sum((x - np.array(c)) ** 2, axis=1) <= r * r)[0].astype(np.int32)
+        if spheres == "many projectors":  # any order of the points, some of them twice
+            sel = rng.permutation(np.concatenate([sel, sel[:5]]))
         P.maps.append(sel)
         P.mats.append(rng.standard_normal((len(sel), q)))
         P.scals.append(rng.uniform(-1, 1, q) * m.vol_pp)
