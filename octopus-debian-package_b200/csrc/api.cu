@@ -1113,29 +1113,46 @@ int choose_zb(const hpsi_mesh *m, int chunks) { return choose_zb(m, chunks, 16);
 static double pass_makespan(const hpsi_mesh *m, int ty, int zb, int chunks, int slots, double extra) {
   const auto &tz = ty == 8 ? m->tile_z8 : m->tile_z;
   const int tyn = ty == 8 ? m->tiles_y8 : m->tiles_y;
-  std::vector<int4> u;  // {band, tile x, tile y, planes}
-  for (int by = 0; by < tyn; ++by)
-    for (int bx = 0; bx < m->tiles_x; ++bx) {
+  struct Column {
+    int band, blocks, planes;  // first z band, its blocks, its planes
+  };
+  std::vector<Column> cols;
+  cols.reserve(tz.size());
+  int band0 = 1 << 30, band1 = 0, tall = 0;
+  for (int bx = 0; bx < m->tiles_x; ++bx)
+    for (int by = 0; by < tyn; ++by) {
       const int2 t = tz[size_t(by) * m->tiles_x + bx];
       if (t.y < 0) continue;
-      for (int z = t.x; z <= t.y; z += zb) u.push_back(make_int4(z / zb, bx, by, std::min(zb, t.y + 1 - z)));
+      const int planes = t.y - t.x + 1, blocks = (planes + zb - 1) / zb;
+      cols.push_back({t.x / zb, blocks, planes});
+      band0 = std::min(band0, t.x / zb);
+      band1 = std::max(band1, t.x / zb + blocks);
+      tall = std::max(tall, planes);
     }
-  std::stable_sort(u.begin(), u.end(), [](const int4 &a, const int4 &b) {
-    if (a.x != b.x) return a.x < b.x;
-    if (a.y != b.y) return a.y < b.y;
-    return a.z < b.z;
-  });
-  std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
-  for (int i = 0; i < std::max(1, slots); ++i) free_at.push(0.0);
-  double end = 0.0;
-  for (const int4 &w : u)
-    for (int c = 0; c < chunks; ++c) {
-      const double t = free_at.top() + double(w.w) + extra;
-      free_at.pop();
-      free_at.push(t);
-      end = std::max(end, t);
+  // slots by the time they come free, in half plane steps (extra is a multiple of
+  // a half): a unit's cost is bounded, so a ring of counters holds them all
+  const int e2 = int(2 * extra), ring = 2 * std::min(zb, tall) + e2 + 1;
+  std::vector<int> free_at(ring, 0);
+  free_at[0] = std::max(1, slots);
+  int now = 0, at = 0, end = 0;
+  for (int band = band0; band < band1; ++band)
+    for (const Column &c : cols) {
+      const int i = band - c.band;
+      if (i < 0 || i >= c.blocks) continue;
+      const int cost = 2 * std::min(zb, c.planes - i * zb) + e2;
+      for (int left = chunks; left > 0;) {
+        while (free_at[at] == 0) {
+          ++now;
+          at = at + 1 == ring ? 0 : at + 1;
+        }
+        const int n = std::min(left, free_at[at]);
+        free_at[at] -= n;
+        free_at[at + cost >= ring ? at + cost - ring : at + cost] += n;
+        left -= n;
+      }
+      end = std::max(end, now + cost);
     }
-  return end;
+  return 0.5 * end;
 }
 
 // z block depth of a single-system pass over 16 x 8 tiles (the blocked pass,
