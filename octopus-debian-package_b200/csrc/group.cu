@@ -28,6 +28,7 @@ namespace hpsi {
 
 PassShape pass_shape(const hpsi_hamiltonian *h, int dtype, long long ld);
 PassShape tmem_shape(int dtype);
+PassShape legacy_shape(int dtype, long long ld);
 int pass_chunks(const PassShape &s, long long ld);
 PassShape default_shape(int dtype, long long ld);
 int pass_sc(int dtype, long long ld);
@@ -103,12 +104,15 @@ static void group_free_units(hpsi_group *g) {
 // units consecutive in the list.  The z block depth is the common number of
 // blocks per tile column with the shortest such schedule (a unit costs its
 // output planes + TMEM_UNIT_EXTRA).
-static hpsi_status group_build_tmem(hpsi_group *g, int dtype, const std::vector<long long> &ld, long long sig) {
+// forced_zb: block depth of an override, or 0.
+static hpsi_status group_build_tmem(hpsi_group *g, int dtype, const std::vector<long long> &ld, long long sig,
+                                    int forced_zb) {
   const int n = int(g->hams.size());
   const PassShape shape = tmem_shape(dtype);
   g->blk = false;
   g->sc = shape.sc;
   auto depth = [&](int s, int blocks) {
+    if (forced_zb > 0) return forced_zb;
     int tall = 1;
     for (auto &t : g->hams[s]->mesh->tile_z)
       if (t.y >= 0) tall = std::max(tall, t.y - t.x + 1);
@@ -201,11 +205,32 @@ static hpsi_status group_build(hpsi_group *g, int dtype, const std::vector<long 
   group_free_units(g);
   const int n = int(g->hams.size());
   g->shapes.assign(n, PassShape{});
-  // the tensor-memory pass takes any width of 16-byte rows; the shape overrides
-  // keep the forms below
-  g->tmem = !std::getenv(dtype == HPSI_C128 ? "HPSI_PASS_SHAPE64" : "HPSI_PASS_SHAPE32");
-  for (int s = 0; s < n; ++s) g->tmem = g->tmem && (dtype == HPSI_C128 || ld[s] % 2 == 0);
-  if (g->tmem) return group_build_tmem(g, dtype, ld, sig);
+  // the tensor-memory pass takes any width of 16-byte rows, but for batches of at
+  // most a quarter of its chunk on many points in all, where it would work on empty
+  // lanes (see pass_shape).  One Taylor step of equal boxes, us, one-complex pass /
+  // tensor-memory pass:
+  //   width (FP64)       1           2           3           4
+  //   16 x 20^3      151 / 169   166 / 169   257 / 170   219 / 170
+  //   6 x 48^3       245 / 288   279 / 290   453 / 300   396 / 307
+  //   4 x 64^3       252 / 361   281 / 372   651 / 384   403 / 389
+  //   3 x 100^3      731 / 1005  853 / 1014 1847 / 1034 1218 / 1034
+  // (FP32 alike at twice the widths.)  A shape override that names it takes it at
+  // its z depth; the others keep the forms below.
+  const bool forced = std::getenv(dtype == HPSI_C128 ? "HPSI_PASS_SHAPE64" : "HPSI_PASS_SHAPE32") != nullptr;
+  long long points = 0;
+  bool rows16 = true, narrow = true, named = forced;
+  int zb = 0;
+  for (int s = 0; s < n; ++s) {
+    points += g->hams[s]->mesh->np;
+    rows16 = rows16 && (dtype == HPSI_C128 || ld[s] % 2 == 0);
+    narrow = narrow && 4 * ld[s] <= tmem_shape(dtype).sc;
+    if (!forced) continue;
+    const PassShape sh = default_shape(dtype, ld[s]);
+    named = named && sh.tmem;
+    zb = sh.zb;
+  }
+  g->tmem = rows16 && (forced ? named : !(narrow && points > 500000));
+  if (g->tmem) return group_build_tmem(g, dtype, ld, sig, zb);
   // the blocked pass when every width is a multiple of its chunk
   const PassShape bs = blk_shape(dtype);
   g->blk = true;
@@ -215,7 +240,8 @@ static hpsi_status group_build(hpsi_group *g, int dtype, const std::vector<long 
     for (int s = 0; s < n; ++s)
       if (!g->shapes[s].blk || g->shapes[s].rx != g->shapes[0].rx || g->shapes[s].ry != g->shapes[0].ry ||
           g->shapes[s].cplx != g->shapes[0].cplx || g->shapes[s].unroll != g->shapes[0].unroll ||
-          g->shapes[s].tmem != g->shapes[0].tmem || g->shapes[s].sc != g->shapes[0].sc || g->shapes[s].ty != g->shapes[0].ty || ld[s] % g->shapes[s].sc) {
+          g->shapes[s].tmem || g->shapes[s].sc != g->shapes[0].sc || g->shapes[s].ty != g->shapes[0].ty ||
+          ld[s] % g->shapes[s].sc) {
         g->blk = false;
         break;
       }
@@ -223,7 +249,7 @@ static hpsi_status group_build(hpsi_group *g, int dtype, const std::vector<long 
   // common state chunk: the smallest preferred chunk over the systems
   int sc = g->blk ? g->shapes[0].sc : (dtype == HPSI_C128 ? 4 : 8);
   for (int s = 0; s < n && !g->blk; ++s) {
-    PassShape sh = pass_shape(g->hams[s], dtype, ld[s]);
+    PassShape sh = narrow ? legacy_shape(dtype, ld[s]) : pass_shape(g->hams[s], dtype, ld[s]);
     sc = std::min(sc, sh.blk ? (dtype == HPSI_C128 ? 4 : 8) : sh.sc);
     g->shapes[s] = sh;
   }

@@ -68,10 +68,24 @@ def test_autotune_keeps_results(cuda):
     assert shape32["sc"] in (2, 4, 8)
 
 
+# shape overrides of the grouped launch: the blocked pass, the tensor-memory pass with
+# z blocks of five planes
+FORMS = {"default": None,
+         "blocked": {"c128": "8,2,0,9,1,2,0,8", "c64": "16,2,0,9,1,2,1,8"},
+         "tensor memory": {"c128": "8,2,5,9,1,2,0,8,0,0,0,1", "c64": "16,2,5,9,1,2,1,8,0,0,0,1"}}
+
+
+def _force(monkeypatch, form, dtype):
+    if FORMS[form]:
+        monkeypatch.setenv({"c128": "HPSI_PASS_SHAPE64", "c64": "HPSI_PASS_SHAPE32"}[dtype], FORMS[form][dtype])
+
+
+@pytest.mark.parametrize("form", list(FORMS))
 @pytest.mark.parametrize("dtype", ["c128", "c64"])
-def test_group_blocked_pass_matches_single_systems(cuda, dtype):
+def test_group_blocked_pass_matches_single_systems(cuda, dtype, form, monkeypatch):
     """Every width a multiple of the blocked pass's chunk (8 complex128 / 16
-    complex64 states): the grouped launch runs the blocked pass kernel."""
+    complex64 states): the grouped launch of each form (without a field: the blocked
+    pass in its field-free form) against single systems in the default one."""
     import torch
     from hpsi import lib
     from hpsi.stencil import laplacian_weights, star_points
@@ -93,6 +107,7 @@ def test_group_blocked_pass_matches_single_systems(cuda, dtype):
         xs.append(x)
         refs.append(r)
         nsts.append(nst)
+    _force(monkeypatch, form, dtype)
     g = lib.Group([h for _, h in hams])
     tol = 1e-13 if dtype == "c128" else 1e-6
     for graph in (False, True):
@@ -106,11 +121,11 @@ def test_group_blocked_pass_matches_single_systems(cuda, dtype):
     g.close()
 
 
+@pytest.mark.parametrize("form", list(FORMS))
 @pytest.mark.parametrize("dtype", ["c128", "c64"])
-def test_group_with_laser_field_matches_single_systems(cuda, dtype):
-    """Systems with a laser field in the group (the persistent pass with the
-    field term; without a field in any system it takes the field-free form):
-    each system as its own Taylor steps with the same field."""
+def test_group_with_laser_field_matches_single_systems(cuda, dtype, form, monkeypatch):
+    """Systems with a laser field in the group (the blocked pass with the field
+    term): each system as its own Taylor steps with the same field."""
     import torch
     from hpsi import lib
     from hpsi.stencil import laplacian_weights, star_points
@@ -133,6 +148,7 @@ def test_group_with_laser_field_matches_single_systems(cuda, dtype):
         hams.append((dm, ham))
         xs.append(x)
         refs.append(r)
+    _force(monkeypatch, form, dtype)
     g = lib.Group([h for _, h in hams])
     tol = 1e-13 if dtype == "c128" else 1e-6
     ys = [x.clone() for x in xs]
@@ -143,3 +159,31 @@ def test_group_with_laser_field_matches_single_systems(cuda, dtype):
         b = r.cpu().numpy().astype(np.complex128)
         assert rel_maxnorm_per_state(a, b) <= tol
     g.close()
+
+
+@pytest.mark.parametrize("dtype,widths", [("c128", (1, 2, 1)), ("c128", (2, 2, 2)), ("c128", (1, 3, 2)),
+                                          ("c64", (2, 4, 2)), ("c64", (4, 4, 4)), ("c64", (2, 6, 4))])
+def test_group_of_narrow_batches(cuda, dtype, widths):
+    """More than 500,000 points in all: batches of at most a quarter of the chunk in the
+    one-complex pass, with one wider batch among them in the tensor-memory pass."""
+    import torch
+    from hpsi import lib
+    from hpsi.mesh import index_box_mesh
+    from hpsi.stencil import laplacian_weights, star_points
+    tdt = torch.complex128 if dtype == "c128" else torch.complex64
+    gen = torch.Generator(device=cuda).manual_seed(4)
+    hams, xs = [], []
+    for i, ld in enumerate(widths):
+        m = index_box_mesh((56, 57 + i, 55), 0.3)
+        v = np.random.default_rng(i).uniform(-1, 0, m.np)
+        hams.append(lib.Hamiltonian(lib.DeviceMesh(m), laplacian_weights(m.spacing), star_points(), v=v))
+        xs.append(torch.randn((m.np_part, ld), dtype=tdt, device=cuda, generator=gen))
+    single = [x.clone() for x in xs]
+    for H, x in zip(hams, single):
+        for _ in range(2):
+            H.taylor_step(x, 0.004)
+    ys = [x.clone() for x in xs]
+    lib.Group(hams).taylor_steps(ys, 2, 0.004)
+    for H, y, x in zip(hams, ys, single):
+        n = H.dmesh.mesh.np
+        assert (y - x)[:n].abs().max().item() <= (1e-13 if dtype == "c128" else 1e-6) * x[:n].abs().max().item()
