@@ -238,32 +238,16 @@ PassShape legacy_shape(int dtype, long long ld) {
   return dtype == HPSI_C128 ? PassShape{sc, 16, 16, 2} : PassShape{sc, 16, 16, 4};
 }
 
-// Shape of the register-blocked pass (one real lane per thread, 16 x 8 tiles).
+// Shape of the register-blocked pass (16 x 8 tiles), a candidate of the autotuner:
+// FP64 2 x 2 cells of one real lane, FP32 2 x 2 cells of one complex state with
+// packed multiply-adds (512 threads).
 PassShape blk_shape(int dtype) {
-  // measured on the R = 12 bohr sphere (128 states): FP64 2 x 2 cells of one
-  // real lane (512 threads); FP32 2 x 2 cells of one complex state with
-  // packed multiply-adds (512 threads)
   PassShape s = dtype == HPSI_C128 ? PassShape{blk_chunk_states<double>(), 16, 8, 2}
                                    : PassShape{blk_chunk_states<float>(), 16, 8, 2};
   s.blk = 1;
   s.rx = 2;
   s.cplx = dtype == HPSI_C128 ? 0 : 1;
   s.unroll = 9;  // planes per unrolled group of the z march (9: no rotation)
-  return s;
-}
-
-// Register-blocked pass over half chunks (64 bytes: FP64 4 states, FP32 8),
-// 16 x 8 tiles, 1 x 4 cells, 256 threads and two CTAs per SM: the default
-// for widths that are a multiple of the half chunk but not of the chunk.
-// Measured on the R = 12 sphere against the one-complex pass: FP32 8 / 24 /
-// 40 states 0.144 / 0.302 / 0.414 -> 0.111 / 0.208 / 0.326 ms, FP64 4 / 12 /
-// 20 states 0.133 / 0.284 / 0.384 -> 0.106 / 0.201 / 0.323 ms.
-PassShape half_chunk_shape(int dtype) {
-  PassShape s = blk_shape(dtype);
-  s.sc /= 2;
-  s.ty = 8;
-  s.rx = 1;
-  s.ry = 4;
   return s;
 }
 
@@ -280,44 +264,39 @@ PassShape tmem_shape(int dtype) {
 // State chunks of a pass over ld states.
 int pass_chunks(const PassShape &s, long long ld) { return int((ld + s.sc - 1) / s.sc); }
 
-PassShape default_shape(int dtype, long long ld) {
-  const PassShape b = blk_shape(dtype);
-  PassShape s = ld % b.sc == 0         ? b
-                : ld % (b.sc / 2) == 0 ? half_chunk_shape(dtype)
-                                       : legacy_shape(dtype, ld);
-  // experiment override: HPSI_PASS_SHAPE64 / HPSI_PASS_SHAPE32 = "sc,ry,zb,unroll,blk,rx,cplx,ty,tma,mb,mma,tmem"
+// Experiment override: HPSI_PASS_SHAPE64 / HPSI_PASS_SHAPE32 =
+// "sc,ry,zb,unroll,blk,rx,cplx,ty,tma,0,mma,tmem".  False where none is set or the
+// one set does not serve this width.
+bool forced_shape(int dtype, long long ld, PassShape &s) {
   const char *env = std::getenv(dtype == HPSI_C128 ? "HPSI_PASS_SHAPE64" : "HPSI_PASS_SHAPE32");
-  if (env) {
-    int a = 0, b = 0, c = 0, u = 0, t = 0, x = 0, cx = -1, ty = 0, tm = 0, mb = 0, mm = 0, tn = 0;
-    if (std::sscanf(env, "%d,%d,%d,%d,%d,%d,%d,%d,%d,%d,%d,%d", &a, &b, &c, &u, &t, &x, &cx, &ty, &tm, &mb, &mm,
-                    &tn) >= 2 &&
-        a > 0 &&
-        (ld % a == 0 || (t && tn))) {
-      if (t && (tn || tm || mb)) {
-        // tensor-memory pass (its stages are handed over by mbarriers; tma: box
-        // copies of contiguous halo runs)
-        s = tmem_shape(dtype);
-        s.tma = tm ? 1 : 0;
-      } else if (t) {
-        s = blk_shape(dtype);  // chunk (128 or 64 bytes), block, element, z depth and group are taken
-        if (a == s.sc / 2) {
-          s.sc = a;  // 64-byte chunks ride 16 x 16 tiles unless ty = 8 is given
-          s.ty = ty == 8 ? 8 : 16;
-        }
-        if (u == 1 || u == 3 || u == 9) s.unroll = u;
-        if (x > 0) s.rx = x;
-        if (b > 0) s.ry = b;
-        if (cx >= 0) s.cplx = cx;
-        s.mma = mm ? 1 : 0;
-      } else {
-        s = legacy_shape(dtype, ld);
-        s.sc = a;
-        s.ry = b;
-      }
-      s.zb = c;
+  if (!env) return false;
+  int a = 0, b = 0, c = 0, u = 0, t = 0, x = 0, cx = -1, ty = 0, tm = 0, unused = 0, mm = 0, tn = 0;
+  if (std::sscanf(env, "%d,%d,%d,%d,%d,%d,%d,%d,%d,%d,%d,%d", &a, &b, &c, &u, &t, &x, &cx, &ty, &tm, &unused, &mm,
+                  &tn) < 2 ||
+      a <= 0 || unused || (ld % a != 0 && !(t && tn)))
+    return false;
+  if (t && (tn || tm)) {
+    // tensor-memory pass (tma: box copies of contiguous halo runs)
+    s = tmem_shape(dtype);
+    s.tma = tm ? 1 : 0;
+  } else if (t) {
+    s = blk_shape(dtype);  // chunk (128 or 64 bytes), block, element, z depth and group are taken
+    if (a == s.sc / 2) {
+      s.sc = a;  // 64-byte chunks ride 16 x 16 tiles unless ty = 8 is given
+      s.ty = ty == 8 ? 8 : 16;
     }
+    if (u == 1 || u == 3 || u == 9) s.unroll = u;
+    if (x > 0) s.rx = x;
+    if (b > 0) s.ry = b;
+    if (cx >= 0) s.cplx = cx;
+    s.mma = mm ? 1 : 0;
+  } else {
+    s = legacy_shape(dtype, ld);
+    s.sc = a;
+    s.ry = b;
   }
-  return s;
+  s.zb = c;
+  return true;
 }
 
 }  // namespace hpsi
@@ -1501,13 +1480,14 @@ hpsi_status run_ket(hpsi_hamiltonian *h, const T *proj, long long ld, int nst, T
 // (FP32 alike at twice the widths; below 48^3 points the tensor-memory pass takes
 // 16-17 us, the others 24-37.)
 PassShape pass_shape(const hpsi_hamiltonian *h, int dtype, long long ld) {
+  PassShape s;
+  if (forced_shape(dtype, ld, s)) return s;
   const auto &t = h->tuned[dtype == HPSI_C128 ? 0 : 1];
-  if (std::getenv(dtype == HPSI_C128 ? "HPSI_PASS_SHAPE64" : "HPSI_PASS_SHAPE32")) return default_shape(dtype, ld);
   if (t.ld == ld) return t.shape;
-  const PassShape s = tmem_shape(dtype);
+  s = tmem_shape(dtype);
   const bool rows16 = dtype == HPSI_C128 || ld % 2 == 0;
   const bool narrow = 4 * ld <= s.sc && h->mesh->np > 200000;
-  return rows16 && !narrow ? s : default_shape(dtype, ld);
+  return rows16 && !narrow ? s : legacy_shape(dtype, ld);
 }
 
 // Arguments of one fused pass (no launch).  in: rows to stencil; out: result

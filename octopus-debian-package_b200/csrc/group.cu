@@ -30,7 +30,7 @@ PassShape pass_shape(const hpsi_hamiltonian *h, int dtype, long long ld);
 PassShape tmem_shape(int dtype);
 PassShape legacy_shape(int dtype, long long ld);
 int pass_chunks(const PassShape &s, long long ld);
-PassShape default_shape(int dtype, long long ld);
+bool forced_shape(int dtype, long long ld, PassShape &s);
 int pass_sc(int dtype, long long ld);
 int choose_zb(const hpsi_mesh *m, int chunks, int ty);
 hpsi_status mesh_items(hpsi_mesh *m, int zb, int ty, const int4 **items, int *nitems);
@@ -216,27 +216,25 @@ static hpsi_status group_build(hpsi_group *g, int dtype, const std::vector<long 
   //   3 x 100^3      731 / 1005  853 / 1014 1847 / 1034 1218 / 1034
   // (FP32 alike at twice the widths.)  A shape override that names it takes it at
   // its z depth; the others keep the forms below.
-  const bool forced = std::getenv(dtype == HPSI_C128 ? "HPSI_PASS_SHAPE64" : "HPSI_PASS_SHAPE32") != nullptr;
   long long points = 0;
-  bool rows16 = true, narrow = true, named = forced;
+  bool rows16 = true, narrow = true, forced = true, named = true;
   int zb = 0;
   for (int s = 0; s < n; ++s) {
     points += g->hams[s]->mesh->np;
     rows16 = rows16 && (dtype == HPSI_C128 || ld[s] % 2 == 0);
     narrow = narrow && 4 * ld[s] <= tmem_shape(dtype).sc;
-    if (!forced) continue;
-    const PassShape sh = default_shape(dtype, ld[s]);
+    PassShape sh;
+    forced = forced && forced_shape(dtype, ld[s], sh);
     named = named && sh.tmem;
-    zb = sh.zb;
+    if (forced) zb = sh.zb;
   }
   g->tmem = rows16 && (forced ? named : !(narrow && points > 500000));
   if (g->tmem) return group_build_tmem(g, dtype, ld, sig, zb);
-  // the blocked pass when every width is a multiple of its chunk
-  const PassShape bs = blk_shape(dtype);
-  g->blk = true;
-  for (int s = 0; s < n; ++s) g->blk = g->blk && ld[s] % bs.sc == 0;
+  // the blocked pass where an override names it and every width is a multiple of its chunk
+  g->blk = forced;
+  for (int s = 0; s < n; ++s) g->blk = g->blk && ld[s] % blk_shape(dtype).sc == 0;
   if (g->blk) {
-    for (int s = 0; s < n; ++s) g->shapes[s] = default_shape(dtype, ld[s]);
+    for (int s = 0; s < n; ++s) forced_shape(dtype, ld[s], g->shapes[s]);
     for (int s = 0; s < n; ++s)
       if (!g->shapes[s].blk || g->shapes[s].rx != g->shapes[0].rx || g->shapes[s].ry != g->shapes[0].ry ||
           g->shapes[s].cplx != g->shapes[0].cplx || g->shapes[s].unroll != g->shapes[0].unroll ||
@@ -540,7 +538,7 @@ static hpsi_status autotune_t(hpsi_hamiltonian *h, int dtype, long long ld, cuda
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   double best = 1e30;
-  PassShape best_shape = default_shape(dtype, ld);
+  PassShape best_shape = legacy_shape(dtype, ld);
   for (const auto &sh0 : cands) {
     PassArgs a;
     PassShape sh = sh0;

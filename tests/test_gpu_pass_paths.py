@@ -1,12 +1,12 @@
 """GPU parity of both stencil-pass kernels against the FP64 CPU oracle.
 
-The register-blocked pass (one real lane per thread, 16 x 8 tiles) serves
-batches whose width is a multiple of its state chunk (8 complex states FP64,
-16 FP32); its half-chunk form (64 bytes: 4 FP64, 8 FP32 states, two CTAs per
-SM) serves widths that are a multiple of half a chunk only (FP64 12, FP32 24
-below); the one-complex-per-thread pass serves the rest.  The kernels are
-forced here through the shape override and compared with the oracle and with
-each other: FP64 to 1e-12 relative max-norm per state, FP32 storage to 2e-5.
+The tensor-memory pass is the default; narrow batches on large meshes take the
+one-complex-per-thread pass ("legacy").  The register-blocked pass (16 x 8 tiles;
+widths that are a multiple of its chunk of 8 FP64 or 16 FP32 states, or of half
+of it) is a candidate of the autotuner.  The kernels are forced here through the
+shape override (a width that an override does not serve runs the default) and
+compared with the oracle and with each other: FP64 to 1e-12 relative max-norm
+per state, FP32 storage to 2e-5.
 """
 import numpy as np
 import pytest
@@ -19,14 +19,16 @@ TOL64 = 1e-12
 TOL32 = 2e-5
 
 LEGACY = {"HPSI_PASS_SHAPE64": "4,2,0,0,0", "HPSI_PASS_SHAPE32": "8,4,0,0,0"}
-# blocked pass: "chunk,ry,zb,group,1,rx,complex"
+# blocked pass: "chunk,ry,zb,group,1,rx,complex,ty"
+# (groups of nine planes, the shapes that also come without the laser term)
+BLK_9 = {"HPSI_PASS_SHAPE64": "8,2,{zb},9,1,2,0,8", "HPSI_PASS_SHAPE32": "16,2,{zb},9,1,2,1,8"}
 BLK_REAL = {"HPSI_PASS_SHAPE64": "8,2,{zb},3,1,2,0", "HPSI_PASS_SHAPE32": "16,4,{zb},1,1,2,0"}
 BLK_CPLX = {"HPSI_PASS_SHAPE64": "8,2,{zb},9,1,2,1", "HPSI_PASS_SHAPE32": "16,2,{zb},3,1,2,1"}
 # 64-byte chunks on 16 x 16 tiles, 1 x 4 cells
 BLK_64B = {"HPSI_PASS_SHAPE64": "4,4,{zb},9,1,1,0", "HPSI_PASS_SHAPE32": "8,4,{zb},9,1,1,1"}
 # 64-byte chunks on 16 x 8 tiles, 1 x 4 cells, 256 threads (two CTAs per SM)
 BLK_2CTA = {"HPSI_PASS_SHAPE64": "4,4,{zb},9,1,1,0,8", "HPSI_PASS_SHAPE32": "8,4,{zb},9,1,1,1,8"}
-PATHS = ["default", "blk_real", "blk_cplx", "blk_64b", "blk_2cta", "legacy"]
+PATHS = ["default", "blk_9", "blk_real", "blk_cplx", "blk_64b", "blk_2cta", "legacy"]
 
 
 def _setup(mesh, v=None, proj=None):
@@ -57,7 +59,7 @@ def _set_path(monkeypatch, path, zb=0):
         for k in LEGACY:
             monkeypatch.delenv(k, raising=False)
         return
-    env = {"legacy": LEGACY, "blk_real": BLK_REAL, "blk_cplx": BLK_CPLX, "blk_64b": BLK_64B,
+    env = {"legacy": LEGACY, "blk_9": BLK_9, "blk_real": BLK_REAL, "blk_cplx": BLK_CPLX, "blk_64b": BLK_64B,
            "blk_2cta": BLK_2CTA}[path]
     for k, v in env.items():
         monkeypatch.setenv(k, v.format(zb=zb))
@@ -91,7 +93,7 @@ def test_apply_and_taylor(cuda, monkeypatch, path, dtype, ld, nst):
     assert np.max(np.abs(n - n_ref) / n_ref) <= (1e-12 if dtype == np.complex128 else 1e-6)
 
 
-@pytest.mark.parametrize("path", ["blk_real", "blk_cplx", "blk_64b", "blk_2cta"])
+@pytest.mark.parametrize("path", ["blk_9", "blk_real", "blk_cplx", "blk_64b", "blk_2cta"])
 @pytest.mark.parametrize("zb", [0, 5, 9])
 def test_blk_zblocks_and_tiles(cuda, monkeypatch, zb, path):
     """A box several tiles wide in x and y, cut into z blocks of several depths
@@ -112,7 +114,7 @@ def test_blk_zblocks_and_tiles(cuda, monkeypatch, zb, path):
     assert rel_maxnorm_per_state(y.cpu().numpy(), ref) <= TOL64
 
 
-@pytest.mark.parametrize("path", ["blk_real", "blk_cplx", "blk_64b", "blk_2cta"])
+@pytest.mark.parametrize("path", ["blk_9", "blk_real", "blk_cplx", "blk_64b", "blk_2cta"])
 def test_blk_periodic_and_raw_boundary(cuda, monkeypatch, path):
     """Periodic images without Bloch phase (map to inner rows) and set_bc=False
     (boundary rows read as stored: the input tensor spans np_part rows)."""
@@ -207,7 +209,7 @@ def test_odd_fp32_width_rejected(cuda):
         ham.apply(x, y)
 
 
-@pytest.mark.parametrize("path", ["default", "blk_real", "blk_cplx", "blk_64b", "blk_2cta"])
+@pytest.mark.parametrize("path", ["default", "blk_9", "blk_real", "blk_cplx", "blk_64b", "blk_2cta"])
 @pytest.mark.parametrize("dtype,ld", [(np.complex128, 8), (np.complex64, 16)])
 def test_blk_bloch_phase(cuda, monkeypatch, path, dtype, ld):
     """Bloch-phase periodic images (phase multiplied on load) in the blocked pass."""
@@ -230,3 +232,24 @@ def test_blk_bloch_phase(cuda, monkeypatch, path, dtype, ld):
     ham.apply(x, y)
     tol = TOL64 if dtype == np.complex128 else TOL32
     assert rel_maxnorm_per_state(y.cpu().numpy().astype(np.complex128), ref) <= tol
+
+
+@pytest.mark.parametrize("path", ["blk_9", "blk_real", "blk_cplx", "blk_64b", "blk_2cta", "legacy"])
+@pytest.mark.parametrize("dtype,ld", [(np.complex128, 8), (np.complex64, 16)])
+def test_paths_with_a_field(cuda, monkeypatch, path, dtype, ld):
+    """The laser term of every forced pass: apply and a Taylor step with E pol.r in the
+    potential of the oracle."""
+    _set_path(monkeypatch, path)
+    m, v, proj, psi = small_sphere_system(seed=71, nst=ld, radius=3.9, natoms=2)
+    dm, ham, w, pts = _setup(m, v=v, proj=proj)
+    pol, amp = np.array([0.3, -0.5, 0.8]), 0.07
+    ham.set_field(pol, amp)
+    o = _oracle(m, w, pts, v=v + amp * (m.x[: m.np] @ pol), proj=proj)
+    x = _dev(psi, cuda, ld, dtype)
+    import torch
+    y = torch.zeros((m.np, ld), dtype=x.dtype, device=cuda)
+    ham.apply(x, y)
+    tol = TOL64 if dtype == np.complex128 else TOL32
+    assert rel_maxnorm_per_state(y.cpu().numpy().astype(np.complex128), o.apply(psi)) <= tol
+    ham.taylor_step(x, 0.02)
+    assert rel_maxnorm_per_state(x.cpu().numpy()[: m.np].astype(np.complex128), o.taylor(psi, 0.02, order=4)) <= tol

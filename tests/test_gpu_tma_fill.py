@@ -1,12 +1,8 @@
-"""Variants of the blocked stencil pass that move the same data by other
-means, checked bit for bit against the default (per-thread cp.async fill, one
-barrier per plane):
-
-* TMA fill: runs of eight consecutive batch rows in a halo row arrive as one
-  cp.async.bulk.tensor box (8 rows x 128 bytes) completing on the stage's
-  mbarrier; the other halo cells keep their per-thread copies;
-* mbarrier hand-over: the per-thread fill, with each stage handed over by a
-  full and an empty mbarrier (cp.async arrive-on) instead of the barrier.
+"""TMA fill of the tensor-memory pass, checked bit for bit against its default
+per-thread copies: runs of eight consecutive batch rows in a halo row over the
+tile's columns arrive as one cp.async.bulk.tensor box (8 rows x 128 bytes)
+completing on the stage's mbarrier; the other halo cells keep their per-thread
+copies.
 
 The same values land in shared memory and are summed in the same order, so
 H psi, a Taylor step (with and without the observables of its first pass)
@@ -22,12 +18,10 @@ pytestmark = pytest.mark.gpu
 
 SHAPES = {
     "tma": {"c128": ("HPSI_PASS_SHAPE64", "8,2,0,9,1,2,0,8,1"), "c64": ("HPSI_PASS_SHAPE32", "16,2,0,9,1,2,1,8,1")},
-    "mbar": {"c128": ("HPSI_PASS_SHAPE64", "8,2,0,9,1,2,0,8,0,1"),
-             "c64": ("HPSI_PASS_SHAPE32", "16,2,0,9,1,2,1,8,0,1")},
 }
 
 
-@pytest.mark.parametrize("variant", ["tma", "mbar"])
+@pytest.mark.parametrize("variant", ["tma"])
 @pytest.mark.parametrize("dtype,nst", [("c128", 16), ("c64", 32)])
 def test_fill_variant_equals_default_fill(cuda, dtype, nst, variant, monkeypatch):
     import torch
@@ -61,7 +55,7 @@ def test_fill_variant_equals_default_fill(cuda, dtype, nst, variant, monkeypatch
         assert np.array_equal(np.asarray(a), np.asarray(b))
 
 
-@pytest.mark.parametrize("variant", ["tma", "mbar"])
+@pytest.mark.parametrize("variant", ["tma"])
 def test_fill_variant_box_mesh_default_order(cuda, variant, monkeypatch):
     """A box mesh (long runs of consecutive rows in the blocked point order:
     most of the halo arrives by TMA) at a width of several state chunks."""
