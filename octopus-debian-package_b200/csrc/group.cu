@@ -482,8 +482,10 @@ static hpsi_status autotune_t(hpsi_hamiltonian *h, int dtype, long long ld, cuda
   std::vector<PassShape> cands;
   const int maxsc = dtype == HPSI_C128 ? 4 : 8;
   const int ry = dtype == HPSI_C128 ? 2 : 4;
-  for (int sc = maxsc; sc >= 1 && sc >= maxsc / 2; sc >>= 1) {
-    if (ld % sc) continue;
+  // one-complex pass: the widest state chunk that divides the width (narrow batches
+  // on large meshes run it by default), and its half
+  const int sc0 = pass_sc(dtype, ld);
+  for (int sc = sc0; sc == sc0 || (sc >= 1 && sc >= maxsc / 2); sc >>= 1) {
     for (int zb : {0, 16, 24, 32, 48, 64, 96, 1 << 20}) cands.push_back(PassShape{sc, 16, 16, ry, zb});
   }
   // blocked pass: the instantiated cell blocks x z block depths

@@ -187,3 +187,21 @@ def test_group_of_narrow_batches(cuda, dtype, widths):
     for H, y, x in zip(hams, ys, single):
         n = H.dmesh.mesh.np
         assert (y - x)[:n].abs().max().item() <= (1e-13 if dtype == "c128" else 1e-6) * x[:n].abs().max().item()
+
+
+def test_autotune_of_one_state_knows_the_one_complex_pass(cuda):
+    """One state on a large mesh: the one-complex pass (2 rows per thread) takes 2/3 of
+    the tensor-memory pass's time, which the autotuner must not choose instead."""
+    import torch
+    from hpsi import lib
+    from hpsi.mesh import index_box_mesh
+    from hpsi.stencil import laplacian_weights, star_points
+    m = index_box_mesh((96, 96, 96), 0.25)
+    H = lib.Hamiltonian(lib.DeviceMesh(m), laplacian_weights(m.spacing), star_points())
+    x = torch.randn((m.np_part, 1), dtype=torch.complex128, device=cuda)
+    y0, y1 = (torch.zeros((m.np, 1), dtype=torch.complex128, device=cuda) for _ in range(2))
+    H.apply(x, y0)
+    shape, _ = H.autotune(lib.HPSI_C128, 1)
+    assert shape["ry"] == 2 and shape["sc"] == 1
+    H.apply(x, y1)
+    assert (y1 - y0).abs().max().item() <= 1e-13 * y0.abs().max().item()
