@@ -600,6 +600,8 @@ hpsi_status launch_ket_blocks_w(const KetArgs &k, int rb, cudaStream_t st) {
 //   29.6 rows, 9 projectors, phases   25 / 24    47 / 32  103 / 130  21 / 19  37 / 29   70 / 91
 //   30.4 rows, 18 projectors, phases  26 / 26    71 / 37  168 / 152  23 / 18  55 / 33  108 / 106
 //   9.6 rows, 9 projectors, phases    45 / 136  121 / 185 281 / 607  35 / 92  90 / 160 210 / 526
+//   31.4 rows, 9 projectors, phases,
+//   8,779 rows in all                 13 / 12    16 / 12   27 / 22   13 / 12  15 / 12   24 / 19
 // The lines below lie between measured sides of 24 such sets (1 to 32 projectors, 9.6 to
 // 31.6 rows, 2 to 128 states).
 template <typename T>
@@ -607,8 +609,10 @@ static bool ket_blocks_better(const KetArgs &k) {
   const double rows = k.rows_per_block, q = k.nproj_per_point;
   const bool f64 = sizeof(T) == 8;
   if (k.phase) {
-    if (k.nst > 16 && k.nst <= 32) return rows >= 25;
-    return rows >= 28 && q >= (f64 || k.nst <= 64 ? 16 : 24);
+    if (k.nst > 32)  // (few rows do not fill the GPU one warp each)
+      return rows >= 28 && (q >= (f64 || k.nst <= 64 ? 16 : 24) || (q >= 8 && k.nk <= 16000));
+    if (k.nst > 16) return rows >= 25;
+    return rows >= 28 && (q >= 16 || (f64 && k.nst > 8 && q >= 8 && rows >= 29));
   }
   if (k.nst > 32) return rows >= 20;
   if (k.nst > 16) return rows >= KET_BLOCK_ROWS;
