@@ -115,21 +115,23 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
                : "d"(a), "d"(b));
 }
 
-// One complex state (16 bytes FP64, 8 FP32) to shared memory, zero where !ok.
+// One complex state (16 bytes FP64, 8 FP32; REALS: FP32 in two pieces of 4) to shared
+// memory, zero where !ok.
+template <bool REALS = false>
 __device__ __forceinline__ void copy_state(double *d, const double *g, bool ok) {
   const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(d));
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(g), "r"(ok ? 16 : 0));
 }
+template <bool REALS = false>
 __device__ __forceinline__ void copy_state(float *d, const float *g, bool ok) {
   const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(d));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(g), "r"(ok ? 8 : 0));
-}
-// The same in pieces of one real.
-__device__ __forceinline__ void copy_state_reals(float *d, const float *g, bool ok) {
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(d));
+  if constexpr (REALS) {
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s + 4 * i), "l"(g + i), "r"(ok ? 4 : 0));
+    for (int i = 0; i < 2; ++i)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s + 4 * i), "l"(g + i), "r"(ok ? 4 : 0));
+  } else {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(g), "r"(ok ? 8 : 0));
+  }
 }
 // Row pitch of a staged K x 64 block: the four K rows of a fragment read fall
 // into different bank groups (FP64 pitch = 4 mod 16, FP32 = 8 mod 32).
@@ -196,25 +198,18 @@ __global__ void __launch_bounds__(256) gram_kernel(const T *a, long long lda, co
         const long long row = p0 + (long long)k * GK + pp;
         const bool in = row < p1;
         const bool ua = in && u0 + l < n, vb = in && v0 + l < n;
-        auto copy = [](T *d, const T *g, bool ok) {
-          if constexpr (REALS)
-            copy_state_reals(d, g, ok);
-          else
-            copy_state(d, g, ok);
-        };
-        copy(sa + (s * GK + pp) * PITCH + l, ua ? a + row * 2 * lda + u0 + l : a, ua);
-        if (!same) copy(sb + (s * GK + pp) * PITCH + l, vb ? b + row * 2 * ldb + v0 + l : b, vb);
+        copy_state<REALS>(sa + (s * GK + pp) * PITCH + l, ua ? a + row * 2 * lda + u0 + l : a, ua);
+        if (!same) copy_state<REALS>(sb + (s * GK + pp) * PITCH + l, vb ? b + row * 2 * ldb + v0 + l : b, vb);
       }
     }
     cp_async_commit();
   };
-  double *o = partial + (long long)blockIdx.y * n * n;
   double c[2][4][2] = {};
   for (int k = 0; k < GST - 1; ++k) stage(k);
   for (int k = 0; k < nk; ++k) {
     if constexpr (FOLD) {
       if (k && k % GFOLD == 0) {
-        double *oc = o + (long long)gridDim.y * n * n;
+        double *o = partial + (long long)blockIdx.y * n * n, *oc = o + (long long)gridDim.y * n * n;
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -243,25 +238,28 @@ __global__ void __launch_bounds__(256) gram_kernel(const T *a, long long lda, co
     }
   }
   cp_async_wait<0>();
+  double *o = partial + (long long)blockIdx.y * n * n;
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int u = u0 + wu + 8 * i + (lane >> 2), v = v0 + wv + 8 * j + 2 * (lane & 3);
-      if (u >= n || v >= n) continue;
-      if constexpr (FOLD)
-        gram_fold(o, o + (long long)gridDim.y * n * n, (long long)u * n + v, nk <= GFOLD, c[i][j]);
-      else
-        *reinterpret_cast<double2 *>(o + (long long)u * n + v) = make_double2(c[i][j][0], c[i][j][1]);
+      if constexpr (FOLD) {
+        if (u < n && v < n)
+          gram_fold(o, o + (long long)gridDim.y * n * n, (long long)u * n + v, nk <= GFOLD, c[i][j]);
+      } else {
+        if (u < n && v < n) *reinterpret_cast<double2 *>(o + (long long)u * n + v) = make_double2(c[i][j][0], c[i][j][1]);
+      }
     }
 }
 
 // S[i][j] = dV * (conj(a_i) . b_j) from the real Gram G (n = 2 * nst); sym:
 // G holds the tiles on and above the diagonal, entries below it are conjugates.
 // block (32, 8): 8 slices of the splits per entry, folded in a fixed order.
-// rest: the partials' remainders follow them.
+// FOLD: the partials' remainders follow them.
+template <bool FOLD>
 __global__ void __launch_bounds__(256) gram_finalize(const double *partial, int splits, int nst, double dv, int sym,
-                                                     int rest, double *S) {
+                                                     double *S) {
   __shared__ double red[8][32][4];
   const int i = blockIdx.y, j = blockIdx.x * 32 + threadIdx.x;
   const int n = 2 * nst;
@@ -277,7 +275,7 @@ __global__ void __launch_bounds__(256) gram_finalize(const double *partial, int 
       kadd(re, g1.y);
       kadd(im, g0.y);
       kadd(im, -g1.x);
-      if (rest) {
+      if constexpr (FOLD) {
         const double2 *R0 = G0 + (long long)splits * n * nst;
         re.c += R0[0].x + R0[nst].y;
         im.c += R0[0].y - R0[nst].x;
@@ -666,7 +664,8 @@ hpsi_status launch_gram(const T *a, long long lda, const T *b, long long ldb, in
   }
   kern<<<dim3(unsigned(pairs), unsigned(splits)), 256, smem, st>>>(a, lda, b, ldb, np, n, tiles, sym, partial);
   HPSI_CHECK_LAUNCH();
-  gram_finalize<<<dim3((nst + 31) / 32, nst), dim3(32, 8), 0, st>>>(partial, splits, nst, dv, sym, fold, S);
+  auto fin = fold ? gram_finalize<true> : gram_finalize<false>;
+  fin<<<dim3((nst + 31) / 32, nst), dim3(32, 8), 0, st>>>(partial, splits, nst, dv, sym, S);
   HPSI_CHECK_LAUNCH();
   return HPSI_OK;
 }
