@@ -426,28 +426,20 @@ hpsi_status hpsi_mesh_create(const hpsi_mesh_desc *d, hpsi_mesh **out) {
   m->tiles_x = (B.nxo + PASS_TILE - 1) / PASS_TILE;
   m->tiles_y = (B.nyo + PASS_TILE - 1) / PASS_TILE;
   m->tile_z.assign(size_t(m->tiles_x) * m->tiles_y, make_int2(1 << 30, -1));
-  for (int i = 0; i < np; ++i) {
-    const int c = cell_of_row[i];
-    const int x = c % B.NX, y = (c / B.NX) % B.NY, z = c / (B.NX * B.NY);
-    int2 &t = m->tile_z[size_t((y - HAL) / PASS_TILE) * m->tiles_x + (x - HAL) / PASS_TILE];
-    t.x = std::min(t.x, z);
-    t.y = std::max(t.y, z);
-  }
-  for (auto &t : m->tile_z)
-    if (t.y >= 0) m->column_planes += t.y - t.x + 1;
   m->tiles_y8 = 2 * m->tiles_y;
   m->tile_z8.assign(size_t(m->tiles_x) * m->tiles_y8, make_int2(1 << 30, -1));
   std::vector<int2> col_z(size_t(B.NX) * B.NY, make_int2(1 << 30, -(1 << 30)));
   for (int i = 0; i < np; ++i) {
-    const int c = cell_of_row[i];
-    const int x = c % B.NX, y = (c / B.NX) % B.NY, z = c / (B.NX * B.NY);
-    int2 &t = m->tile_z8[size_t((y - HAL) / 8) * m->tiles_x + (x - HAL) / PASS_TILE];
-    t.x = std::min(t.x, z);
-    t.y = std::max(t.y, z);
-    int2 &cz = col_z[size_t(y) * B.NX + x];
-    cz.x = std::min(cz.x, z);
-    cz.y = std::max(cz.y, z);
+    const int x = d->lxyz[3 * i] - B.lo[0], y = d->lxyz[3 * i + 1] - B.lo[1], z = d->lxyz[3 * i + 2] - B.lo[2];
+    for (int2 *t : {&m->tile_z[size_t((y - HAL) / PASS_TILE) * m->tiles_x + (x - HAL) / PASS_TILE],
+                    &m->tile_z8[size_t((y - HAL) / 8) * m->tiles_x + (x - HAL) / PASS_TILE],
+                    &col_z[size_t(y) * B.NX + x]}) {
+      t->x = std::min(t->x, z);
+      t->y = std::max(t->y, z);
+    }
   }
+  for (auto &t : m->tile_z)
+    if (t.y >= 0) m->column_planes += t.y - t.x + 1;
   m->np = np;
   m->np_part = npp;
   m->order = ord;
