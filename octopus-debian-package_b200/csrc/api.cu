@@ -75,30 +75,6 @@ __global__ void scatter_cells_kernel(const double *v, const int *cell_of_row, in
   if (i < n) vcell[cell_of_row[i]] = v[i];
 }
 
-// Tables of the projectors that the device makes itself: the values in FP32,
-// the covered rows' numbers (kidx, -1 before) and the values in block order (KetArgs::pk).
-__global__ void __launch_bounds__(256) kb_layout_kernel(const double *pt, long long nval, const int *krows, int nk,
-                                                        const int4 *blk, int nblk, const int2 *brow, const int4 *ent,
-                                                        float *ptf, int *kidx, double *pk, float *pkf) {
-  const long long t0 = blockIdx.x * 256LL + threadIdx.x, step = gridDim.x * 256LL;
-  for (long long i = t0; i < nval; i += step) ptf[i] = float(pt[i]);
-  for (long long i = t0; i < nk; i += step) kidx[krows[i]] = int(i);
-  for (int b = blockIdx.x; b < nblk; b += gridDim.x) {
-    const int4 D = blk[b];
-    const int n = D.y & 255, ne = D.y >> 8;
-    int w = D.w;
-    for (int e = 0; e < ne; ++e) {
-      const int q = ent[D.z + e].z;
-      for (int i = threadIdx.x; i < n * q; i += 256) {
-        const double v = pt[ent[brow[D.x + i / q].y + e].x + i % q];
-        pk[w + i] = v;
-        pkf[w + i] = float(v);
-      }
-      w += n * q;
-    }
-  }
-}
-
 // rho[r] (+)= the density of row r from the fused partials: the KB ket's row
 // sums for covered rows (their final values), the pass's chunk sums elsewhere;
 // fixed summation order.
@@ -665,8 +641,8 @@ hpsi_status hpsi_hamiltonian::ensure_bra_stream() {
 }
 
 void hpsi_hamiltonian::proj_free() {
-  dev_free(kb_tables);  // (holds every table below)
-  kb_tables = nullptr;
+  for (void *p : kb_tables) dev_free(p);  // (hold every table below)
+  kb_tables.clear();
   d_kidx = nullptr;
   d_kblk = nullptr;
   d_brow = nullptr;
@@ -823,72 +799,6 @@ hpsi_status hpsi_hamiltonian_set_phase_corr(hpsi_hamiltonian *h, const double *p
   return HPSI_OK;
 }
 
-// Covered rows of the projector spheres, in mesh order: krows[nk], kptr[nk + 1],
-// ent their entries in matrix order; and in blocks of rows with the same list of
-// matrices (KetArgs::blk, brow; lists in the order of their first row).  A
-// row's list is a number: matrix i leads from a list to the list with i at its
-// end, so that one pass over the points finds them all.
-struct KbRows {
-  std::vector<int> krows, kptr;
-  std::vector<int4> ent, blk;
-  std::vector<int2> brow;
-};
-static void kb_rows(int np, const std::vector<int4> &mat, const std::vector<int> &prow, const int *map, KbRows &o) {
-  struct List {
-    int len, nproj;   // matrices, projectors of all of them
-    int from, next;   // last matrix seen at this list, the list it leads to
-    int rows, first;  // rows of the list, place of the next one
-  };
-  std::vector<List> lists(1, List{0, 0, -1, 0, 0, 0});  // list 0: no matrix
-  std::vector<int> id(np, 0);
-  for (int i = 0; i < int(mat.size()); ++i)
-    for (int k = 0; k < mat[i].x; ++k) {
-      int &at = id[map[mat[i].z + k]];
-      if (lists[at].from != i) {
-        lists[at].from = i;
-        lists[at].next = int(lists.size());
-        lists.push_back(List{lists[at].len + 1, lists[at].nproj + mat[i].y, -1, 0, 0, 0});
-      }
-      at = lists[at].next;
-    }
-  std::vector<int> order;  // lists by their first row
-  int nk = 0;
-  for (int r = 0; r < np; ++r)
-    if (id[r]) {
-      if (lists[id[r]].rows++ == 0) order.push_back(id[r]);
-      ++nk;
-    }
-  int at = 0, npk = 0;
-  for (int l : order) {
-    List &L = lists[l];
-    L.first = at;
-    for (int i = 0; i < L.rows; i += 32) {
-      const int n = std::min(32, L.rows - i);
-      o.blk.push_back(make_int4(at + i, n + 256 * L.len, 0, npk));
-      npk += n * L.nproj;
-    }
-    at += L.rows;
-  }
-  o.krows.reserve(nk);
-  o.kptr.reserve(size_t(nk) + 1);
-  o.kptr.push_back(0);
-  o.brow.resize(nk);
-  for (int r = 0; r < np; ++r)
-    if (id[r]) {
-      List &L = lists[id[r]];
-      const int e = o.kptr.back();
-      o.brow[L.first++] = make_int2(r, e);
-      o.krows.push_back(r);
-      o.kptr.push_back(e + L.len);
-      id[r] = e;  // place of the row's next entry
-    }
-  for (int4 &b : o.blk) b.z = o.brow[b.x].y;
-  o.ent.resize(o.kptr.back());
-  for (int i = 0; i < int(mat.size()); ++i)
-    for (int k = 0; k < mat[i].x; ++k)
-      o.ent[id[map[mat[i].z + k]]++] = make_int4(mat[i].w + k * mat[i].y, prow[i], mat[i].y, mat[i].z + k);
-}
-
 hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, const int32_t *npoints,
                                             const int32_t *nprojs, const int32_t *map, const double *matrices,
                                             const double *scal) {
@@ -939,11 +849,11 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, c
   const int npk = nblk ? int(nval) : 0;
   int minp = 1 << 30;
   for (int i = 0; i < nmat; ++i) minp = std::min(minp, int(npoints[i]));
-  // one allocation for all tables; those without a source are made on the device
+  // those without a source are made on the device
   struct Part {
     void **dp;
     const void *src;
-    size_t bytes;
+    size_t bytes, chunk = 0, at = 0;
   };
   std::vector<Part> parts;
   auto up = [&](auto **dp, const void *src, size_t n) {
@@ -964,14 +874,26 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, c
   up(&h->d_brow, R.brow.data(), nblk ? nk : 0);
   up(&h->d_pk, nullptr, npk);
   up(&h->d_pk_f, nullptr, npk);
-  size_t total = 0;
-  for (const Part &q : parts) total += (q.bytes + 255) / 256 * 256;
-  hpsi_status s = dev_alloc(&h->kb_tables, std::max<size_t>(total, 256));
-  char *at = static_cast<char *>(h->kb_tables);
+  // Small allocations take 2 us (3 us to free), those of more than a 2 MB page 330 us
+  // (260 us): the tables above 1 MB share one, the others have their own.
+  std::vector<size_t> chunks(1, 0);
+  for (Part &q : parts) {
+    const size_t n = (q.bytes + 255) / 256 * 256;
+    if (n > 1 << 20) {
+      q.at = chunks[0];
+      chunks[0] += n;
+    } else {
+      q.chunk = chunks.size();
+      chunks.push_back(n);
+    }
+  }
+  hpsi_status s = HPSI_OK;
+  h->kb_tables.assign(chunks.size(), nullptr);
+  for (size_t i = 0; i < chunks.size() && !s; ++i)
+    if (chunks[i]) s = dev_alloc(&h->kb_tables[i], chunks[i]);
   for (const Part &q : parts) {
     if (s) break;
-    *q.dp = at;
-    at += (q.bytes + 255) / 256 * 256;
+    *q.dp = static_cast<char *>(h->kb_tables[q.chunk]) + q.at;
     const cudaError_t e =
         q.bytes && q.src ? cudaMemcpy(*q.dp, q.src, q.bytes, cudaMemcpyHostToDevice) : cudaSuccess;
     if (e != cudaSuccess) {
@@ -980,16 +902,9 @@ hpsi_status hpsi_hamiltonian_set_projectors(hpsi_hamiltonian *h, int32_t nmat, c
     }
   }
   if (!s) {
-    cudaError_t e = cudaMemsetAsync(h->d_kidx, 0xff, size_t(m->np) * sizeof(int), nullptr);
-    kb_layout_kernel<<<4 * m->num_sms, 256>>>(h->d_pt, nval, h->d_krows, nk, h->d_kblk, nblk, h->d_brow, h->d_kb_ent,
-                                              h->d_pt_f, h->d_kidx, h->d_pk, h->d_pk_f);
-    g_launches++;
-    if (e == cudaSuccess) e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // the set-up call returns with its tables in place
-    if (e != cudaSuccess) {
-      set_error(std::string("hpsi_hamiltonian_set_projectors: ") + cudaGetErrorString(e));
-      s = HPSI_ERR_CUDA;
-    }
+    const KbTables t = {h->d_pt, nval, h->d_krows, nk, h->d_kblk, nblk, h->d_brow, h->d_kb_ent,
+                        h->d_pt_f, h->d_kidx, m->np, h->d_pk, h->d_pk_f};
+    s = launch_kb_layout(t, m->num_sms);
   }
   if (s) {
     h->proj_free();

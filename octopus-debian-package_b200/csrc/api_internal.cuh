@@ -107,7 +107,7 @@ struct hpsi_hamiltonian {
   int *d_src_phase = nullptr;
   // KB projectors
   int nmat = 0, nprojections = 0, max_nproj = 0;
-  void *kb_tables = nullptr;  // one allocation for the tables of the projectors
+  std::vector<void *> kb_tables;  // allocations of the tables of the projectors
   int4 *d_mat = nullptr;
   int *d_proj_row = nullptr, *d_map = nullptr;
   double *d_pt = nullptr, *d_scal = nullptr;

@@ -672,4 +672,92 @@ template hpsi_status launch_ket<float>(const KetArgs &, cudaStream_t);
 template hpsi_status launch_bra<double>(const ProjArgs &, bool, int, cudaStream_t);
 template hpsi_status launch_bra<float>(const ProjArgs &, bool, int, cudaStream_t);
 
+void kb_rows(int np, const std::vector<int4> &mat, const std::vector<int> &prow, const int *map, KbRows &o) {
+  struct List {
+    int len, nproj;   // matrices, projectors of all of them
+    int from, next;   // last matrix seen at this list, the list it leads to
+    int rows, first;  // rows of the list, place of the next one
+  };
+  std::vector<List> lists(1, List{0, 0, -1, 0, 0, 0});  // list 0: no matrix
+  std::vector<int> id(np, 0);
+  for (int i = 0; i < int(mat.size()); ++i)
+    for (int k = 0; k < mat[i].x; ++k) {
+      int &at = id[map[mat[i].z + k]];
+      if (lists[at].from != i) {
+        lists[at].from = i;
+        lists[at].next = int(lists.size());
+        lists.push_back(List{lists[at].len + 1, lists[at].nproj + mat[i].y, -1, 0, 0, 0});
+      }
+      at = lists[at].next;
+    }
+  std::vector<int> order;  // lists by their first row
+  int nk = 0;
+  for (int r = 0; r < np; ++r)
+    if (id[r]) {
+      if (lists[id[r]].rows++ == 0) order.push_back(id[r]);
+      ++nk;
+    }
+  int at = 0, npk = 0;
+  for (int l : order) {
+    List &L = lists[l];
+    L.first = at;
+    for (int i = 0; i < L.rows; i += 32) {
+      const int n = std::min(32, L.rows - i);
+      o.blk.push_back(make_int4(at + i, n + 256 * L.len, 0, npk));
+      npk += n * L.nproj;
+    }
+    at += L.rows;
+  }
+  o.krows.reserve(nk);
+  o.kptr.reserve(size_t(nk) + 1);
+  o.kptr.push_back(0);
+  o.brow.resize(nk);
+  for (int r = 0; r < np; ++r)
+    if (id[r]) {
+      List &L = lists[id[r]];
+      const int e = o.kptr.back();
+      o.brow[L.first++] = make_int2(r, e);
+      o.krows.push_back(r);
+      o.kptr.push_back(e + L.len);
+      id[r] = e;  // place of the row's next entry
+    }
+  for (int4 &b : o.blk) b.z = o.brow[b.x].y;
+  o.ent.resize(o.kptr.back());
+  for (int i = 0; i < int(mat.size()); ++i)
+    for (int k = 0; k < mat[i].x; ++k)
+      o.ent[id[map[mat[i].z + k]]++] = make_int4(mat[i].w + k * mat[i].y, prow[i], mat[i].y, mat[i].z + k);
+}
+
+// Tables of the projectors that the device makes itself: the values in FP32,
+// the covered rows' numbers (kidx, -1 before) and the values in block order (KetArgs::pk).
+namespace {
+__global__ void __launch_bounds__(256) kb_layout_kernel(const KbTables t) {
+  const long long t0 = blockIdx.x * 256LL + threadIdx.x, step = gridDim.x * 256LL;
+  for (long long i = t0; i < t.nval; i += step) t.ptf[i] = float(t.pt[i]);
+  for (long long i = t0; i < t.nk; i += step) t.kidx[t.krows[i]] = int(i);
+  for (int b = blockIdx.x; b < t.nblk; b += gridDim.x) {
+    const int4 D = t.blk[b];
+    const int n = D.y & 255, ne = D.y >> 8;
+    int w = D.w;
+    for (int e = 0; e < ne; ++e) {
+      const int q = t.ent[D.z + e].z;
+      for (int i = threadIdx.x; i < n * q; i += 256) {
+        const double v = t.pt[t.ent[t.brow[D.x + i / q].y + e].x + i % q];
+        t.pk[w + i] = v;
+        t.pkf[w + i] = float(v);
+      }
+      w += n * q;
+    }
+  }
+}
+}  // namespace
+
+hpsi_status launch_kb_layout(const KbTables &t, int num_sms) {
+  HPSI_TRY_CUDA(cudaMemsetAsync(t.kidx, 0xff, size_t(t.np) * sizeof(int), nullptr));
+  kb_layout_kernel<<<4 * num_sms, 256>>>(t);
+  HPSI_CHECK_LAUNCH();
+  HPSI_TRY_CUDA(cudaStreamSynchronize(nullptr));
+  return HPSI_OK;
+}
+
 }  // namespace hpsi

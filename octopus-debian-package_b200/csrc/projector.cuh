@@ -1,6 +1,8 @@
 // KB projector bra kernels (see projector.cu).
 #pragma once
 
+#include <vector>
+
 #include "common.cuh"
 
 namespace hpsi {
@@ -74,5 +76,36 @@ template <typename T>
 hpsi_status launch_bra(const ProjArgs &p, bool use_tensor, int ksplit, cudaStream_t st);
 template <typename T>
 hpsi_status launch_ket(const KetArgs &k, cudaStream_t st);
+
+// Covered rows of the projector spheres, in mesh order: krows[nk], kptr[nk + 1],
+// ent their entries in matrix order; and in blocks of rows with the same list of
+// matrices (KetArgs::blk, brow; lists in the order of their first row).  A
+// row's list is a number: matrix i leads from a list to the list with i at its
+// end, so that one pass over the points finds them all.
+struct KbRows {
+  std::vector<int> krows, kptr;
+  std::vector<int4> ent, blk;
+  std::vector<int2> brow;
+};
+void kb_rows(int np, const std::vector<int4> &mat, const std::vector<int> &prow, const int *map, KbRows &o);
+
+// Tables of the projectors on the device; launch_kb_layout makes those from ptf on
+// (the values in FP32, the covered rows' numbers, the values in block order) and
+// waits for them.
+struct KbTables {
+  const double *pt;
+  long long nval;
+  const int *krows;
+  int nk;
+  const int4 *blk;
+  int nblk;
+  const int2 *brow;
+  const int4 *ent;
+  float *ptf;
+  int *kidx, np;
+  double *pk;
+  float *pkf;
+};
+hpsi_status launch_kb_layout(const KbTables &t, int num_sms);
 
 }  // namespace hpsi
