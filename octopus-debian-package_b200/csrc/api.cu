@@ -1074,8 +1074,11 @@ int choose_zb_tmem(const hpsi_mesh *m, int chunks) {
   int best = 1 << 20;
   double best_t = 1e300;
   // deepest first; no shallower ones once a depth gives four waves of units (they
-  // only add halo planes, and the first call on a mesh waits for this choice)
-  std::vector<int> cands = {1 << 20, 64, 48, 40, 32, 24, 20, 16, 12};
+  // only add halo planes, and the first call on a mesh waits for this choice).  Down
+  // to two planes: rods and slabs have few tile columns (14 x 14 x 400 points, 8 FP64
+  // states: 34 us with blocks of 12 planes at least, 18 with three; 100 x 100 x 6:
+  // 24 us whole, 16 with two; the blocked pass took 30 and 20)
+  std::vector<int> cands = {1 << 20, 64, 48, 40, 32, 24, 20, 16, 12, 10, 8, 6, 5, 4, 3, 2};
   for (int n = 2; n <= 16 && (tall + n - 1) / n >= 4; ++n) cands.push_back((tall + n - 1) / n);
   std::sort(cands.begin(), cands.end(), std::greater<int>());
   cands.erase(std::unique(cands.begin(), cands.end()), cands.end());

@@ -38,7 +38,7 @@ def _oracle(m, v=None, **more):
     return O.Hamiltonian(m, laplacian_weights(m.spacing), star_points(), v=v, **more)
 
 
-@pytest.mark.parametrize("zb", [0, 4, 5, 100])
+@pytest.mark.parametrize("zb", [0, 1, 2, 3, 4, 5, 100])
 @pytest.mark.parametrize("shape", [(16, 17, 9), (33, 15, 6), (5, 4, 12)])
 @pytest.mark.parametrize("dtype,nst", [("c128", 1), ("c128", 8), ("c128", 13), ("c64", 2), ("c64", 16), ("c64", 22)])
 def test_tile_and_chunk_edges(cuda, dtype, nst, shape, zb, monkeypatch):
