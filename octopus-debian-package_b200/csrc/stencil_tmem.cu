@@ -26,17 +26,19 @@
 // compute.  A stage changes hands through a full barrier (every producer
 // thread's copies) and an empty barrier (every consumer warp, after its last
 // read of the stage); each wait is bounded and records HPSI_ERR_TIMEOUT in
-// p.err.  The register split leaves the consumers 208 registers: a few bytes of
-// spills in either role cost 10-60 % (the hand-over waits for local stores).
+// p.err.  The register split leaves the consumers 208 registers; the hand-over
+// waits for local stores, so that spills in the loop over the planes cost 10-60 %.
+// The apply forms have none, the FP64 Horner forms 16 bytes, the grouped kernels 16 to
+// 24, with phases 76 to 120.
 //
 // Measured (B200, CUDA events; the blocked pass of stencil_blk.cu before):
 // R = 12 sphere, 904,089 points, 128 states: apply 1.472 -> 0.984 ms FP64 (3.77
 // TB/s of psi read once and H psi written once), 0.731 -> 0.517 FP32; Horner pass
 // 1.688 -> 1.282 and 0.832 -> 0.664; 64^3 box, 32 states, FP64 0.114 -> 0.073 ms;
 // 48^3, 16 states 0.042 -> 0.024.  On 64 planes of 16 x 16 tiles (one CTA per
-// SM) the counters read: issue slots 60 %, shared-memory pipe 51 %, FP64 pipe 44 %
-// busy, and an SM takes 2,840 cycles a plane where the FP64 pipe alone needs
-// 1,660: what bounds it now is the latency of two computing warps per scheduler.
+// SM) the counters read: issue slots 61 %, shared-memory pipe 50 %, FP64 pipe 44 %
+// busy, and an SM takes 3,700 cycles a plane step where the FP64 pipe alone needs
+// 1,600: what bounds it now is the latency of two computing warps per scheduler.
 // Tried and not kept: one persistent CTA per SM over a static unit list (15 %
 // slower: it loses the neighbouring tiles' L2 reuse and the hardware's balancing),
 // waits that sleep in hardware, loads of tensor memory that wait in one
